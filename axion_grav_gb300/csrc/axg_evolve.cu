@@ -404,7 +404,14 @@ __device__ __forceinline__ void site_u(const FusedParams<double> &P, double S, d
 // pointwise fields of plane k arrive by TMA in a kPwStages ring (`gpw`
 // continues across columns like `gplane`); without it they are loaded into
 // registers at the top of each plane.
-template <typename R, int TX, int TY, bool UIJ, bool PW>
+//
+// RAG: N need not be a multiple of the tile (FP32, N a multiple of 4 so that
+// the rows' byte stride and the wrapped halo coordinates stay multiples of 16
+// bytes).  The last tiles of a row, column or z-range reach past the lattice:
+// TMA fills those elements with zeros, their threads neither compute nor
+// store, and the sites at x, y = N - 1 take their neighbour from the halo box
+// (loaded at coordinate 0) instead of from inside the tile.
+template <typename R, int TX, int TY, bool UIJ, bool PW, bool RAG = false>
 __device__ __forceinline__ bool fused_column(const CUtensorMap *tm_prow, const CUtensorMap *tm_pbody,
                                              const CUtensorMap *tm_phalo, const CUtensorMap *tm_urow,
                                              const CUtensorMap *tm_ubody, const CUtensorMap *tm_uhalo,
@@ -414,9 +421,14 @@ __device__ __forceinline__ bool fused_column(const CUtensorMap *tm_prow, const C
   using L = StageLayout<R, TX, TY, UIJ>;
   using PL = PwLayout<R, TX, TY, UIJ>;
   using V = typename V2<R>::T;
-  const int n = P.n, zc = P.zc;
+  int zc = P.zc;
+  if constexpr (RAG) zc = P.n - z0 < zc ? P.n - z0 : zc;
+  const int n = P.n;
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
   const int nplanes = zc + 2;
+  const bool inside = !RAG || (x0 + tx < n && y0 + ty < n);
+  // a site inside the tile whose x + 1 (y + 1) is across the lattice's edge
+  const bool xedge = RAG && x0 + tx == n - 1, yedge = RAG && y0 + ty == n - 1;
 
   auto issue = [&](int p) {
     int z = z0 - 1 + p;
@@ -426,9 +438,9 @@ __device__ __forceinline__ bool fused_column(const CUtensorMap *tm_prow, const C
     const uint32_t bar = smem_u32(&bars[s]);
     mbar_expect_tx(bar, (uint32_t)L::tx_bytes);
     const int ym = y0 == 0 ? n - 1 : y0 - 1;
-    const int yp = y0 + TY == n ? 0 : y0 + TY;
+    const int yp = (RAG ? y0 + TY >= n : y0 + TY == n) ? 0 : y0 + TY;
     const int xpl = x0 - L::PHW < 0 ? x0 - L::PHW + n : x0 - L::PHW;
-    const int xr = x0 + TX == n ? 0 : x0 + TX;
+    const int xr = (RAG ? x0 + TX >= n : x0 + TX == n) ? 0 : x0 + TX;
     tma_phi<R>(smem_u32(st + L::phi_main), tm_prow, x0, ym, z, bar);
     tma_phi<R>(smem_u32(st + L::phi_main + TX * (int)sizeof(V)), tm_pbody, x0, y0, z, bar);
     tma_phi<R>(smem_u32(st + L::phi_main + (TY + 1) * TX * (int)sizeof(V)), tm_prow, x0, yp, z, bar);
@@ -518,7 +530,7 @@ __device__ __forceinline__ bool fused_column(const CUtensorMap *tm_prow, const C
       }
     }
 
-    if (ok) {
+    if (ok && inside) {
       const unsigned char *sp = smem + stage_of(p - 1) * L::bytes;
       const unsigned char *sc = smem + stage_of(p) * L::bytes;
       const unsigned char *sn = smem + snext * L::bytes;
@@ -527,9 +539,9 @@ __device__ __forceinline__ bool fused_column(const CUtensorMap *tm_prow, const C
       const V *phr = reinterpret_cast<const V *>(sc + L::phi_hr);
       const V c0 = pm[(ty + 1) * TX + tx];
       const V xm = tx > 0 ? pm[(ty + 1) * TX + tx - 1] : phl[ty * L::PHW + L::PHW - 1];
-      const V xp = tx < TX - 1 ? pm[(ty + 1) * TX + tx + 1] : phr[ty * L::PHW];
+      const V xp = tx < TX - 1 && !xedge ? pm[(ty + 1) * TX + tx + 1] : phr[ty * L::PHW];
       const V ym = pm[ty * TX + tx];
-      const V yp = pm[(ty + 2) * TX + tx];
+      const V yp = pm[(yedge ? TY + 1 : ty + 2) * TX + tx];
       const V zm = reinterpret_cast<const V *>(sp + L::phi_main)[(ty + 1) * TX + tx];
       const V zp = reinterpret_cast<const V *>(sn + L::phi_main)[(ty + 1) * TX + tx];
 
@@ -553,9 +565,9 @@ __device__ __forceinline__ bool fused_column(const CUtensorMap *tm_prow, const C
           const int o = (c * TY + ty) * TX + tx;
           const R uc = ub[o];
           const R uxm = tx > 0 ? ub[o - 1] : uhl[(c * TY + ty) * L::UHW + L::UHW - 1];
-          const R uxp = tx < TX - 1 ? ub[o + 1] : uhr[(c * TY + ty) * L::UHW];
+          const R uxp = tx < TX - 1 && !xedge ? ub[o + 1] : uhr[(c * TY + ty) * L::UHW];
           const R uym = ty > 0 ? ub[o - TX] : ut[c * TX + tx];
-          const R uyp = ty < TY - 1 ? ub[o + TX] : ubt[c * TX + tx];
+          const R uyp = ty < TY - 1 && !yedge ? ub[o + TX] : ubt[c * TX + tx];
           const R uzm = ubp[o], uzp = ubn[o];
           R cc = sizeof(R) == 4 ? cuv[c] : R(0), udn, un;
           site_u(P, S[c], uc, uxm, uxp, uym, uyp, uzm, uzp, udv[c], cc, udn, un);
@@ -593,7 +605,7 @@ __device__ __forceinline__ void init_stage_barriers(uint64_t *bars) {
   __syncthreads();
 }
 
-template <typename R, int TX, int TY, bool UIJ, bool PW>
+template <typename R, int TX, int TY, bool UIJ, bool PW, bool RAG>
 __global__ void __launch_bounds__(TX *TY, (sizeof(R) == 4 && TX * TY <= 256 ? 2 : 1))
     k_fused(const __grid_constant__ CUtensorMap tm_prow, const __grid_constant__ CUtensorMap tm_pbody,
             const __grid_constant__ CUtensorMap tm_phalo, const __grid_constant__ CUtensorMap tm_urow,
@@ -607,11 +619,11 @@ __global__ void __launch_bounds__(TX *TY, (sizeof(R) == 4 && TX * TY <= 256 ? 2 
   unsigned char *pwsmem = smem + kStages * L::bytes;
   uint64_t *bars = reinterpret_cast<uint64_t *>(pwsmem + (PW ? kPwStages * PL::bytes : 0));
   init_stage_barriers(bars);
-  const int ncx = P.n / TX;
+  const int ncx = RAG ? (P.n + TX - 1) / TX : P.n / TX;
   const int x0 = (blockIdx.x % ncx) * TX, y0 = (blockIdx.x / ncx) * TY, z0 = blockIdx.y * P.zc;
   uint32_t gplane = 0, gpw = 0;
-  fused_column<R, TX, TY, UIJ, PW>(&tm_prow, &tm_pbody, &tm_phalo, &tm_urow, &tm_ubody, &tm_uhalo, pwm.m, P, x0,
-                                   y0, z0, smem, bars, gplane, pwsmem, bars + kStages, gpw);
+  fused_column<R, TX, TY, UIJ, PW, RAG>(&tm_prow, &tm_pbody, &tm_phalo, &tm_urow, &tm_ubody, &tm_uhalo, pwm.m, P, x0,
+                                        y0, z0, smem, bars, gplane, pwsmem, bars + kStages, gpw);
 }
 
 // ------------------------------------------------------------------------
@@ -680,48 +692,66 @@ __global__ void __launch_bounds__(TX *TY, (sizeof(R) == 4 && TX * TY <= 256 ? 2 
 }
 
 // ------------------------------------------------------------------------
-// The fused step as a plain stencil kernel: one thread per site, the stencil
-// read from global memory (through L1 / L2).  It serves lattices that no TMA
-// tile shape fits (N not a multiple of 32) and runs the same per-site
-// arithmetic as the tiled kernels, so it gives the same bits.
+// The fused step as a plain stencil kernel: the stencil is read from global
+// memory (through L1 / L2).  It runs the same per-site arithmetic as the
+// tiled kernels, so it gives the same bits, and serves the lattices where it
+// is the faster one (step_shape) or that TMA cannot address.
+// Threads are numbered along a z-plane, row after row, so a row length that
+// is no multiple of the warp leaves no lane idle; a thread walks zc planes
+// and keeps its column's values at z and z - 1 in registers.
 // ------------------------------------------------------------------------
 template <typename R, bool UIJ>
 __global__ void __launch_bounds__(256) k_fused_plain(const typename V2<R>::T *__restrict__ phi_in,
                                                      const R *__restrict__ u_in, FusedParams<R> P) {
   using V = typename V2<R>::T;
-  const int n = P.n;
-  const int ix = blockIdx.x * blockDim.x + threadIdx.x, iy = blockIdx.y * blockDim.y + threadIdx.y, iz = blockIdx.z;
-  if (ix >= n || iy >= n) return;
-  const int64_t n2 = (int64_t)n * n;
-  const int xm1 = ix == 0 ? n - 1 : ix - 1, xp1 = ix + 1 == n ? 0 : ix + 1;
-  const int ym1 = iy == 0 ? n - 1 : iy - 1, yp1 = iy + 1 == n ? 0 : iy + 1;
-  const int zm1 = iz == 0 ? n - 1 : iz - 1, zp1 = iz + 1 == n ? 0 : iz + 1;
-  const int64_t row = (int64_t)iz * n2 + (int64_t)iy * n;
-  const int64_t s = row + ix, sxm = row + xm1, sxp = row + xp1;
-  const int64_t sym = (int64_t)iz * n2 + (int64_t)ym1 * n + ix, syp = (int64_t)iz * n2 + (int64_t)yp1 * n + ix;
-  const int64_t szm = (int64_t)zm1 * n2 + (int64_t)iy * n + ix, szp = (int64_t)zp1 * n2 + (int64_t)iy * n + ix;
-  const V c0 = phi_in[s], xm = phi_in[sxm], xp = phi_in[sxp], ym = phi_in[sym], yp = phi_in[syp], zm = phi_in[szm],
-          zp = phi_in[szp];
-  const V pd = P.phid[s];
-  V cp{};
-  if constexpr (sizeof(R) == 4) cp = P.cphi[s];
-  V pdn, pn;
-  site_phi(P, c0, xm, xp, ym, yp, zm, zp, pd, cp, pdn, pn);
-  P.phid[s] = pdn;
-  if constexpr (sizeof(R) == 4) P.cphi[s] = cp;
-  P.phi_out[s] = pn;
+  const int n = P.n, n2 = n * n;
+  const int o = blockIdx.x * blockDim.x + threadIdx.x;
+  if (o >= n2) return;
+  const int iy = o / n, ix = o - iy * n;
+  const int oxm = ix == 0 ? o + n - 1 : o - 1, oxp = ix + 1 == n ? o + 1 - n : o + 1;
+  const int oym = iy == 0 ? o + n2 - n : o - n, oyp = iy + 1 == n ? o + n - n2 : o + n;
+  const int z0 = blockIdx.y * P.zc, z1 = z0 + P.zc < n ? z0 + P.zc : n;
+  const int64_t below = (int64_t)(z0 == 0 ? n - 1 : z0 - 1) * n2 + o;
+  V zm = phi_in[below], c0 = phi_in[(int64_t)z0 * n2 + o];
+  R uzm[UIJ ? 6 : 1], uc[UIJ ? 6 : 1];
   if constexpr (UIJ) {
-    R S[6];
-    site_sources(P, xm, xp, ym, yp, zm, zp, S);
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
-      const R *u = u_in + c * P.n3;
-      R cc = sizeof(R) == 4 ? P.cu[c * P.n3 + s] : R(0), udn, un;
-      site_u(P, S[c], u[s], u[sxm], u[sxp], u[sym], u[syp], u[szm], u[szp], P.ud[c * P.n3 + s], cc, udn, un);
-      P.ud[c * P.n3 + s] = udn;
-      if constexpr (sizeof(R) == 4) P.cu[c * P.n3 + s] = cc;
-      P.u_out[c * P.n3 + s] = un;
+      uzm[c] = u_in[c * P.n3 + below];
+      uc[c] = u_in[c * P.n3 + (int64_t)z0 * n2 + o];
     }
+  }
+  for (int z = z0; z < z1; ++z) {
+    const int64_t b = (int64_t)z * n2, s = b + o, above = (int64_t)(z + 1 == n ? 0 : z + 1) * n2 + o;
+    const V zp = phi_in[above];
+    const V xm = phi_in[b + oxm], xp = phi_in[b + oxp], ym = phi_in[b + oym], yp = phi_in[b + oyp];
+    const V pd = P.phid[s];
+    V cp{};
+    if constexpr (sizeof(R) == 4) cp = P.cphi[s];
+    V pdn, pn;
+    site_phi(P, c0, xm, xp, ym, yp, zm, zp, pd, cp, pdn, pn);
+    P.phid[s] = pdn;
+    if constexpr (sizeof(R) == 4) P.cphi[s] = cp;
+    P.phi_out[s] = pn;
+    if constexpr (UIJ) {
+      R S[6];
+      site_sources(P, xm, xp, ym, yp, zm, zp, S);
+#pragma unroll
+      for (int c = 0; c < 6; ++c) {
+        const R *u = u_in + c * P.n3;
+        const R uzp = u[above];
+        R cc = sizeof(R) == 4 ? P.cu[c * P.n3 + s] : R(0), udn, un;
+        site_u(P, S[c], uc[c], u[b + oxm], u[b + oxp], u[b + oym], u[b + oyp], uzm[c], uzp, P.ud[c * P.n3 + s], cc, udn,
+               un);
+        P.ud[c * P.n3 + s] = udn;
+        if constexpr (sizeof(R) == 4) P.cu[c * P.n3 + s] = cc;
+        P.u_out[c * P.n3 + s] = un;
+        uzm[c] = uc[c];
+        uc[c] = uzp;
+      }
+    }
+    zm = c0;
+    c0 = zp;
   }
 }
 
@@ -832,21 +862,22 @@ int build_tmaps(axg_ctx *ctx, int cfg) {
   return AXG_OK;
 }
 
-template <typename R, int TX, int TY, bool UIJ, bool PW>
+template <typename R, int TX, int TY, bool UIJ, bool PW, bool RAG = false>
 int launch_fused_t(axg_ctx *ctx, const FusedParams<R> &P, const char *name) {
   constexpr int smem = fused_smem_bytes<R, TX, TY, UIJ, PW>();
   static bool attr_set = false;
   if (!attr_set) {
-    AXG_CUDA_TRY(ctx, cudaFuncSetAttribute(k_fused<R, TX, TY, UIJ, PW>,
+    AXG_CUDA_TRY(ctx, cudaFuncSetAttribute(k_fused<R, TX, TY, UIJ, PW, RAG>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr_set = true;
   }
   const int b = ctx->cur;
-  dim3 grid((unsigned)((ctx->n / TX) * (ctx->n / TY)), (unsigned)(ctx->n / P.zc));
+  const int n = (int)ctx->n;
+  dim3 grid((unsigned)(((n + TX - 1) / TX) * ((n + TY - 1) / TY)), (unsigned)((n + P.zc - 1) / P.zc));
   dim3 block(TX, TY);
   PwMaps pwm;
   for (int q = 0; q < 4; ++q) pwm.m[q] = ctx->tm.pw[q];
-  AXG_LAUNCH(ctx, name, (k_fused<R, TX, TY, UIJ, PW>), grid, block, smem, ctx->tm.phi_row[b],
+  AXG_LAUNCH(ctx, name, (k_fused<R, TX, TY, UIJ, PW, RAG>), grid, block, smem, ctx->tm.phi_row[b],
              ctx->tm.phi_body[b], ctx->tm.phi_halo[b], ctx->tm.u_row[b], ctx->tm.u_body[b],
              ctx->tm.u_halo[b], pwm, P);
   return AXG_OK;
@@ -855,6 +886,12 @@ int launch_fused_t(axg_ctx *ctx, const FusedParams<R> &P, const char *name) {
 template <typename R, bool UIJ>
 int launch_fused_cfg(axg_ctx *ctx, const FusedParams<R> &P, int cfg, const char *name) {
   const axg_tile_cfg t = kTiles[cfg];
+  if constexpr (sizeof(R) == 4) {
+    if (ctx->n % t.tx) {  // ragged lattice (step_shape picks pointwise-TMA tiles only)
+      if (t.ty == 8) return launch_fused_t<R, 32, 8, UIJ, true, true>(ctx, P, name);
+      return launch_fused_t<R, 32, 4, UIJ, true, true>(ctx, P, name);
+    }
+  }
   if (t.pw) {
     if (t.tx == 32 && t.ty == 8) return launch_fused_t<R, 32, 8, UIJ, true>(ctx, P, name);
     if (t.tx == 32 && t.ty == 4) return launch_fused_t<R, 32, 4, UIJ, true>(ctx, P, name);
@@ -897,17 +934,7 @@ int axg_evo_tile_supported(const axg_ctx *ctx, int i) {
   return 1;
 }
 
-int axg_evo_default_tile(const axg_ctx *ctx) {
-  // the first supported shape in the preference order
-  const bool fp32 = ctx->p.precision == AXG_PREC_FP32_MIXED;
-  for (int i = 0; i < kNumTiles; ++i) {
-    const int cfg = axg_evo_tile_preference(fp32, i);
-    if (axg_evo_tile_supported(ctx, cfg)) return cfg;
-  }
-  return -1;
-}
-
-// Preferred order for a context that was not autotuned.  FP32: the shapes
+// Preferred order for an ensemble that was not autotuned.  FP32: the shapes
 // with the pointwise fields in the TMA ring first (the autotuner's picks at
 // 256^3 to 1024^3); FP64 is bound by the FP64 pipe and nearly indifferent
 // to the shape.
@@ -960,21 +987,65 @@ int axg_evo_kick_plain(axg_ctx *ctx, double t, double dt) {
   return AXG_OK;
 }
 
+namespace {
+// Which kernel a fused step runs, and the z-planes a CTA walks.  cfg: an index
+// of kTiles, or -1 for the plain stencil kernel.
+struct StepShape {
+  int cfg, zc;
+  bool suffix;  // the timed kernel's name ends in _plain: the lattice has no tile, or the plain kernel was asked for
+};
+
+// A tile chosen by axg_set_tile / axg_autotune, else by this rule (us per
+// step, GB300, FP32 with six u_ij unless said):
+//  * the TMA kernel marches a CTA through its planes one after another, about
+//    1.4 us a plane, so small lattices leave the chip waiting: plain 6.2
+//    against 22.7 at 32^3, 12.4 / 22.7 at 64^3, 14.9 / 22.7 at 76^3, but
+//    33 / 25 at 88^3 and 47 / 33 at 96^3, where traffic to L2 and HBM starts
+//    to count.  phi alone has a quarter of the bytes and less reuse to gain:
+//    4.2 / 12.4 at 32^3, 36.5 / 40 at 160^3, 88.5 / 92 at 224^3, 129 / 126 at
+//    256^3, 1000 / 927 at 512^3;
+//  * FP64 is bound by the FP64 pipe; the plain kernel's many small CTAs fill
+//    it best (14.5 against 107 at 32^3, 598 / 720 at 128^3, 4.76 / 4.79 ms at
+//    256^3);
+//  * TMA needs rows of a multiple of 16 bytes: N a multiple of 4;
+//  * of the TMA tiles 32 x 8 x 32 moves the fewest halo bytes (3.90 against
+//    4.08 ms at 512^3) unless its larger CTAs leave the last of their waves
+//    (2 per SM, 152 SMs) mostly empty: 139 against 130 at 160^3, 48.6 / 32.9
+//    at 96^3.  phi alone: 32 x 4 x 16 (126 against 139 at 256^3, 927 / 941
+//    at 512^3).
+// Planes of the plain kernel: one per CTA while that fills the chip, then
+// four (column values kept in registers: 806 -> 792 at 256^3, 145 -> 129 phi
+// alone); one in FP64 (82 against 92 at 64^3).  Ragged lattices split z evenly.
+StepShape step_shape(const axg_ctx *ctx) {
+  const int n = (int)ctx->n;
+  const bool fp32 = ctx->p.precision == AXG_PREC_FP32_MIXED, uij = ctx->p.gw_mode == AXG_GW_UIJ;
+  const char *pe = std::getenv("AXG_FUSED_PLAIN");  // 1: the plain kernel for any N (tests compare the two)
+  const bool asked = pe && pe[0] == '1';
+  const StepShape plain{-1, fp32 && n >= 56 ? 4 : 1, asked || n % 32 != 0};
+  if (asked) return plain;
+  if (ctx->tile_cfg >= 0 && axg_evo_tile_supported(ctx, ctx->tile_cfg))
+    return {ctx->tile_cfg, kTiles[ctx->tile_cfg].zc, false};
+  if (!fp32 || (n & 3) || n <= (uij ? 80 : 224)) return plain;
+  constexpr int kTile8 = 8, kTile4 = 10;  // 32 x 8 x 32 and 32 x 4 x 16, pointwise fields by TMA
+  const double waves = (double)((n + 31) / 32) * ((n + 7) / 8) * ((n + 31) / 32) / (2 * 152);
+  const int cfg = uij && waves > 0.83 * std::ceil(waves) ? kTile8 : kTile4;
+  const int chunks = (n + kTiles[cfg].zc - 1) / kTiles[cfg].zc;
+  return {cfg, (n + chunks - 1) / chunks, false};
+}
+}  // namespace
+
 int axg_evo_kick_drift(axg_ctx *ctx, double t, double dt, double dtd) {
   if (ctx->p.precision == AXG_PREC_FP64_PLAIN)
     return axg_set_error(ctx, AXG_ERR_STATE, "fused step requested on the FP64-plain path");
-  int cfg = ctx->tile_cfg >= 0 ? ctx->tile_cfg : axg_evo_default_tile(ctx);
-  // no TMA tile shape fits (N not a multiple of 32): the plain stencil
-  // kernel; AXG_FUSED_PLAIN=1 selects it for any N (tests compare the two)
-  const char *pe = std::getenv("AXG_FUSED_PLAIN");
-  const bool plain = cfg < 0 || !axg_evo_tile_supported(ctx, cfg) || (pe && pe[0] == '1');
+  const StepShape shape = step_shape(ctx);
+  const bool plain = shape.cfg < 0;
+  const int cfg = shape.cfg;
   if (!plain) AXG_TRY(build_tmaps(ctx, cfg));
   double f[4], pot[4];
   axg_kick_coeffs(&ctx->p, t, dt, f, pot);
   const bool uij = ctx->p.gw_mode == AXG_GW_UIJ;
   const int b = ctx->cur, o = 1 - b;
-  const axg_tile_cfg tc = plain ? axg_tile_cfg{32, 8, 1, 0} : kTiles[cfg];
-  const dim3 pblock(32, 8), pgrid((unsigned)((ctx->n + 31) / 32), (unsigned)((ctx->n + 7) / 8), (unsigned)ctx->n);
+  const dim3 pblock(256), pgrid((unsigned)((ctx->n3 / ctx->n + 255) / 256), (unsigned)((ctx->n + shape.zc - 1) / shape.zc));
   if (ctx->p.precision == AXG_PREC_FP32_MIXED) {
     FusedParams<float> P;
     P.phi_out = (float2 *)ctx->phi[o];
@@ -985,7 +1056,7 @@ int axg_evo_kick_drift(axg_ctx *ctx, double t, double dt, double dtd) {
     P.cu = (float *)ctx->cu;
     P.n3 = ctx->n3;
     P.n = (int)ctx->n;
-    P.zc = tc.zc;
+    P.zc = shape.zc;
     P.f1 = (float)f[0];
     P.f2 = (float)f[1];
     P.f3 = (float)f[2];
@@ -1001,10 +1072,12 @@ int axg_evo_kick_drift(axg_ctx *ctx, double t, double dt, double dtd) {
     P.d_pow2 = 0;
     P.err = ctx->d_err;
     if (plain && uij)
-      AXG_LAUNCH(ctx, "fused_kd_fp32_uij_plain", (k_fused_plain<float, true>), pgrid, pblock, 0,
+      AXG_LAUNCH(ctx, shape.suffix ? "fused_kd_fp32_uij_plain" : "fused_kd_fp32_uij",
+                 (k_fused_plain<float, true>), pgrid, pblock, 0,
                  (const float2 *)ctx->phi[b], (const float *)ctx->u[b], P);
     else if (plain)
-      AXG_LAUNCH(ctx, "fused_kd_fp32_phi_plain", (k_fused_plain<float, false>), pgrid, pblock, 0,
+      AXG_LAUNCH(ctx, shape.suffix ? "fused_kd_fp32_phi_plain" : "fused_kd_fp32_phi",
+                 (k_fused_plain<float, false>), pgrid, pblock, 0,
                  (const float2 *)ctx->phi[b], (const float *)ctx->u[b], P);
     else if (uij) AXG_TRY((launch_fused_cfg<float, true>(ctx, P, cfg, "fused_kd_fp32_uij")));
     else AXG_TRY((launch_fused_cfg<float, false>(ctx, P, cfg, "fused_kd_fp32_phi")));
@@ -1018,7 +1091,7 @@ int axg_evo_kick_drift(axg_ctx *ctx, double t, double dt, double dtd) {
     P.cu = nullptr;
     P.n3 = ctx->n3;
     P.n = (int)ctx->n;
-    P.zc = tc.zc;
+    P.zc = shape.zc;
     P.f1 = f[0];
     P.f2 = f[1];
     P.f3 = f[2];
@@ -1034,10 +1107,12 @@ int axg_evo_kick_drift(axg_ctx *ctx, double t, double dt, double dtd) {
     P.inv_d = 1.0 / P.d;
     P.err = ctx->d_err;
     if (plain && uij)
-      AXG_LAUNCH(ctx, "fused_kd_fp64_uij_plain", (k_fused_plain<double, true>), pgrid, pblock, 0,
+      AXG_LAUNCH(ctx, shape.suffix ? "fused_kd_fp64_uij_plain" : "fused_kd_fp64_uij",
+                 (k_fused_plain<double, true>), pgrid, pblock, 0,
                  (const double2 *)ctx->phi[b], (const double *)ctx->u[b], P);
     else if (plain)
-      AXG_LAUNCH(ctx, "fused_kd_fp64_phi_plain", (k_fused_plain<double, false>), pgrid, pblock, 0,
+      AXG_LAUNCH(ctx, shape.suffix ? "fused_kd_fp64_phi_plain" : "fused_kd_fp64_phi",
+                 (k_fused_plain<double, false>), pgrid, pblock, 0,
                  (const double2 *)ctx->phi[b], (const double *)ctx->u[b], P);
     else if (uij) AXG_TRY((launch_fused_cfg<double, true>(ctx, P, cfg, "fused_kd_fp64_uij")));
     else AXG_TRY((launch_fused_cfg<double, false>(ctx, P, cfg, "fused_kd_fp64_phi")));

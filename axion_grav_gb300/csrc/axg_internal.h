@@ -262,7 +262,6 @@ int axg_encode_tmap(axg_ctx *ctx, CUtensorMap *m, CUtensorMapDataType dt, int ra
 int axg_evo_tile_count();
 axg_tile_cfg axg_evo_tile(int i);
 int axg_evo_tile_supported(const axg_ctx *ctx, int i);
-int axg_evo_default_tile(const axg_ctx *ctx);
 int axg_evo_tile_preference(bool fp32, int rank);  // tile index of the rank-th preferred shape
 int axg_evo_build_tmaps(axg_ctx *ctx, int cfg);
 // one launch over every member's columns (ensemble.cu drives it); persistent
