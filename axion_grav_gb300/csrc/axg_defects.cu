@@ -24,7 +24,7 @@
 //                  corner difference within the margin of +-pi is redone in
 //                  FP64)
 //   4. compaction: string and wall cells listed in cell order
-//   5. fits      : string cells lane-scheduled from a counter -- the search
+//   5. fits      : string cells by groups of eight lanes -- the search
 //                  of position_string (1001 random starts, screened in FP32,
 //                  + Nelder-Mead, defects_3d.f90:435-603; the chi2 in
 //                  float-float on the FP32 pipes, axg_ffchi2.h), string_length
@@ -439,83 +439,132 @@ __device__ double string_length(const double pos[3], const double dir[3]) {
   return 0.0;
 }
 
-__device__ __forceinline__ bool out_of_box(const double t[4]) {
-  const double mx[4] = {1.0, kRefPi, sqrt(3.0) / 2, kRefPi};
-  const double mn[4] = {-1.0, -kRefPi, 0.0, -kRefPi};
-  for (int k = 0; k < 4; ++k)
-    if (t[k] > mx[k] || t[k] < mn[k]) return true;
-  return false;
+// ---- string fits (defects_3d.f90:435-603) ----
+//
+// The fit of one string cell is a random search over 1001 starts, which keeps
+// the kNumSimp + 1 best, followed by a Nelder-Mead simplex of up to 1000
+// iterations (tol 0.05 on chi2).  In evolved fields about two thirds of the
+// string cells never reach the tolerance and run all 1000 iterations, one or
+// two chi2 after another: a cell is a serial chain of about 2000 chi2, each of
+// 8 atan2 (one per corner) and 2 sin / cos.  With one lane per cell the chain
+// took 57 ms whatever the lattice, lanes of a warp diverged over the search
+// stages (12 of 32 active at 128^3), and every lane issued the FP64 work of
+// its own simplex.
+//
+// Here eight lanes fit one cell, lane `sub` = corner `sub`.  A chi2 is one
+// atan2 per lane; the terms go through shared memory and are added in the
+// reference's corner order.  Lane sub also holds coordinate sub & 3 of every
+// vertex (mu, phi, radius, angle), so the simplex arithmetic is one FP64
+// operation where a lane with a whole vertex issued four.  chi2 values are
+// kept as ordered integers (dkey): their comparisons stay off the FP64 pipe,
+// which GB300 issues at 1/64 of the FP32 rate.  Three kernels, so that the
+// lanes of a warp always run the same kind of work:
+//   k_string_start   the random search, eight starts screened at a time;
+//   k_string_simplex the simplex; groups take cells from a counter;
+//   k_string_result  one thread per cell: length, velocity and output row.
+// The whole search is bit-identical to the sequential one of the CPU
+// restatement.  String fits, ms: 104.5 -> 36.8 at 128^3 (1.3e5 cells, FP32),
+// 58.1 -> 12 at 64^3, 55 -> 5.2 at 32^3.  At 128^3 the issue slots bound it
+// (ncu at 64^3: 68 % issue active, FP64 pipe 37 %; about 800 instructions per
+// warp and chi2), on small lattices the chain of a cell.
+constexpr int kGrp = 8;                 // lanes per cell
+constexpr int kFitThreads = 128;        // 16 cells per CTA
+constexpr int kIdle = 2;                // groups of a warp without work that end the eight-lane simplex
+constexpr int kRounds = 4;              // random starts screened per lane before the next evaluations
+constexpr int kFitStride = 5 * 4 + 5;   // doubles per cell of the simplex scratch: p[vertex][coordinate], chi2[vertex]
+constexpr int64_t kFitChunk = 1 << 21;  // cells per pass of the three kernels (420 MB of scratch at most)
+
+// a double as an integer of the same order; -0 becomes +0.  An involution.
+__device__ __forceinline__ long long dkey(double v) {
+  const long long b = __double_as_longlong(v);
+  return b == (long long)0x8000000000000000ULL ? 0 : b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ double dkey_value(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
 }
 
-// Start point i of the random search (defects_3d.f90:463-470): four
-// uniforms from two Philox draws, mapped onto the parameter box.
-__device__ __forceinline__ void string_start(uint64_t seed, uint64_t cell, int i, double t[4]) {
-  const double max_s[4] = {1.0, kRefPi, sqrt(3.0) / 2, kRefPi};
-  const double min_s[4] = {-1.0, -kRefPi, 0.0, -kRefPi};
-  double x[4];
-  for (int k = 0; k < 4; k += 2) {
-    const int j = i * 4 + k;
-    const axd_u32x4 r = axd_draw(seed, 3u, (uint32_t)(j >> 1), cell);
-    x[k] = axd_u01(r.v[0], r.v[1]);
-    x[k + 1] = axd_u01(r.v[2], r.v[3]);
-  }
-  for (int k = 0; k < 4; ++k) t[k] = max_s[k] * x[k] + min_s[k] * (1 - x[k]);
+// bounds of parameter k (mu, phi, radius, angle)
+__device__ __forceinline__ double string_max(int k) {
+  return k == 0 ? 1.0 : (k == 2 ? sqrt(3.0) / 2 : kRefPi);
+}
+__device__ __forceinline__ double string_min(int k) { return k == 0 ? -1.0 : (k == 2 ? 0.0 : -kRefPi); }
+
+// Coordinate k of start point i of the random search (defects_3d.f90:
+// 463-470): two uniforms per Philox draw, mapped onto the parameter box.
+__device__ __forceinline__ double string_start(uint64_t seed, uint64_t cell, int i, int k) {
+  const axd_u32x4 r = axd_draw(seed, 3u, (uint32_t)((i * 4 + k) >> 1), cell);
+  const double x = (k & 1) ? axd_u01(r.v[2], r.v[3]) : axd_u01(r.v[0], r.v[1]);
+  return string_max(k) * x + string_min(k) * (1 - x);
 }
 
-// A lower bound of calc_chi2_string(ph, t) from an FP32 evaluation, or -inf
-// where the FP32 value cannot be bounded (a corner too close to the string
-// axis for its angle to be resolved, or a phase difference within the error
-// of the +-pi wrap).  Error budget, all generous:
-//   du, dv: angles and radius rounded to FP32, sqrt(1 - mu^2) from an FP64
-//           product, CUDA sincosf (2 ulp), products and sums of terms below
-//           2.4 in magnitude: |error| <= kDuv = 4e-6;
-//   angle : atan2f (3 ulp of pi) plus the rotation of (du, dv) by an error
-//           of kDuv at radius r: e = kAng + 2 kDuv / (r - 2 kDuv);
+// A lower bound of the chi2 of start i from an FP32 evaluation, or -inf where
+// the FP32 value cannot be bounded (a corner too close to the string axis for
+// its angle to be resolved, or a phase difference within the error of the
+// +-pi wrap).  The start is formed in FP32 too, from the top 32 bits of its
+// uniforms: x and 1 - x each to 2^-25 relative and 2^-32 absolute, so mu to
+// 2e-7, the angles to 7e-7, the radius to 1e-7, and sqrt(1 - mu^2) =
+// 2 sqrt(x (1 - x)) to 4e-7 (x within 2^-20 of 0 or 1 is not screened).
+// Error budget, all generous:
+//   du, dv: those, __sincosf (absolute error 2^-21 on [-pi, pi]), products
+//           and sums of terms below 2.4 in magnitude come to 3.1e-6:
+//           |error| <= kDuv = 5e-6;
+//   angle : the polynomial arctangent (Hastings' five terms, Abramowitz and
+//           Stegun 4.4.47: 1.16e-5 on [0, 1]; ratio and quadrant sums in
+//           FP32 below 6e-7) within kAng, plus the rotation of (du, dv) by an
+//           error of kDuv at radius r: e = kAng + 2 kDuv / (r - 2 kDuv).
+//           With atan2f the screens took 1.8 times the instructions, and a
+//           bound 3e-4 tighter in chi2 saves no evaluation;
 //   phase : FP32 rounding of ph, of the difference and of the wrap
 //           constants, within kPh = 2e-6;
 //   chi2  : a = <d^2> moves by at most (2 pi + E) E, b^2 = <d>^2 by at most
 //           (2 pi + E + 2e-6)(E + 2e-6), FP32 summation by below 2e-5;
-// and the total is doubled, plus 1e-4.
-//
-// Kept out of line: inlined into the search step (with its eight atan2f and
-// two sincosf) it made the string-fit loop's code outgrow the instruction
-// cache (ncu at 128^3: 9.1 "no instruction" stalls per issue); one copy took
-// the 128^3 fits from 152 to 106 ms.
-__device__ __noinline__ float chi2_string_lower(const float phf[8], const double t[4]) {
-  constexpr float kDuv = 4e-6f, kAng = 2e-6f, kPh = 2e-6f;
+// and the total is doubled, plus 1e-4 (which also covers the 1e-14 between
+// the FP64 chi2 and the float-float chi2 the search uses).
+__device__ __forceinline__ float chi2_start_lower(const float phf[8], uint64_t seed, uint64_t cell, int i) {
+  constexpr float kDuv = 5e-6f, kAng = 1.3e-5f, kPh = 2e-6f;
   constexpr float kPiF = (float)kRefPi, kTwoPiF = (float)kRefTwoPi;
-  const float mu = (float)t[0], ph = (float)t[1], rad = (float)t[2], ang = (float)t[3];
+  const axd_u32x4 r0 = axd_draw(seed, 3u, (uint32_t)(2 * i), cell), r1 = axd_draw(seed, 3u, (uint32_t)(2 * i + 1), cell);
+  const uint32_t xm = r0.v[0];
+  if (xm < 4096u || xm > 0xffffefffu) return -INFINITY;
+  constexpr float k32 = 2.3283064365386963e-10f;  // 2^-32
+  const float x0 = (float)xm * k32, y0 = (float)~xm * k32;
+  const float mu = x0 - y0, sm = 2 * sqrtf(x0 * y0);
+  const float ph = kTwoPiF * ((float)r0.v[2] * k32) - kPiF;
+  const float rad = 0.86602540378443864676f * ((float)r1.v[0] * k32);
+  const float ang = kTwoPiF * ((float)r1.v[2] * k32) - kPiF;
   float s4, c4, sp, cp;
-  sincosf(ang, &s4, &c4);
-  sincosf(ph, &sp, &cp);
-  // 1 - mu^2 is formed in FP64: for |mu| near 1 the FP32 rounding of mu
-  // alone would move sqrt(1 - mu^2) by up to 5e-4
-  const float u0 = rad * c4, v0 = rad * s4, sm = sqrtf((float)((1.0 - t[0]) * (1.0 + t[0])));
-  float a = 0.0f, b = 0.0f, E = 0.0f;
-  for (int iz = 0; iz <= 1; ++iz) {
-    const float z = iz - 0.5f;
-    for (int iy = 0; iy <= 1; ++iy) {
-      const float y = iy - 0.5f;
-      for (int ix = 0; ix <= 1; ++ix) {
-        const float x = ix - 0.5f;
-        const int i = (iz * 2 + iy) * 2 + ix;
-        const float du = -u0 + mu * (x * cp + y * sp) - z * sm;
-        const float dv = -v0 - x * sp + y * cp;
-        const float r = sqrtf(du * du + dv * dv);
-        if (!(r > 8 * kDuv)) return -INFINITY;
-        const float e = kAng + kPh + 2 * kDuv / (r - 2 * kDuv);
-        float d = phf[i] - atan2f(dv, du);
-        if (!(fabsf(fabsf(d) - kPiF) > e + kPh)) return -INFINITY;
-        if (d >= kPiF)
-          d = d - kTwoPiF;
-        else if (d < -kPiF)
-          d = d + kTwoPiF;
-        a = a + d * d;
-        b = b + d;
-        E = fmaxf(E, e);
-      }
-    }
+  __sincosf(ang, &s4, &c4);
+  __sincosf(ph, &sp, &cp);
+  const float u0 = rad * c4, v0 = rad * s4;
+  float a = 0.0f, b = 0.0f, rmin = INFINITY, wmin = INFINITY;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const float x = (c & 1) - 0.5f, y = ((c >> 1) & 1) - 0.5f, z = (c >> 2) - 0.5f;
+    const float du = -u0 + mu * (x * cp + y * sp) - z * sm;
+    const float dv = -v0 - x * sp + y * cp;
+    rmin = fminf(rmin, du * du + dv * dv);
+    const float au = fabsf(du), av = fabsf(dv);
+    const float q = __fdividef(fminf(au, av), fmaxf(au, av)), q2 = q * q;
+    float at = fmaf(q2, 0.0208351f, -0.0851330f);
+    at = fmaf(q2, at, 0.1801410f);
+    at = fmaf(q2, at, -0.3302995f);
+    at = q * fmaf(q2, at, 0.9998660f);
+    if (av > au) at = 1.5707963267948966f - at;
+    if (du < 0.0f) at = 3.1415926535897932f - at;
+    float d = phf[c] - copysignf(at, dv);
+    wmin = fminf(wmin, fabsf(fabsf(d) - kPiF));
+    if (d >= kPiF)
+      d = d - kTwoPiF;
+    else if (d < -kPiF)
+      d = d + kTwoPiF;
+    a = a + d * d;
+    b = b + d;
   }
+  // one E for all corners, from the smallest radius
+  const float r = sqrtf(rmin);
+  if (!(r > 8 * kDuv)) return -INFINITY;
+  const float E = kAng + kPh + 2 * kDuv / (r - 2 * kDuv);
+  if (!(wmin > E + kPh)) return -INFINITY;
   a = a / 8;
   b = b / 8;
   const float tp = (float)kRefTwoPi;
@@ -523,43 +572,265 @@ __device__ __noinline__ float chi2_string_lower(const float phf[8], const double
   return (a - b * b) - bound;
 }
 
-// defects_3d.f90:435-603, as a per-lane state machine.
-//
-// The fit of one string cell is a random search over 1001 starts followed by
-// a Nelder-Mead simplex of up to 1000 iterations (tol 0.05 on chi2).  In
-// evolved fields about two thirds of the string cells never reach the
-// tolerance and run all 1000 iterations.  Written as one loop per thread,
-// a warp ran its slowest cell's iteration count, and the expansion,
-// contraction and shrink branches one after another.  Here each lane holds
-// the search state of one cell and advances it to its next chi2
-// evaluation; every pass of the scheduling loop makes at most one chi2
-// evaluation per lane, at a lane-specific point, so the 8 atan2 of the
-// evaluations run on all active lanes together.  A lane whose cell is done
-// writes the cell's results and takes the next cell from a global counter.
-//
-// The random search keeps kNumSimp + 1 of the starts, in the order drawn.
-// Once that set is full, a start changes it only if its chi2 is at most the
-// value in the last slot.  That value can rise (the first two starts are
-// kept unsorted, defects_3d.f90:471-476, and a larger early value moves up
-// the list), but never above the largest value kept at any earlier time.
-// The starts are therefore screened with FP32 lower bounds
-// (chi2_string_lower) against the largest kept value; only the starts that
-// pass are evaluated, in draw order.  A screened-out start has a chi2 above
-// any threshold the sequential search could have compared it with (the
-// bound's 1e-4 margin covers the 1e-14 between the FP64 chi2 it was
-// derived for and the float-float chi2 the search uses).  Every chi2 that
-// enters a decision or the kept state is the float-float value of
-// axd_chi2_string_ff (axg_ffchi2.h), which the CPU restatement evaluates
-// too, so the fit is bit-identical to its sequential search.
-struct StringSearch {
-  double p_s[5][4], chi2_s[5], c_s[4], t_s[4], s_s[4], chi2;
-  int n0, i, it, stage;
-  bool expand;
+// sin (even lanes) or cos (odd lanes) of the reduced argument by the series of
+// axd_ff_sincos: the coefficients of the lane's series, float-float for the
+// first five terms and FP32 for the others, kept in registers.
+struct LaneSeries {
+  axd_ff k[5];
+  float f[4];
+  bool cosine;
+  __device__ explicit LaneSeries(bool c) : cosine(c) {
+    // (-1)^k / (2k+1)! and (-1)^k / (2k)!, as in axd_ff_sincos
+    const float ks[9][2] = {{1.0f, 0.0f},
+                            {-0.1666666716337204f, 4.967053879312289e-09f},
+                            {0.008333333767950535f, -4.34617203337595e-10f},
+                            {-0.00019841270113829523f, 2.725596874933456e-12f},
+                            {2.7557318844628753e-06f, 3.793571224297229e-14f},
+                            {-2.5052107943679403e-08f, 0.0f},
+                            {1.6059044372074283e-10f, 0.0f},
+                            {-7.647163609812713e-13f, 0.0f},
+                            {2.8114573589663704e-15f, 0.0f}};
+    const float kc[9][2] = {{1.0f, 0.0f},
+                            {-0.5f, 0.0f},
+                            {0.0416666679084301f, -1.2417634698280722e-09f},
+                            {-0.0013888889225199819f, 3.3631094437103215e-11f},
+                            {2.4801587642286904e-05f, -3.40699609366682e-13f},
+                            {-2.755731998149713e-07f, 0.0f},
+                            {2.0876755879584152e-09f, 0.0f},
+                            {-1.147074536050896e-11f, 0.0f},
+                            {4.7794772561329454e-14f, 0.0f}};
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      if (i < 5) k[i] = c ? axd_ff_mk(kc[i][0], kc[i][1]) : axd_ff_mk(ks[i][0], ks[i][1]);
+      else f[i - 5] = c ? kc[i][0] : ks[i][0];
+    }
+  }
+  // the series at r (r2 = r r), the operations of axd_ff_sincos
+  __device__ __forceinline__ axd_ff operator()(axd_ff r, axd_ff r2) const {
+    float q = f[3];
+#pragma unroll
+    for (int i = 2; i >= 0; --i) q = AXF_FMA(q, r2.h, f[i]);
+    axd_ff p = axd_ff_mk(q, 0.0f);
+#pragma unroll
+    for (int i = 4; i >= 0; --i) p = axd_ff_add(axd_ff_mul(p, r2), k[i]);
+    return axd_ff_mul(p, cosine ? axd_ff_mk(1.0f, 0.0f) : r);  // times (1, 0) is exact
+  }
 };
 
+// axd_chi2_string_ff by the eight lanes of a group, every lane returning it.
+// pc: the phase of corner `sub`; P: coordinate sub & 3 of the point.  All 32
+// lanes of the warp call it together (lanes without a point pass any finite
+// P).  Lanes 0-3 of the group reduce the angle, 4-7 phi, even lanes run the
+// sine series and odd lanes the cosine; each lane forms its corner's d and d^2; even lanes then add the eight d^2 and odd lanes
+// the eight d, in corner order, from shared memory (buf: the warp's 4 x 9
+// float4, the ninth keeping the groups on different banks).
+__device__ __forceinline__ double chi2_group(axd_ff pc, double P, int lane, float4 *buf, const LaneSeries &series) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const axd_ff refpi = axd_ff_mk(3.1415927410125732f, -8.742257051608249e-08f);
+  const axd_ff tworefpi = axd_ff_mk(6.2831854820251465f, -1.7484514103216497e-07f);
+  const int sub = lane & 7, base = lane & ~7;
+  auto from = [&](axd_ff v, int l) {
+    return axd_ff_mk(__shfl_sync(kAll, v.h, base + l), __shfl_sync(kAll, v.l, base + l));
+  };
+  const axd_ff p = axd_ff_from(P);
+  const axd_ff mu = from(p, 0), rad = from(p, 2), arg = from(p, sub < 4 ? 3 : 1);
+  axd_ff sc;  // sin (even lanes) or cos (odd lanes) of arg, as axd_ff_sincos
+  {
+    const float P1 = 1.5707963705062866f, P2 = -4.371138828673793e-08f, P3 = -1.7151245100058819e-15f;
+    const float kf = AXF_RINT(AXF_MUL(arg.h, 0.6366197723675814f));
+    axd_ff r = axd_ff_add(arg, axd_ff_mk(-AXF_MUL(kf, P1), 0.0f));
+    r = axd_ff_add(r, axd_ff_mk(-AXF_MUL(kf, P2), 0.0f));
+    r = axd_ff_add(r, axd_ff_mk(-AXF_MUL(kf, P3), 0.0f));
+    const int q = (int)kf & 3;
+    const axd_ff own = series(r, axd_ff_mul(r, r));
+    // arg = q pi/2 + r: for odd q the sine is the neighbour lane's cosine series and the other way round
+    const axd_ff other = axd_ff_mk(__shfl_xor_sync(kAll, own.h, 1), __shfl_xor_sync(kAll, own.l, 1));
+    sc = (q & 1) ? other : own;
+    if ((sub & 1) ? (q == 1 || q == 2) : (q == 2 || q == 3)) sc = axd_ff_neg(sc);
+  }
+  const axd_ff s4 = from(sc, 0), c4 = from(sc, 1), sp = from(sc, 4), cp = from(sc, 5);
+  const axd_ff u0 = axd_ff_mul(rad, c4), v0 = axd_ff_mul(rad, s4);
+  const axd_ff sm = axd_ff_sqrt(axd_ff_sub(axd_ff_mk(1.0f, 0.0f), axd_ff_mul(mu, mu)));
+  const axd_ff hcp = axd_ff_mulf(cp, 0.5f), hsp = axd_ff_mulf(sp, 0.5f), hsm = axd_ff_mulf(sm, 0.5f);
+  const int ix = sub & 1, iy = (sub >> 1) & 1, iz = sub >> 2;
+  const axd_ff xc = ix ? hcp : axd_ff_neg(hcp), ys = iy ? hsp : axd_ff_neg(hsp);
+  const axd_ff xs = ix ? hsp : axd_ff_neg(hsp), yc = iy ? hcp : axd_ff_neg(hcp);
+  const axd_ff zs = iz ? hsm : axd_ff_neg(hsm);
+  const axd_ff du = axd_ff_sub(axd_ff_add(axd_ff_neg(u0), axd_ff_mul(mu, axd_ff_add(xc, ys))), zs);
+  const axd_ff dv = axd_ff_add(axd_ff_sub(axd_ff_neg(v0), xs), yc);
+  axd_ff d = axd_ff_sub(pc, axd_ff_atan2(dv, du));
+  if (axd_ff_ge(d, refpi))
+    d = axd_ff_sub(d, tworefpi);
+  else if (axd_ff_gt(axd_ff_neg(refpi), d))
+    d = axd_ff_add(d, tworefpi);
+  const axd_ff d2 = axd_ff_mul(d, d);
+  float4 *gb = buf + (lane >> 3) * (kGrp + 1);
+  gb[sub] = make_float4(d2.h, d2.l, d.h, d.l);
+  __syncwarp();
+  const float2 *q = reinterpret_cast<const float2 *>(gb) + (sub & 1);
+  axd_ff acc = axd_ff_mk(0.0f, 0.0f);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float2 t = q[2 * i];
+    acc = axd_ff_add(acc, axd_ff_mk(t.x, t.y));
+  }
+  __syncwarp();
+  acc = axd_ff_mulf(acc, 0.125f);
+  const axd_ff a = from(acc, 0), b = from(acc, 1);
+  return axd_ff_to(axd_ff_sub(a, axd_ff_mul(b, b)));
+}
+
+// the corner phases of cell s: lane sub's corner
+__device__ __forceinline__ double corner_phase(const double *__restrict__ ph64, int n, int64_t s, int sub) {
+  const int ix = (int)(s % n), iy = (int)((s / n) % n), iz = (int)(s / ((int64_t)n * n));
+  return ph64[corner(n, ix, iy, iz, sub)];
+}
+
+// The random search of one cell per group (defects_3d.f90:460-500).  It keeps
+// kNumSimp + 1 starts in the order drawn; once that set is full, a start
+// changes it only if its chi2 is at most the value in the last slot.  That
+// value can rise (the first two starts are kept unsorted, defects_3d.f90:
+// 471-476, and a larger early value moves up the list), but never above the
+// largest value kept at any earlier time.  Each lane forms the FP32 lower
+// bounds of kRounds starts; those not above the largest kept value are
+// evaluated in draw order, each looked at again against the value kept by
+// then.  A screened-out start has a chi2 above any threshold the sequential
+// search could have compared it with.  About 30 of the 1001 are evaluated;
+// rounds of 32 starts let the warp's four groups evaluate theirs together.  out: p[vertex][coordinate], chi2[vertex] per cell.
+__global__ void __launch_bounds__(kFitThreads) k_string_start(const double *__restrict__ ph64, int n, uint64_t seed,
+                                                              const int64_t *__restrict__ cells, int64_t ncell,
+                                                              double *__restrict__ out) {
+  __shared__ float4 sbuf[kFitThreads / 32][4 * (kGrp + 1)];
+  const int lane = threadIdx.x & 31, sub = lane & 7, base = lane & ~7, k = sub & 3;
+  float4 *buf = sbuf[threadIdx.x >> 5];
+  const LaneSeries series(sub & 1);
+  const int64_t c = (int64_t)blockIdx.x * (kFitThreads / kGrp) + threadIdx.x / kGrp;
+  const bool live = c < ncell;
+  const int64_t s = cells[live ? c : ncell - 1];
+  const double pd = corner_phase(ph64, n, s, sub);
+  const axd_ff pc = axd_ff_from(pd);
+  float phf[8];
+  {
+    const float f = (float)pd;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) phf[i] = __shfl_sync(0xffffffffu, f, base + i);
+  }
+  // a corner phase that is no number makes every chi2 one: no comparison of
+  // the search holds, the first five starts stay and the simplex does not run
+  const bool bad = (__ballot_sync(0xffffffffu, isnan(pd)) >> base) & 0xff;
+  double p[kNumSimp + 1];
+  long long ch[kNumSimp + 1];
+  // the starts that fill the set, in the order of defects_3d.f90:471-490
+#pragma unroll
+  for (int i = 0; i <= kNumSimp; ++i) {
+    const double t = string_start(seed, (uint64_t)s, i, k);
+    const long long x = dkey(chi2_group(pc, t, lane, buf, series));
+    bool go = true;
+    if (i >= 2) {
+#pragma unroll
+      for (int q = i; q >= 1; --q) {
+        const bool move = go && !bad && x <= ch[q - 1];
+        if (move) {
+          ch[q] = ch[q - 1];
+          p[q] = p[q - 1];
+        } else if (go) {
+          ch[q] = x;
+          p[q] = t;
+          go = false;
+        }
+      }
+      if (go) {
+        ch[0] = x;
+        p[0] = t;
+      }
+    } else {
+      ch[i] = x;
+      p[i] = t;
+    }
+  }
+  for (int i0 = kNumSimp + 1; i0 <= kMaxIter; i0 += kRounds * kGrp) {
+    float lb[kRounds];
+#pragma unroll 1
+    for (int r = 0; r < kRounds; ++r) {
+      const int i = i0 + r * kGrp + sub;
+      const float v = i <= kMaxIter ? chi2_start_lower(phf, seed, (uint64_t)s, i) : INFINITY;
+#pragma unroll
+      for (int q = 0; q < kRounds; ++q)
+        if (q == r) lb[q] = v;
+    }
+    unsigned todo = 0xffffffffu;  // starts i0 + bit not yet passed over, in draw order
+    for (;;) {
+      long long top = ch[0];
+#pragma unroll
+      for (int q = 1; q <= kNumSimp; ++q) top = ch[q] > top ? ch[q] : top;
+      // (double)lb > top, as floats: lb exceeds top exactly when it exceeds top rounded down
+      const float thr = __double2float_rd(dkey_value(top));
+      unsigned m = 0;
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r)
+        m |= ((__ballot_sync(0xffffffffu, live && !bad && !(lb[r] > thr)) >> base) & 0xffu) << (kGrp * r);
+      m &= todo;
+      if (!__any_sync(0xffffffffu, m != 0)) break;
+      const int j = m ? __ffs(m) - 1 : 0;
+      todo = m ? (0xfffffffeu << j) : 0;
+      const double t = string_start(seed, (uint64_t)s, i0 + j, k);
+      const long long x = dkey(chi2_group(pc, t, lane, buf, series));
+      if (m && x <= ch[kNumSimp]) {
+        bool go = true;
+#pragma unroll
+        for (int q = kNumSimp; q >= 1; --q) {
+          const bool move = go && x <= ch[q - 1];
+          if (move) {
+            ch[q] = ch[q - 1];
+            p[q] = p[q - 1];
+          } else if (go) {
+            ch[q] = x;
+            p[q] = t;
+            go = false;
+          }
+        }
+        if (go) {
+          ch[0] = x;
+          p[0] = t;
+        }
+      }
+    }
+  }
+  if (live && sub < 4) {
+    double *o = out + c * kFitStride;
+#pragma unroll
+    for (int q = 0; q <= kNumSimp; ++q) {
+      o[4 * q + k] = p[q];
+      if (sub == 0) o[20 + q] = dkey_value(ch[q]);
+    }
+  }
+}
+
+// Orders the simplex by chi2 as the reference's bubble sort does (strict
+// comparisons, so equal values keep their order).  sorted: vertices 0..3 are
+// in order already and only the last one has to find its place.
+__device__ __forceinline__ void simplex_sort(double p[kNumSimp + 1], long long ch[kNumSimp + 1], bool sorted) {
+  auto order = [&](int m) {  // swap vertices m and m + 1 when out of order
+    const bool sw = ch[m] > ch[m + 1];
+    const double a = p[m];
+    p[m] = sw ? p[m + 1] : a;
+    p[m + 1] = sw ? a : p[m + 1];
+    const long long q = ch[m];
+    ch[m] = sw ? ch[m + 1] : q;
+    ch[m + 1] = sw ? q : ch[m + 1];
+  };
+  if (!sorted) {
+#pragma unroll
+    for (int i0 = kNumSimp - 1; i0 >= 1; --i0)
+#pragma unroll
+      for (int m = 0; m < i0; ++m) order(m);
+  }
+#pragma unroll
+  for (int m = kNumSimp - 1; m >= 0; --m) order(m);
+}
+
 enum : int {
-  kSearch = 0,
-  kNmStart,
+  kNmStart = 0,
   kNmReflect,
   kNmSecondPrep,
   kNmSecond,
@@ -568,182 +839,169 @@ enum : int {
   kFinished
 };
 
-__device__ __forceinline__ void search_init(StringSearch &S) {
-  for (int a = 0; a < 5; ++a) {
-    S.chi2_s[a] = 0.0;
-    for (int k = 0; k < 4; ++k) S.p_s[a][k] = 0.0;
-  }
-  S.n0 = -1;
-  S.i = 0;
-  S.it = 0;
-  S.stage = kSearch;
-  S.expand = false;
-  S.chi2 = 0.0;
-}
-
-// the random-search bookkeeping of one exactly evaluated start (t_s, chi2)
-__device__ __forceinline__ void search_insert(StringSearch &S, double chi2) {
-  if (S.n0 <= 0) {
-    S.n0 = S.n0 + 1;
-    S.chi2_s[S.n0] = chi2;
-    for (int k = 0; k < 4; ++k) S.p_s[S.n0][k] = S.t_s[k];
-    return;
-  }
-  if (S.n0 < kNumSimp || chi2 <= S.chi2_s[S.n0]) {
-    S.n0 = S.n0 + 1 < kNumSimp ? S.n0 + 1 : kNumSimp;
-    int i0 = S.n0;
-    while (chi2 <= S.chi2_s[i0 - 1]) {
-      if (i0 <= kNumSimp) {
-        S.chi2_s[i0] = S.chi2_s[i0 - 1];
-        for (int k = 0; k < 4; ++k) S.p_s[i0][k] = S.p_s[i0 - 1][k];
-      }
-      i0 = i0 - 1;
-      if (i0 == 0) break;
-    }
-    S.chi2_s[i0] = chi2;
-    for (int k = 0; k < 4; ++k) S.p_s[i0][k] = S.t_s[k];
-  }
-}
-
-// the expansion / contraction decision with the second point's chi2
-__device__ __forceinline__ void search_second(StringSearch &S, double chi2s) {
-  if (S.expand) {
-    if (S.chi2 <= chi2s) {
-      S.chi2_s[kNumSimp] = S.chi2;
-      for (int k = 0; k < 4; ++k) S.p_s[kNumSimp][k] = S.t_s[k];
+// The Nelder-Mead simplex (defects_3d.f90:501-603), one cell per group, as a
+// state machine that advances to its next chi2: every pass of the loop
+// evaluates one chi2 per group, together for the warp's four groups, and a
+// group whose cell is done takes the next from *next (zero at launch).  The
+// grid is sized to the resident CTAs.  sim: as k_string_start leaves it; the
+// best vertex and its chi2 come back in its first row.
+__global__ void __launch_bounds__(kFitThreads, 6) k_string_simplex(const double *__restrict__ ph64, int n,
+                                                                const int64_t *__restrict__ cells, int64_t ncell,
+                                                                double *__restrict__ sim,
+                                                                unsigned long long *__restrict__ next,
+                                                                int2 *__restrict__ rest, unsigned *__restrict__ nrest) {
+  __shared__ float4 sbuf[kFitThreads / 32][4 * (kGrp + 1)];
+  const int lane = threadIdx.x & 31, sub = lane & 7, base = lane & ~7, k = sub & 3;
+  const unsigned gmask = 0xffu << base;
+  float4 *buf = sbuf[threadIdx.x >> 5];
+  const LaneSeries series(sub & 1);
+  const long long kmax = dkey(string_max(k)), kmin = dkey(string_min(k));
+  const long long chi2max = dkey(8 * kRefPi * kRefPi), tol = dkey(0.05);
+  double p[kNumSimp + 1] = {}, sum = 0.0, t = 0.0, s2 = 0.0, P = 0.0;
+  long long ch[kNumSimp + 1] = {}, x = 0;  // x: chi2 of the reflected point
+  axd_ff pc = axd_ff_mk(0.0f, 0.0f);
+  int64_t c = 0;
+  int stage = kFinished, it = 0;
+  bool expand = false, done = false, sorted = false;  // sorted: vertices 0..3 are in order
+  unsigned idle = 0;                                  // lanes whose group is done
+  auto outside = [&](double v) {  // any coordinate out of the box
+    const long long q = dkey(v);
+    return (__ballot_sync(gmask, q > kmax || q < kmin)) != 0;
+  };
+  // the expansion / contraction decision with the second point's chi2
+  auto second = [&](long long xs) {
+    if (expand) {
+      const bool first = x <= xs;
+      ch[kNumSimp] = first ? x : xs;
+      p[kNumSimp] = first ? t : s2;
+      stage = kNmSort;
+    } else if (xs <= ch[kNumSimp]) {
+      ch[kNumSimp] = xs;
+      p[kNumSimp] = s2;
+      stage = kNmSort;
     } else {
-      S.chi2_s[kNumSimp] = chi2s;
-      for (int k = 0; k < 4; ++k) S.p_s[kNumSimp][k] = S.s_s[k];
+      stage = kShrink1;
     }
-    S.stage = kNmSort;
-  } else if (chi2s <= S.chi2_s[kNumSimp]) {
-    S.chi2_s[kNumSimp] = chi2s;
-    for (int k = 0; k < 4; ++k) S.p_s[kNumSimp][k] = S.s_s[k];
-    S.stage = kNmSort;
-  } else {
-    S.stage = kShrink1;
-  }
-}
-
-// Advance S to its next chi2 evaluation; true with the point in P, false
-// when the lane has none this pass (screening budget spent, or finished).
-__device__ bool search_prepare(StringSearch &S, const float phf[8], uint64_t seed, uint64_t cell, double P[4],
-                               int screen) {
-  const double chi2max = 8 * kRefPi * kRefPi, tol = 0.05;
+  };
+  auto fetch = [&]() {
+    unsigned long long q = 0;
+    if (sub == 0) q = atomicAdd(next, 1ull);
+    c = (int64_t)__shfl_sync(gmask, q, base);
+    if (c >= ncell) {
+      done = true;
+      return;
+    }
+    const double pd = corner_phase(ph64, n, cells[c], sub);
+    pc = axd_ff_from(pd);
+    const double *o = sim + c * kFitStride;
+#pragma unroll
+    for (int q2 = 0; q2 <= kNumSimp; ++q2) {
+      p[q2] = o[4 * q2 + k];
+      ch[q2] = dkey(o[20 + q2]);
+    }
+    it = 0;
+    sorted = false;  // the random search leaves its first two starts as drawn
+    // a chi2 that is no number compares false with the tolerance
+    stage = isnan(o[20]) ? kFinished : kNmStart;
+  };
+  // an iteration's start with the queue empty and kIdle groups of the warp
+  // done: the rest of this cell goes to k_string_simplex_warp
+  auto hand_over = [&]() {
+    if (__popc(idle) < kIdle * kGrp) return false;
+    double *o = sim + c * kFitStride;
+#pragma unroll
+    for (int q2 = 0; q2 <= kNumSimp; ++q2) {
+      if (sub < 4) o[4 * q2 + k] = p[q2];
+      if (sub == 0) o[20 + q2] = dkey_value(ch[q2]);
+    }
+    if (sub == 0) rest[atomicAdd(nrest, 1u)] = make_int2((int)c, it);
+    done = true;
+    return true;
+  };
+  fetch();
   for (;;) {
-    if (S.stage == kSearch) {
-      if (S.i > kMaxIter) {
-        S.stage = kNmStart;
-        continue;
+    idle = __ballot_sync(0xffffffffu, done);
+    while (!done) {  // to the next chi2, or the next cell
+      if (stage == kNmSort) {
+        simplex_sort(p, ch, sorted);
+        sorted = true;
+        stage = kNmStart;
       }
-      if (S.n0 < kNumSimp) {  // filling the kept set: no screen
-        string_start(seed, cell, S.i, S.t_s);
-        for (int k = 0; k < 4; ++k) P[k] = S.t_s[k];
-        return true;
-      }
-      double thr = S.chi2_s[0];
-      for (int k = 1; k <= kNumSimp; ++k) thr = S.chi2_s[k] > thr ? S.chi2_s[k] : thr;
-      for (int k = 0; k <= kNumSimp; ++k)
-        if (S.chi2_s[k] != S.chi2_s[k]) thr = INFINITY;
-      for (int cnt = 0; cnt < screen && S.i <= kMaxIter; ++cnt) {
-        string_start(seed, cell, S.i, S.t_s);
-        if (!((double)chi2_string_lower(phf, S.t_s) > thr)) {
-          for (int k = 0; k < 4; ++k) P[k] = S.t_s[k];
-          return true;
+      if (stage == kNmStart) {
+        if (ch[0] > tol && it < kMaxIter) {
+          if (hand_over()) continue;
+          ++it;
+          sum = ((0.0 + p[0]) + p[1]) + p[2] + p[3];
+        } else {
+          stage = kFinished;
         }
-        S.i = S.i + 1;
       }
-      if (S.i > kMaxIter) {
-        S.stage = kNmStart;
-        continue;
+      if (stage == kNmStart || stage == kNmSecondPrep) {
+        // with the centroid c = sum / 4: the reflected point 2 c - p, the
+        // expansion 3 c - 4 p or the contraction 1.5 c - 0.5 p.  Scaling by
+        // a power of two is exact, so a sum rounds as a multiple of c does.
+        static_assert(kNumSimp == 4, "the centroid scaling is 1 / kNumSimp");
+        const bool reflect = stage == kNmStart;
+        if (!reflect) expand = x < ch[kNumSimp];
+        const double alpha = reflect ? 0.5 : (expand ? 0.75 : 0.375), beta = reflect ? 1.0 : (expand ? 4.0 : 0.5);
+        const double v = alpha * sum - axg_mul_pow2(p[kNumSimp], beta);
+        const bool out = outside(v);
+        if (reflect) {
+          t = v;
+          stage = out ? kNmSecondPrep : kNmReflect;
+          x = out ? chi2max : x;
+        } else {
+          s2 = v;
+          stage = kNmSecond;
+          if (out) second(chi2max);
+        }
+        if (!out) {
+          P = v;
+          break;
+        }
       }
-      return false;
-    }
-    if (S.stage == kNmStart) {
-      if (!(S.chi2_s[0] > tol && S.it < kMaxIter)) {
-        S.stage = kFinished;
-        return false;
-      }
-      S.it = S.it + 1;
-      for (int k = 0; k < 4; ++k) S.c_s[k] = 0.0;
-      for (int i0 = 0; i0 < kNumSimp; ++i0)
-        for (int k = 0; k < 4; ++k) S.c_s[k] = S.c_s[k] + S.p_s[i0][k];
-      static_assert(kNumSimp == 4, "the centroid scaling below is 1 / kNumSimp");
-      for (int k = 0; k < 4; ++k) S.c_s[k] = S.c_s[k] * 0.25;  // exact: the same value as / kNumSimp
-      for (int k = 0; k < 4; ++k) S.t_s[k] = 2 * S.c_s[k] - S.p_s[kNumSimp][k];
-      if (out_of_box(S.t_s)) {
-        S.chi2 = chi2max;
-        S.stage = kNmSecondPrep;
-        continue;
-      }
-      for (int k = 0; k < 4; ++k) P[k] = S.t_s[k];
-      S.stage = kNmReflect;
-      return true;
-    }
-    if (S.stage == kNmSecondPrep) {
-      S.expand = S.chi2 < S.chi2_s[kNumSimp];
-      if (S.expand)
-        for (int k = 0; k < 4; ++k) S.s_s[k] = 3 * S.c_s[k] - 4 * S.p_s[kNumSimp][k];
-      else
-        for (int k = 0; k < 4; ++k) S.s_s[k] = 1.5 * S.c_s[k] - 0.5 * S.p_s[kNumSimp][k];
-      if (out_of_box(S.s_s)) {
-        search_second(S, chi2max);
-        continue;
-      }
-      for (int k = 0; k < 4; ++k) P[k] = S.s_s[k];
-      S.stage = kNmSecond;
-      return true;
-    }
-    if (S.stage == kNmSort) {
-      for (int i0 = kNumSimp - 1; i0 >= 0; --i0)
-        for (int m = 0; m <= i0; ++m)
-          if (S.chi2_s[m] > S.chi2_s[m + 1]) {
-            for (int k = 0; k < 4; ++k) {
-              const double tt = S.p_s[m][k];
-              S.p_s[m][k] = S.p_s[m + 1][k];
-              S.p_s[m + 1][k] = tt;
-            }
-            const double c = S.chi2_s[m];
-            S.chi2_s[m] = S.chi2_s[m + 1];
-            S.chi2_s[m + 1] = c;
+      if (stage >= kShrink1 && stage < kNmSort) {  // shrink towards the best vertex
+        const int j = stage - kShrink1 + 1;
+#pragma unroll
+        for (int q = 1; q <= kNumSimp; ++q)
+          if (q == j) {
+            p[q] = axg_mul_pow2(p[q] + p[0], 0.5);
+            P = p[q];
           }
-      S.stage = kNmStart;
-      continue;
+        sorted = false;
+        break;
+      }
+      if (stage == kFinished) {
+        double *o = sim + c * kFitStride;
+        if (sub < 4) o[k] = p[0];
+        if (sub == 0) o[20] = dkey_value(ch[0]);
+        fetch();
+      }
     }
-    if (S.stage >= kShrink1 && S.stage < kNmSort) {  // shrink towards the best vertex
-      const int j = S.stage - kShrink1 + 1;
-      for (int k = 0; k < 4; ++k) S.p_s[j][k] = 0.5 * (S.p_s[j][k] + S.p_s[0][k]);
-      for (int k = 0; k < 4; ++k) P[k] = S.p_s[j][k];
-      return true;
+    __syncwarp();
+    if (__all_sync(0xffffffffu, done)) break;
+    const long long v = dkey(chi2_group(pc, P, lane, buf, series));
+    if (stage == kNmReflect) {
+      x = v;
+      stage = kNmSecondPrep;
+    } else if (stage == kNmSecond) {
+      second(v);
+    } else if (!done) {
+      const int j = stage - kShrink1 + 1;
+#pragma unroll
+      for (int q = 1; q <= kNumSimp; ++q)
+        if (q == j) ch[q] = v;
+      stage = j < kNumSimp ? stage + 1 : kNmSort;
     }
-    return false;  // kFinished
-  }
-}
-
-// S takes the chi2 of the point search_prepare returned
-__device__ void search_consume(StringSearch &S, double v) {
-  if (S.stage == kSearch) {
-    search_insert(S, v);
-    S.i = S.i + 1;
-  } else if (S.stage == kNmReflect) {
-    S.chi2 = v;
-    S.stage = kNmSecondPrep;
-  } else if (S.stage == kNmSecond) {
-    search_second(S, v);
-  } else {
-    const int j = S.stage - kShrink1 + 1;
-    S.chi2_s[j] = v;
-    S.stage = j < kNumSimp ? S.stage + 1 : kNmSort;
   }
 }
 
 // position, direction, goodness of fit and length from the best vertex
-__device__ void string_result(const StringSearch &S, double pos[3], double dir[3], double *gof, double *sl) {
-  const double mu = S.p_s[0][0], phi = S.p_s[0][1];
+__device__ void string_result(const double p[4], double chi2, double pos[3], double dir[3], double *gof, double *sl) {
+  const double mu = p[0], phi = p[1];
   double s4, c4, sp, cp;
-  axd_sincos(S.p_s[0][3], &s4, &c4);
-  const double u0 = S.p_s[0][2] * c4, v0 = S.p_s[0][2] * s4;
-  const double chi2 = S.chi2_s[0];
+  axd_sincos(p[3], &s4, &c4);
+  const double u0 = p[2] * c4, v0 = p[2] * s4;
   axd_sincos(phi, &sp, &cp);
   const double sq = sqrt(1.0 - mu * mu);
   dir[0] = sq * cp;
@@ -930,18 +1188,22 @@ __device__ void wall_grid_fill(WallGrid &g) {
 
 // The direction search of position_wall screened in FP32.  Per direction
 // the reference forms d_i = pp_i . d0, W = sum d_i, S = sum d_i^2 and
-// chi2 = S - m w^2 with w = max(W, 0) / m, i.e. chi2 = S - max(W, 0)^2 / m.
-// With |pp| < 0.87 (each component in (-0.5, 0.5)), |d0| = 1 and m <= 12,
-// the FP32 value differs from the FP64 one by less than kWallScreenErr:
-// inputs rounded to FP32 and three products and two sums move d by < 5e-7,
-// so W by < 1.3e-5 and S by < 2e-5; max(W, 0)^2 / m is Lipschitz in W
-// (either branch of the reference's w < 0 test), < 9e-5 for |W| <= 10.4;
-// the remaining roundings are below 1e-5.  The FP32 error is thus below
-// 1.3e-4; the screen allows 1e-3.  A direction whose FP32 value exceeds the
-// smallest FP32 value by more than twice that cannot hold the FP64 minimum,
-// so evaluating only the others in FP64, in the reference's loop order and
-// with its strict-less update, selects the same direction and w.
-constexpr float kWallScreenErr = 1e-3f;
+// chi2 = S - m w^2 with w = max(W, 0) / m.  With the points' mean c and
+// q_i = pp_i - c that is
+//   chi2 = sum (q_i . d0)^2 + m min(c . d0, 0)^2,
+// a sum of squares without cancellation, so its FP32 value is good to a few
+// ulp of chi2 itself.  q_i and c are formed in FP64 and rounded; with
+// |q_i| < 1.8, |d0| = 1 and m <= 12 a projection is off by less than 7e-7
+// (2^-24 for each factor and operation), so the sum of squares by less than
+// 2 sqrt(12 chi2) 7e-7 + 6e-12, the second term by 2e-6 sqrt(chi2), and the
+// FP32 summation by 1.5e-6 chi2; kWallErr covers their sum.  A direction whose
+// FP32 value exceeds the smallest one by more than both errors cannot hold
+// the FP64 minimum, so evaluating only the others in FP64, in the reference's
+// loop order and with its strict-less update, selects the same direction and
+// w.  (Screened as S - max(W, 0)^2 / m, whose error is 1e-4 of S, cells with
+// close crossing points kept tens of directions, and a warp evaluated ~85 of
+// them in FP64 one after another.)
+__device__ __forceinline__ float wall_err(float f) { return 1e-5f * sqrtf(f) + 2e-6f * f + 1e-10f; }
 
 __device__ void position_wall(const double ph[8], const WallGrid &grid, double pos[3], double dir[3], double *gof,
                               double *wa) {
@@ -984,49 +1246,77 @@ __device__ void position_wall(const double ph[8], const WallGrid &grid, double p
     *wa = 0.0;
     return;
   }
-  float ppf[12][3];
-  for (int i = 0; i < m; ++i)
-    for (int k = 0; k < 3; ++k) ppf[i][k] = (float)pp[i][k];
+  // the centred points in FP32 registers; those past m are zero and add
+  // nothing (indexed by a loop over m they lived in local memory, and the 800
+  // screens of a cell waited on its loads)
+  double cen[3];
+  for (int k = 0; k < 3; ++k) {
+    cen[k] = 0.0;
+    for (int i = 0; i < m; ++i) cen[k] = cen[k] + pp[i][k];
+    cen[k] = cen[k] / m;
+  }
+  const float c0 = (float)cen[0], c1 = (float)cen[1], c2 = (float)cen[2];
+  float q[12][3];
+#pragma unroll
+  for (int i = 0; i < 12; ++i)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) q[i][k] = i < m ? (float)(pp[i][k] - cen[k]) : 0.0f;
   auto screen = [&](int idx) {
-    const float *g = grid.f[idx];
-    float W = 0.0f, S = 0.0f;
-    for (int i = 0; i < m; ++i) {
-      const float d = ppf[i][0] * g[0] + ppf[i][1] * g[1] + ppf[i][2] * g[2];
-      W += d;
-      S += d * d;
+    const float g0 = grid.f[idx][0], g1 = grid.f[idx][1], g2 = grid.f[idx][2];
+    const float w = fminf(fmaf(c2, g2, fmaf(c1, g1, c0 * g0)), 0.0f);
+    float f = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) {
+      const float d = fmaf(q[i][2], g2, fmaf(q[i][1], g1, q[i][0] * g0));
+      f = fmaf(d, d, f);
     }
-    const float wp = fmaxf(W, 0.0f);
-    return S - wp * wp / (float)m;
+    return fmaf((float)m * w, w, f);
   };
   float fmin = INFINITY;
   for (int idx = 0; idx < 400; ++idx) fmin = fminf(fmin, screen(idx));
-  const float fcut = fmin + 2 * kWallScreenErr;
-  double chi2min = 6.0, mut = 0.0, phit = 0.0, wt = 0.0;
-  for (int imu = 1; imu <= 20; ++imu) {
-    for (int iphi = 1; iphi <= 20; ++iphi) {
-      if (!(screen((imu - 1) * 20 + (iphi - 1)) <= fcut)) continue;
-      const double *d0 = grid.d0[(imu - 1) * 20 + (iphi - 1)];
-      const double mu = d0[2], phi = d0[3];
-      double w = 0.0, chi2 = 0.0;
-      for (int i = 0; i < m; ++i) {
-        double d = pp[i][0] * d0[0] + pp[i][1] * d0[1];
-        d = d + pp[i][2] * d0[2];
-        w = w + d;
-        chi2 = chi2 + d * d;
-      }
-      if (w < 0.0)
-        w = 0.0;
-      else
-        w = w / m;
-      chi2 = chi2 - m * w * w;
-      if (chi2 < chi2min) {
-        chi2min = chi2;
-        mut = mu;
-        phit = phi;
-        wt = w;
-      }
+  const float fcut = fmin + wall_err(fmin);
+  auto kept = [&](int idx) {
+    const float f = screen(idx);
+    return f - wall_err(f) <= fcut;
+  };
+  // the directions to evaluate, in the reference's loop order: listed first
+  // and then evaluated one per lane at a time, so that the FP64 work of the
+  // warp's cells runs together (evaluated where the screen found them, each
+  // of a warp's candidates issued it alone)
+  constexpr int kCand = 8;
+  uint16_t cand[kCand];
+  int ncand = 0;
+  for (int idx = 0; idx < 400; ++idx)
+    if (kept(idx)) {
+      if (ncand < kCand) cand[ncand] = (uint16_t)idx;
+      ++ncand;
     }
-  }
+  double chi2min = 6.0, mut = 0.0, phit = 0.0, wt = 0.0;
+  auto evaluate = [&](int idx) {
+    const double *d0 = grid.d0[idx];
+    double w = 0.0, chi2 = 0.0;
+    for (int i = 0; i < m; ++i) {
+      double d = pp[i][0] * d0[0] + pp[i][1] * d0[1];
+      d = d + pp[i][2] * d0[2];
+      w = w + d;
+      chi2 = chi2 + d * d;
+    }
+    if (w < 0.0)
+      w = 0.0;
+    else
+      w = w / m;
+    chi2 = chi2 - m * w * w;
+    if (chi2 < chi2min) {
+      chi2min = chi2;
+      mut = d0[2];
+      phit = d0[3];
+      wt = w;
+    }
+  };
+  for (int c = 0; c < ncand && c < kCand; ++c) evaluate(cand[c]);
+  if (ncand > kCand)  // a flat minimum: the rest as found
+    for (int idx = cand[kCand - 1] + 1; idx < 400; ++idx)
+      if (kept(idx)) evaluate(idx);
   double spt, cpt;
   axd_sincos(phit, &spt, &cpt);
   const double sqt = sqrt(1 - mut * mut);
@@ -1087,72 +1377,111 @@ __device__ void position_wall(const double ph[8], const WallGrid &grid, double p
   *wa = area;
 }
 
-// FP32 screens per start-phase pass of a lane (search_prepare): a pass
-// screens at most this many random starts, so lanes in the start phase hold
-// the warp's Nelder-Mead lanes back for a few FP32 bounds only (8 measured
-// fastest of 2..32 at 128^3).
-constexpr int kScreenPerPass = 8;
-
-// String fits, lane-scheduled: each lane takes cells from *next (zero at
-// launch) and advances its search one chi2 evaluation per pass (see
-// search_prepare); the grid is sized to the resident CTAs.  The float-float
-// chi2 is a long chain of dependent FP32 operations, so the kernel is bound
-// by latency: capped at 96 registers (a few spills) it holds 5 CTAs per SM
-// instead of 3 (128^3: 237 -> 158 ms; 4, 6 and 8 CTAs measured slower).
-template <typename V>
-__global__ void __launch_bounds__(128, 5) k_string_fit(const V *__restrict__ phi, const V *__restrict__ cphi,
-                                                    const double *__restrict__ ph64, const V *__restrict__ phid, int n,
-                                                    double dspa, uint64_t seed, const int64_t *__restrict__ cells,
-                                                    int64_t ncell, double *__restrict__ out,
-                                                    unsigned long long *__restrict__ next) {
-  StringSearch S;
-  axd_ff pcf[8];  // corner phases as float-float pairs (the chi2 runs in float-float)
-  float phf[8];
-  int64_t k = -1, s = 0;
-  auto fetch = [&]() {
-    k = (int64_t)atomicAdd(next, 1ull);
-    if (k >= ncell) {
-      k = -1;
-      return;
-    }
-    s = cells[k];
-    const int ix = (int)(s % n), iy = (int)((s / n) % n), iz = (int)(s / ((int64_t)n * n));
-    for (int c = 0; c < 8; ++c) {
-      const double pc = ph64[corner(n, ix, iy, iz, c)];
-      pcf[c] = axd_ff_from(pc);
-      phf[c] = (float)pc;
-    }
-    search_init(S);
-  };
-  fetch();
+// The simplex with a warp per cell, for the cells left when the queue of
+// k_string_simplex runs dry and for lattices with few of them: then the serial
+// chain of chi2 sets the time.  The four groups evaluate an iteration's
+// reflected, expanded and contracted points at once (the two that the
+// sequential search would not have asked for are dropped), and the four
+// vertices of a shrink, so an iteration is one chi2 long instead of two to
+// six.  list: (cell, iterations done), or null for cells 0 .. *count - 1.
+__global__ void __launch_bounds__(kFitThreads, 6) k_string_simplex_warp(const double *__restrict__ ph64, int n,
+                                                                     const int64_t *__restrict__ cells,
+                                                                     const int2 *__restrict__ list,
+                                                                     const unsigned *__restrict__ count, int64_t ncell,
+                                                                     double *__restrict__ sim,
+                                                                     unsigned long long *__restrict__ next) {
+  __shared__ float4 sbuf[kFitThreads / 32][4 * (kGrp + 1)];
+  const int lane = threadIdx.x & 31, sub = lane & 7, k = sub & 3, g = lane >> 3;
+  float4 *buf = sbuf[threadIdx.x >> 5];
+  const LaneSeries series(sub & 1);
+  const long long kmax = dkey(string_max(k)), kmin = dkey(string_min(k));
+  const long long chi2max = dkey(8 * kRefPi * kRefPi), tol = dkey(0.05);
+  if (list) ncell = *count;
   for (;;) {
-    if (k >= 0 && S.stage == kFinished) {
-      const int ix = (int)(s % n), iy = (int)((s / n) % n), iz = (int)(s / ((int64_t)n * n));
-      double pos[3], dir[3], vel[3], gof, l;
-      string_result(S, pos, dir, &gof, &l);
-      velocity_string(phi, cphi, phid, n, dspa, ix, iy, iz, pos, vel);
-      double *r = out + 13 * k;
-      r[0] = pos[0] + ix + 0.5;
-      r[1] = pos[1] + iy + 0.5;
-      r[2] = pos[2] + iz + 0.5;
-      r[3] = dir[0];
-      r[4] = dir[1];
-      r[5] = dir[2];
-      r[6] = vel[0];
-      r[7] = vel[1];
-      r[8] = vel[2];
-      r[9] = gof;
-      r[10] = l;
-      r[11] = (double)s;
-      r[12] = -1.0;
-      fetch();
+    unsigned long long q = 0;
+    if (lane == 0) q = atomicAdd(next, 1ull);
+    q = __shfl_sync(0xffffffffu, q, 0);
+    if ((int64_t)q >= ncell) return;
+    const int64_t c = list ? list[q].x : (int64_t)q;
+    int it = list ? list[q].y : 0;
+    const axd_ff pc = axd_ff_from(corner_phase(ph64, n, cells[c], sub));
+    double *o = sim + c * kFitStride;
+    double p[kNumSimp + 1];
+    long long ch[kNumSimp + 1];
+#pragma unroll
+    for (int v = 0; v <= kNumSimp; ++v) {
+      p[v] = o[4 * v + k];
+      ch[v] = dkey(o[20 + v]);
     }
-    if (__all_sync(0xffffffffu, k < 0)) break;
-    double P[4];
-    const bool need = k >= 0 && search_prepare(S, phf, seed, (uint64_t)s, P, kScreenPerPass);
-    __syncwarp();
-    if (need) search_consume(S, axd_chi2_string_ff(pcf, P));
+    if (isnan(o[20])) continue;  // a chi2 that is no number compares false with the tolerance
+    bool sorted = false;
+    for (; ch[0] > tol && it < kMaxIter; ++it) {
+      const double sum = ((0.0 + p[0]) + p[1]) + p[2] + p[3];
+      // group 0: reflected, 1: expanded, 2: contracted (3: contracted, unused);
+      // the scalings of k_string_simplex
+      const double alpha = g == 0 ? 0.5 : (g == 1 ? 0.75 : 0.375), beta = g == 0 ? 1.0 : (g == 1 ? 4.0 : 0.5);
+      const double pt = alpha * sum - axg_mul_pow2(p[kNumSimp], beta);
+      const long long q = dkey(pt);
+      const unsigned out = __ballot_sync(0xffffffffu, q > kmax || q < kmin);
+      long long v = dkey(chi2_group(pc, pt, lane, buf, series));
+      if ((out >> (lane & ~7)) & 0xff) v = chi2max;
+      const long long x = __shfl_sync(0xffffffffu, v, 0), xe = __shfl_sync(0xffffffffu, v, 8),
+                      xc = __shfl_sync(0xffffffffu, v, 16);
+      const double t = __shfl_sync(0xffffffffu, pt, k), te = __shfl_sync(0xffffffffu, pt, 8 + k),
+                   tc = __shfl_sync(0xffffffffu, pt, 16 + k);
+      if (x < ch[kNumSimp]) {
+        const bool first = x <= xe;
+        ch[kNumSimp] = first ? x : xe;
+        p[kNumSimp] = first ? t : te;
+      } else if (xc <= ch[kNumSimp]) {
+        ch[kNumSimp] = xc;
+        p[kNumSimp] = tc;
+      } else {  // shrink towards the best vertex, group g vertex g + 1
+#pragma unroll
+        for (int v2 = 1; v2 <= kNumSimp; ++v2) p[v2] = axg_mul_pow2(p[v2] + p[0], 0.5);
+        const double own = g == 0 ? p[1] : (g == 1 ? p[2] : (g == 2 ? p[3] : p[4]));
+        const long long w = dkey(chi2_group(pc, own, lane, buf, series));
+#pragma unroll
+        for (int v2 = 1; v2 <= kNumSimp; ++v2) ch[v2] = __shfl_sync(0xffffffffu, w, 8 * (v2 - 1));
+        sorted = false;
+      }
+      simplex_sort(p, ch, sorted);
+      sorted = true;
+    }
+    if (lane < 4) o[k] = p[0];
+    if (lane == 0) o[20] = dkey_value(ch[0]);
   }
+}
+
+// Length, velocity and output row of the fitted string cells, one thread per
+// cell (a group of eight lanes per cell would issue their long FP64 chains for
+// one cell at a time).
+template <typename V>
+__global__ void __launch_bounds__(128) k_string_result(const V *__restrict__ phi, const V *__restrict__ cphi,
+                                                       const V *__restrict__ phid, int n, double dspa,
+                                                       const int64_t *__restrict__ cells, int64_t ncell,
+                                                       const double *__restrict__ sim, double *__restrict__ out) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= ncell) return;
+  const int64_t s = cells[k];
+  const int ix = (int)(s % n), iy = (int)((s / n) % n), iz = (int)(s / ((int64_t)n * n));
+  double pos[3], dir[3], vel[3], gof, l;
+  string_result(sim + k * kFitStride, sim[k * kFitStride + 20], pos, dir, &gof, &l);
+  velocity_string(phi, cphi, phid, n, dspa, ix, iy, iz, pos, vel);
+  double *r = out + 13 * k;
+  r[0] = pos[0] + ix + 0.5;
+  r[1] = pos[1] + iy + 0.5;
+  r[2] = pos[2] + iz + 0.5;
+  r[3] = dir[0];
+  r[4] = dir[1];
+  r[5] = dir[2];
+  r[6] = vel[0];
+  r[7] = vel[1];
+  r[8] = vel[2];
+  r[9] = gof;
+  r[10] = l;
+  r[11] = (double)s;
+  r[12] = -1.0;
 }
 
 __global__ void __launch_bounds__(128) k_wall_fit(const double *__restrict__ ph64, int n,
@@ -1182,13 +1511,31 @@ __global__ void __launch_bounds__(128) k_wall_fit(const double *__restrict__ ph6
   r[9] = -1.0;
 }
 
-// add_string_length / add_wall_area sums (one block; fixed-order tree)
-__global__ void k_defect_sums(const double *__restrict__ strs, int64_t ns,
-                              const double *__restrict__ walls, int64_t nw, double *__restrict__ out) {
-  __shared__ double sh[5][256];
-  double a[5] = {0, 0, 0, 0, 0};  // sl, sqrt(v2), v2, gamma, count of v2<1
-  double wsum = 0.0;
-  for (int64_t k = threadIdx.x; k < ns; k += blockDim.x) {
+// add_string_length / add_wall_area sums in a fixed order: kSumBlocks CTAs
+// each add a strided share (k_defect_sums; one CTA took 1.36 ms for the 5e5
+// rows of a 128^3 lattice, latency of 256 threads' strided loads), then one CTA
+// adds their six sums (k_defect_sums_total).
+constexpr int kSumBlocks = 304;
+
+// the block's sum of a[0..5], result in thread 0
+__device__ __forceinline__ void block_sum6(double a[6]) {
+  __shared__ double sh[6][256];
+  for (int q = 0; q < 6; ++q) sh[q][threadIdx.x] = a[q];
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if ((int)threadIdx.x < o)
+      for (int q = 0; q < 6; ++q) sh[q][threadIdx.x] = sh[q][threadIdx.x] + sh[q][threadIdx.x + o];
+    __syncthreads();
+  }
+  for (int q = 0; q < 6; ++q) a[q] = sh[q][0];
+}
+
+__global__ void __launch_bounds__(256) k_defect_sums(const double *__restrict__ strs, int64_t ns,
+                                                     const double *__restrict__ walls, int64_t nw,
+                                                     double *__restrict__ part) {
+  double a[6] = {0, 0, 0, 0, 0, 0};  // sl, sqrt(v2), v2, gamma, count of v2<1; wa
+  const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t k = first; k < ns; k += step) {
     const double *r = strs + 13 * k;
     a[0] = a[0] + r[10];
     double v2 = r[6] * r[6] + r[7] * r[7];
@@ -1200,24 +1547,19 @@ __global__ void k_defect_sums(const double *__restrict__ strs, int64_t ns,
       a[4] = a[4] + 1.0;
     }
   }
-  for (int64_t k = threadIdx.x; k < nw; k += blockDim.x) wsum = wsum + walls[10 * k + 7];
-  for (int q = 0; q < 5; ++q) sh[q][threadIdx.x] = a[q];
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o)
-      for (int q = 0; q < 5; ++q) sh[q][threadIdx.x] = sh[q][threadIdx.x] + sh[q][threadIdx.x + o];
-    __syncthreads();
-  }
+  for (int64_t k = first; k < nw; k += step) a[5] = a[5] + walls[10 * k + 7];
+  block_sum6(a);
+  if (threadIdx.x < 6) part[6 * blockIdx.x + threadIdx.x] = a[threadIdx.x];
+}
+
+__global__ void __launch_bounds__(256) k_defect_sums_total(const double *__restrict__ part, int nb,
+                                                           double *__restrict__ out) {
+  double a[6] = {0, 0, 0, 0, 0, 0};
+  for (int b = threadIdx.x; b < nb; b += blockDim.x)
+    for (int q = 0; q < 6; ++q) a[q] = a[q] + part[6 * b + q];
+  block_sum6(a);
   if (threadIdx.x == 0)
-    for (int q = 0; q < 5; ++q) out[q] = sh[q][0];
-  __syncthreads();
-  sh[0][threadIdx.x] = wsum;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) sh[0][threadIdx.x] = sh[0][threadIdx.x] + sh[0][threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[5] = sh[0][0];
+    for (int q = 0; q < 6; ++q) out[q] = a[q];
 }
 
 // ---------------- grouping (defects_3d.f90:1235-1652, 1735-2143) ----------------
@@ -1485,6 +1827,7 @@ int axg_def_id_defects(axg_ctx *ctx, double tau, double sl[3], double wa[3], dou
   const int nb = (int)((ctx->n3 + kChunk - 1) / kChunk);
   int *bc = nullptr;
   int64_t *cells = nullptr;
+  double *sim = nullptr;  // simplex scratch of the string fits
   int rc = AXG_OK;
   AXG_TRY(axg_alloc(ctx, (void **)&bc, (size_t)nb * 2 * sizeof(int), "block counts"));
   do {
@@ -1516,32 +1859,56 @@ int axg_def_id_defects(axg_ctx *ctx, double tau, double sl[3], double wa[3], dou
                    (const double2 *)ctx->phi[ctx->cur], (const double2 *)nullptr, ctx->n3, ctx->phase64);
     }
     if (ns > 0) {
-      // resident CTAs only: lanes take cells from a counter (d_cnt[8])
+      // simplex: resident CTAs only, groups take cells from a counter (d_cnt[8])
       int per_sm = 0, sms = 0;
-      AXG_CUDA_TRY(ctx, f32 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_string_fit<float2>, 128, 0)
-                            : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_string_fit<double2>, 128, 0));
+      AXG_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_string_simplex, kFitThreads, 0));
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-      int64_t grid = (int64_t)std::max(per_sm, 1) * std::max(sms, 1);
-      grid = std::min<int64_t>(grid, (ns + 127) / 128);
+      const int64_t resident = (int64_t)std::max(per_sm, 1) * std::max(sms, 1);
       unsigned long long *next = ctx->d_cnt + 8;
-      AXG_CUDA_TRY(ctx, cudaMemsetAsync(next, 0, sizeof(unsigned long long), ctx->stream));
-      if (f32)
-        AXG_LAUNCH(ctx, "string_fit_fp32", k_string_fit<float2>, (unsigned)grid, 128, 0,
-                   (const float2 *)ctx->phi[ctx->cur], (const float2 *)ctx->cphi, ctx->phase64,
-                   (const float2 *)ctx->phid, n, ctx->p.dspa, (uint64_t)ctx->p.seed, cells, ns, ctx->d_strings,
-                   next);
-      else
-        AXG_LAUNCH(ctx, "string_fit_fp64", k_string_fit<double2>, (unsigned)grid, 128, 0,
-                   (const double2 *)ctx->phi[ctx->cur], (const double2 *)nullptr, ctx->phase64,
-                   (const double2 *)ctx->phid, n, ctx->p.dspa, (uint64_t)ctx->p.seed, cells, ns, ctx->d_strings,
-                   next);
+      constexpr int per_cta = kFitThreads / kGrp;
+      // scratch: simplexes, the cells handed over to k_string_simplex_warp (at most the resident groups), their count
+      const int64_t rcap = resident * per_cta;
+      if ((rc = axg_alloc(ctx, (void **)&sim, (size_t)(std::min(ns, kFitChunk) * kFitStride + rcap + 1) * 8, "string fits")))
+        break;
+      int2 *rest = (int2 *)(sim + std::min(ns, kFitChunk) * kFitStride);
+      unsigned *nrest = (unsigned *)(rest + rcap);
+      // few cells: a warp each from the start.  An iteration then costs the
+      // issue slots of two but a third of the time (64^3, 1.5e4 cells: 9.3
+      // against 11.5 ms through k_string_simplex; 128^3, 1.3e5: 30 ms through it)
+      const int64_t few = 5 * (kFitThreads / 32) * resident;
+      for (int64_t c0 = 0; c0 < ns; c0 += kFitChunk) {
+        const int64_t nc = std::min(kFitChunk, ns - c0);
+        AXG_LAUNCH(ctx, "string_start", k_string_start, (unsigned)((nc + per_cta - 1) / per_cta), kFitThreads, 0,
+                   ctx->phase64, n, (uint64_t)ctx->p.seed, cells + c0, nc, sim);
+        AXG_CUDA_TRY(ctx, cudaMemsetAsync(next, 0, sizeof(unsigned long long), ctx->stream));
+        if (nc > few) {
+          AXG_CUDA_TRY(ctx, cudaMemsetAsync(nrest, 0, sizeof(unsigned), ctx->stream));
+          AXG_LAUNCH(ctx, "string_simplex", k_string_simplex,
+                     (unsigned)std::min<int64_t>(resident, (nc + per_cta - 1) / per_cta), kFitThreads, 0, ctx->phase64,
+                     n, cells + c0, nc, sim, next, rest, nrest);
+          AXG_CUDA_TRY(ctx, cudaMemsetAsync(next, 0, sizeof(unsigned long long), ctx->stream));
+        }
+        AXG_LAUNCH(ctx, "string_simplex_warp", k_string_simplex_warp,
+                   (unsigned)std::min<int64_t>(resident, nc > few ? resident : (nc + 3) / 4), kFitThreads, 0,
+                   ctx->phase64, n, cells + c0, nc > few ? rest : nullptr, nrest, nc, sim, next);
+        if (f32)
+          AXG_LAUNCH(ctx, "string_result", k_string_result<float2>, (unsigned)((nc + 127) / 128), 128, 0,
+                     (const float2 *)ctx->phi[ctx->cur], (const float2 *)ctx->cphi, (const float2 *)ctx->phid, n,
+                     ctx->p.dspa, cells + c0, nc, sim, ctx->d_strings + 13 * c0);
+        else
+          AXG_LAUNCH(ctx, "string_result", k_string_result<double2>, (unsigned)((nc + 127) / 128), 128, 0,
+                     (const double2 *)ctx->phi[ctx->cur], (const double2 *)nullptr, (const double2 *)ctx->phid, n,
+                     ctx->p.dspa, cells + c0, nc, sim, ctx->d_strings + 13 * c0);
+      }
     }
     if (nw > 0) {
       AXG_LAUNCH(ctx, "wall_fit", k_wall_fit, (unsigned)((nw + 127) / 128), 128, 0, ctx->phase64, n, cells + ns,
                  nw, ctx->d_walls);
     }
-    AXG_LAUNCH(ctx, "defect_sums", k_defect_sums, 1, 256, 0, ctx->d_strings, ns, ctx->d_walls, nw,
-               ctx->d_red);
+    static_assert(6 + 6 * kSumBlocks <= 4096, "the reduction buffer holds the sums and their parts");
+    const int nsum = (int)std::min<int64_t>(kSumBlocks, (std::max(ns, nw) + 255) / 256 + 1);
+    AXG_LAUNCH(ctx, "defect_sums", k_defect_sums, nsum, 256, 0, ctx->d_strings, ns, ctx->d_walls, nw, ctx->d_red + 6);
+    AXG_LAUNCH(ctx, "defect_sums_total", k_defect_sums_total, 1, 256, 0, ctx->d_red + 6, nsum, ctx->d_red);
     double h[6];
     if (cudaMemcpyAsync(h, ctx->d_red, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
@@ -1580,6 +1947,7 @@ int axg_def_id_defects(axg_ctx *ctx, double tau, double sl[3], double wa[3], dou
   cudaStreamSynchronize(ctx->stream);
   axg_free(ctx, (void **)&bc);
   axg_free(ctx, (void **)&cells);
+  axg_free(ctx, (void **)&sim);
   return rc;
 }
 
