@@ -20,7 +20,9 @@
 #include <cstdlib>
 
 #include "axg_detmath.h"
+#include "axg_gw_source.h"
 #include "axg_internal.h"
+#include "axg_soft64.h"
 #include "axg_tma.h"
 
 namespace {
@@ -31,34 +33,142 @@ constexpr int kPwStages = 2;          // pointwise ring depth (z, prefetch of z+
 // ------------------------------------------------------------------------
 // FP64-plain kernels (evolve.f90:259-281 and 283-339)
 // ------------------------------------------------------------------------
-struct KickCoeffs {
-  double f1, f2, f3, fs;  // fact1, fact2, fact3, source factor
-  double A, B, C, D;      // dV/dphi* = (A|phi|^2+B) phi + C + D conj(phi)
-  double d;               // 2 dspa (grav_waves.f90:331)
-  double inv_d;           // 1/d, used only when d is a power of two (then x/d == x*inv_d exactly)
-  int d_pow2;
+// Coefficients of a kick, and of a drift after it, in FP64: dV/dphi* =
+// (A|phi|^2+B) phi + C + D conj(phi); fs the source factor; d = 2 dspa
+// (grav_waves.f90:331).  The factors that multiply at every site are kept
+// taken apart for axs_mulc; soft is the starting value of its `ok` flags,
+// zero when one of them is outside its window.
+struct Coef64 {
+  axs_const f1, f2, f3, fs, A, h;  // fact1, fact2, fact3, source factor; h: drift step
+  double B, C, D, d, inv_d;
+  int d_pow2;  // d a power of two (x / d == x (1 / d))
+  uint32_t soft;
 };
 
-// x / d, replaced by the exact multiplication by 1/d when d is a power of two
-__device__ __forceinline__ double div_d(double x, double d, double inv_d, int pow2) {
-  return pow2 ? axg_mul_pow2(x, inv_d) : AXD_DIV(x, d);
+__host__ __device__ inline Coef64 make_coef64(const double f[4], const double pot[4], double dspa, double h) {
+  Coef64 k;
+  k.f1 = axs_const_of(f[0]);
+  k.f2 = axs_const_of(f[1]);
+  k.f3 = axs_const_of(f[2]);
+  k.fs = axs_const_of(f[3]);
+  k.A = axs_const_of(pot[0]);
+  k.h = axs_const_of(h);
+  k.d = dspa * 2;
+  k.inv_d = 1.0 / k.d;
+  k.B = pot[1];
+  k.C = pot[2];
+  k.D = pot[3];
+  const axs_const dd = axs_const_of(k.d);
+  k.d_pow2 = dd.hi == 0x100000u && dd.lo == 0u && dd.ok;
+  k.soft = k.f1.ok && k.f2.ok && k.f3.ok && k.fs.ok && k.A.ok ? 0xffffffffu : 0u;
+  return k;
+}
+
+// ---- FP64 arithmetic of one site, in the reference's operation order -------
+//
+// Every product of a site runs on the integer pipes (axg_soft64.h), beside
+// the FP64 pipe that the stencil is bound by: 79 sums stay there of a kick's
+// 128 operations (phi and six u_ij).  Each block counts its operands through
+// the `ok` flags; a block with an operand outside the window (a zero of the
+// initial u_ij, say) is redone with hardware operations, out of line.
+// Us per launch at 128^3, phi and u_ij: kick 535 -> 347 (the 79 sums alone
+// are 310 at the measured FP64 rate), drift 77 -> 66, fused 602 -> 415; phi
+// alone 167 -> 101.  At 100^3, where 2 dx is no power of two, the kick 360 ->
+// 278 and the fused step 382 -> 249.
+
+__device__ __forceinline__ double sum6_64(double xm, double xp, double ym, double yp, double zm, double zp) {
+  double l = AXD_ADD(xm, xp);
+  l = AXD_ADD(l, ym);
+  l = AXD_ADD(l, yp);
+  l = AXD_ADD(l, zm);
+  return AXD_ADD(l, zp);
+}
+
+// 6 x
+__device__ __forceinline__ double six64(double x, uint32_t &ok) {
+  const axs_const six = {0u, 0x180000u, (1025u - 1024u) << 20, 0u, 6.0, 1u};
+  return axs_mulc(x, &six, &ok);
+}
+
+// data2 = fact1*data2 + fact2*dlap + fact3*ddv (evolve.f90:330), dlap
+// (:325-328) = sum - 6 phi, dVdphi (potential.f90:43-60); hardware operations
+__device__ __noinline__ double2 phi_kick64_hw(const Coef64 &k, double2 c, double2 sum, double2 pd) {
+  const double lr = AXD_SUB(sum.x, AXD_MUL(6.0, c.x)), li = AXD_SUB(sum.y, AXD_MUL(6.0, c.y));
+  const double s2 = AXD_ADD(AXD_MUL(c.x, c.x), AXD_MUL(c.y, c.y));
+  const double g = AXD_ADD(AXD_MUL(k.A.v, s2), k.B);
+  double vr = AXD_MUL(g, c.x), vi = AXD_MUL(g, c.y);
+  if (k.D != 0.0) {
+    vr = AXD_ADD(vr, AXD_MUL(k.D, c.x));
+    vi = AXD_SUB(vi, AXD_MUL(k.D, c.y));
+  }
+  vr = AXD_ADD(vr, k.C);
+  double pr = AXD_ADD(AXD_MUL(k.f1.v, pd.x), AXD_MUL(k.f2.v, lr));
+  pr = AXD_ADD(pr, AXD_MUL(k.f3.v, vr));
+  double pi_ = AXD_ADD(AXD_MUL(k.f1.v, pd.y), AXD_MUL(k.f2.v, li));
+  pi_ = AXD_ADD(pi_, AXD_MUL(k.f3.v, vi));
+  return make_double2(pr, pi_);
+}
+
+// sum: the six neighbours' sum
+__device__ __forceinline__ double2 phi_kick64(const Coef64 &k, double2 c, double2 sum, double2 pd) {
+  uint32_t ok = k.soft;
+  const double lr = AXD_SUB(sum.x, six64(c.x, ok)), li = AXD_SUB(sum.y, six64(c.y, ok));
+  const double s2 = AXD_ADD(axs_mul(c.x, c.x, &ok), axs_mul(c.y, c.y, &ok));
+  const double g = AXD_ADD(axs_mulc(s2, &k.A, &ok), k.B);
+  double vr = axs_mul(g, c.x, &ok), vi = axs_mul(g, c.y, &ok);
+  if (k.D != 0.0) {
+    vr = AXD_ADD(vr, AXD_MUL(k.D, c.x));
+    vi = AXD_SUB(vi, AXD_MUL(k.D, c.y));
+  }
+  vr = AXD_ADD(vr, k.C);
+  double pr = AXD_ADD(axs_mulc(pd.x, &k.f1, &ok), axs_mulc(lr, &k.f2, &ok));
+  pr = AXD_ADD(pr, axs_mulc(vr, &k.f3, &ok));
+  double pi_ = AXD_ADD(axs_mulc(pd.y, &k.f1, &ok), axs_mulc(li, &k.f2, &ok));
+  pi_ = AXD_ADD(pi_, axs_mulc(vi, &k.f3, &ok));
+  if (ok & AXS_WINDOW) return make_double2(pr, pi_);
+  return phi_kick64_hw(k, c, sum, pd);
+}
+
+// one u_ij component's kick with source S
+__device__ __noinline__ double u_kick64_hw(const Coef64 &k, double S, double uc, double sum, double udv) {
+  const double lu = AXD_SUB(sum, AXD_MUL(6.0, uc));
+  const double v = AXD_ADD(AXD_MUL(k.f1.v, udv), AXD_MUL(k.f2.v, lu));
+  return AXD_ADD(v, AXD_MUL(k.fs.v, S));
+}
+
+__device__ __forceinline__ double u_kick64(const Coef64 &k, double S, double uc, double sum, double udv) {
+  uint32_t ok = k.soft;
+  const double lu = AXD_SUB(sum, six64(uc, ok));
+  const double v = AXD_ADD(axs_mulc(udv, &k.f1, &ok), axs_mulc(lu, &k.f2, &ok));
+  const double r = AXD_ADD(v, axs_mulc(S, &k.fs, &ok));
+  if (ok & AXS_WINDOW) return r;
+  return u_kick64_hw(k, S, uc, sum, udv);
+}
+
+// x + h v
+__device__ __noinline__ double drift64_hw(double x, double v, double h) { return AXD_ADD(x, AXD_MUL(h, v)); }
+__device__ __forceinline__ double drift64(const axs_const &h, double x, double v) {
+  uint32_t ok = h.ok ? 0xffffffffu : 0u;
+  const double r = AXD_ADD(x, axs_mulc(v, &h, &ok));
+  if (ok & AXS_WINDOW) return r;
+  return drift64_hw(x, v, h.v);
 }
 
 __global__ void k_drift_fp64(double2 *__restrict__ phi, const double2 *__restrict__ phid,
                              double *__restrict__ u, const double *__restrict__ ud, int64_t n3,
-                             double h, int uij) {
+                             axs_const h, int uij) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n3; s += stride) {
     double2 a = phi[s];
     const double2 b = phid[s];
-    a.x = AXD_ADD(a.x, AXD_MUL(h, b.x));
-    a.y = AXD_ADD(a.y, AXD_MUL(h, b.y));
+    a.x = drift64(h, a.x, b.x);
+    a.y = drift64(h, a.y, b.y);
     phi[s] = a;
     if (uij) {
 #pragma unroll
       for (int c = 0; c < 6; ++c) {
         const int64_t i = c * n3 + s;
-        u[i] = AXD_ADD(u[i], AXD_MUL(h, ud[i]));
+        u[i] = drift64(h, u[i], ud[i]);
       }
     }
   }
@@ -72,7 +182,7 @@ template <bool UIJ>
 __global__ void __launch_bounds__(256) k_kick_fp64(const double2 *__restrict__ phi,
                                                    double2 *__restrict__ phid,
                                                    const double *__restrict__ u,
-                                                   double *__restrict__ ud, int n, KickCoeffs k) {
+                                                   double *__restrict__ ud, int n, const __grid_constant__ Coef64 k) {
   const int ix = blockIdx.x * blockDim.x + threadIdx.x;
   const int iy = blockIdx.y * blockDim.y + threadIdx.y;
   const int iz = blockIdx.z;
@@ -87,61 +197,20 @@ __global__ void __launch_bounds__(256) k_kick_fp64(const double2 *__restrict__ p
   const int64_t sz1 = iz1 * n2 + (int64_t)iy * n + ix, sz2 = iz2 * n2 + (int64_t)iy * n + ix;
   const double2 pc = phi[c], px1 = phi[sx1], px2 = phi[sx2], py1 = phi[sy1], py2 = phi[sy2],
                 pz1 = phi[sz1], pz2 = phi[sz2];
-  // dlap (evolve.f90:325-328), left to right
-  double lr = AXD_ADD(px1.x, px2.x);
-  lr = AXD_ADD(lr, py1.x);
-  lr = AXD_ADD(lr, py2.x);
-  lr = AXD_ADD(lr, pz1.x);
-  lr = AXD_ADD(lr, pz2.x);
-  lr = AXD_SUB(lr, AXD_MUL(6.0, pc.x));
-  double li = AXD_ADD(px1.y, px2.y);
-  li = AXD_ADD(li, py1.y);
-  li = AXD_ADD(li, py2.y);
-  li = AXD_ADD(li, pz1.y);
-  li = AXD_ADD(li, pz2.y);
-  li = AXD_SUB(li, AXD_MUL(6.0, pc.y));
-  // dVdphi (potential.f90:43-60)
-  const double s2 = AXD_ADD(AXD_MUL(pc.x, pc.x), AXD_MUL(pc.y, pc.y));
-  const double g = AXD_ADD(AXD_MUL(k.A, s2), k.B);
-  double vr = AXD_MUL(g, pc.x), vi = AXD_MUL(g, pc.y);
-  if (k.D != 0.0) {
-    vr = AXD_ADD(vr, AXD_MUL(k.D, pc.x));
-    vi = AXD_SUB(vi, AXD_MUL(k.D, pc.y));
-  }
-  vr = AXD_ADD(vr, k.C);
-  // data2 = fact1*data2 + fact2*dlap + fact3*ddv (evolve.f90:330)
-  const double2 pd = phid[c];
-  double pr = AXD_ADD(AXD_MUL(k.f1, pd.x), AXD_MUL(k.f2, lr));
-  pr = AXD_ADD(pr, AXD_MUL(k.f3, vr));
-  double pi_ = AXD_ADD(AXD_MUL(k.f1, pd.y), AXD_MUL(k.f2, li));
-  pi_ = AXD_ADD(pi_, AXD_MUL(k.f3, vi));
-  phid[c] = make_double2(pr, pi_);
+  // dlap (evolve.f90:325-328) sums its neighbours left to right
+  const double2 sum = make_double2(sum6_64(px1.x, px2.x, py1.x, py2.x, pz1.x, pz2.x),
+                                   sum6_64(px1.y, px2.y, py1.y, py2.y, pz1.y, pz2.y));
+  phid[c] = phi_kick64(k, pc, sum, phid[c]);
   if constexpr (UIJ) {
-    double dr[3], di[3];
-    dr[0] = div_d(AXD_SUB(px2.x, px1.x), k.d, k.inv_d, k.d_pow2);
-    di[0] = div_d(AXD_SUB(px2.y, px1.y), k.d, k.inv_d, k.d_pow2);
-    dr[1] = div_d(AXD_SUB(py2.x, py1.x), k.d, k.inv_d, k.d_pow2);
-    di[1] = div_d(AXD_SUB(py2.y, py1.y), k.d, k.inv_d, k.d_pow2);
-    dr[2] = div_d(AXD_SUB(pz2.x, pz1.x), k.d, k.inv_d, k.d_pow2);
-    di[2] = div_d(AXD_SUB(pz2.y, pz1.y), k.d, k.inv_d, k.d_pow2);
-    int comp = 0;
+    const double gr[3] = {AXD_SUB(px2.x, px1.x), AXD_SUB(py2.x, py1.x), AXD_SUB(pz2.x, pz1.x)};
+    const double gi[3] = {AXD_SUB(px2.y, px1.y), AXD_SUB(py2.y, py1.y), AXD_SUB(pz2.y, pz1.y)};
+    double S[6];
+    gw_sources_from_diff(gr, gi, k.d, k.inv_d, k.d_pow2, S);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-#pragma unroll
-      for (int j = 0; j <= i; ++j, ++comp) {
-        const double *uc = u + comp * n3;
-        double src = AXD_ADD(AXD_MUL(dr[i], dr[j]), AXD_MUL(di[i], di[j]));
-        src = axg_mul_pow2(src, 2.0);
-        double lu = AXD_ADD(uc[sx1], uc[sx2]);
-        lu = AXD_ADD(lu, uc[sy1]);
-        lu = AXD_ADD(lu, uc[sy2]);
-        lu = AXD_ADD(lu, uc[sz1]);
-        lu = AXD_ADD(lu, uc[sz2]);
-        lu = AXD_SUB(lu, AXD_MUL(6.0, uc[c]));
-        double v = AXD_ADD(AXD_MUL(k.f1, ud[comp * n3 + c]), AXD_MUL(k.f2, lu));
-        v = AXD_ADD(v, AXD_MUL(k.fs, src));
-        ud[comp * n3 + c] = v;
-      }
+    for (int comp = 0; comp < 6; ++comp) {
+      const double *uc = u + comp * n3;
+      ud[comp * n3 + c] = u_kick64(k, S[comp], uc[c], sum6_64(uc[sx1], uc[sx2], uc[sy1], uc[sy2], uc[sz1], uc[sz2]),
+                                   ud[comp * n3 + c]);
     }
   }
 }
@@ -269,9 +338,16 @@ struct FusedParams {
   int64_t n3;
   int n, zc;
   R f1, f2, f3, fsc, dtd, A, B, C, D;
-  double d;  // 2 dspa (FP64 path keeps the reference's division)
-  double inv_d;
-  int d_pow2;
+  int *err;
+};
+
+template <>
+struct FusedParams<double> {
+  double2 *phi_out, *phid, *cphi;
+  double *u_out, *ud, *cu;
+  int64_t n3;
+  int n, zc;
+  Coef64 k;
   int *err;
 };
 
@@ -311,32 +387,9 @@ __device__ __forceinline__ void site_phi(const FusedParams<float> &P, float2 c0,
 __device__ __forceinline__ void site_phi(const FusedParams<double> &P, double2 c0, double2 xm, double2 xp,
                                          double2 ym, double2 yp, double2 zm, double2 zp, double2 pd, double2 &,
                                          double2 &pdn, double2 &pn) {
-  double lr = AXD_ADD(xm.x, xp.x);
-  lr = AXD_ADD(lr, ym.x);
-  lr = AXD_ADD(lr, yp.x);
-  lr = AXD_ADD(lr, zm.x);
-  lr = AXD_ADD(lr, zp.x);
-  lr = AXD_SUB(lr, AXD_MUL(6.0, c0.x));
-  double li = AXD_ADD(xm.y, xp.y);
-  li = AXD_ADD(li, ym.y);
-  li = AXD_ADD(li, yp.y);
-  li = AXD_ADD(li, zm.y);
-  li = AXD_ADD(li, zp.y);
-  li = AXD_SUB(li, AXD_MUL(6.0, c0.y));
-  const double s2 = AXD_ADD(AXD_MUL(c0.x, c0.x), AXD_MUL(c0.y, c0.y));
-  const double g = AXD_ADD(AXD_MUL(P.A, s2), P.B);
-  double vr = AXD_MUL(g, c0.x), vi = AXD_MUL(g, c0.y);
-  if (P.D != 0.0) {
-    vr = AXD_ADD(vr, AXD_MUL(P.D, c0.x));
-    vi = AXD_SUB(vi, AXD_MUL(P.D, c0.y));
-  }
-  vr = AXD_ADD(vr, P.C);
-  double pr = AXD_ADD(AXD_MUL(P.f1, pd.x), AXD_MUL(P.f2, lr));
-  pr = AXD_ADD(pr, AXD_MUL(P.f3, vr));
-  double pi_ = AXD_ADD(AXD_MUL(P.f1, pd.y), AXD_MUL(P.f2, li));
-  pi_ = AXD_ADD(pi_, AXD_MUL(P.f3, vi));
-  pdn = make_double2(pr, pi_);
-  pn = make_double2(AXD_ADD(c0.x, AXD_MUL(P.dtd, pr)), AXD_ADD(c0.y, AXD_MUL(P.dtd, pi_)));
+  const double2 sum = make_double2(sum6_64(xm.x, xp.x, ym.x, yp.x, zm.x, zp.x), sum6_64(xm.y, xp.y, ym.y, yp.y, zm.y, zp.y));
+  pdn = phi_kick64(P.k, c0, sum, pd);
+  pn = make_double2(drift64(P.k.h, c0.x, pdn.x), drift64(P.k.h, c0.y, pdn.y));
 }
 
 // the six sources S_c (c = (1,1),(2,1),(2,2),(3,1),(3,2),(3,3)) at one site
@@ -358,18 +411,9 @@ __device__ __forceinline__ void site_sources(const FusedParams<float> &, float2 
 
 __device__ __forceinline__ void site_sources(const FusedParams<double> &P, double2 xm, double2 xp, double2 ym,
                                              double2 yp, double2 zm, double2 zp, double S[6]) {
-  double dr[3], di[3];
-  dr[0] = div_d(AXD_SUB(xp.x, xm.x), P.d, P.inv_d, P.d_pow2);
-  di[0] = div_d(AXD_SUB(xp.y, xm.y), P.d, P.inv_d, P.d_pow2);
-  dr[1] = div_d(AXD_SUB(yp.x, ym.x), P.d, P.inv_d, P.d_pow2);
-  di[1] = div_d(AXD_SUB(yp.y, ym.y), P.d, P.inv_d, P.d_pow2);
-  dr[2] = div_d(AXD_SUB(zp.x, zm.x), P.d, P.inv_d, P.d_pow2);
-  di[2] = div_d(AXD_SUB(zp.y, zm.y), P.d, P.inv_d, P.d_pow2);
-  int c = 0;
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j <= i; ++j, ++c) S[c] = axg_mul_pow2(AXD_ADD(AXD_MUL(dr[i], dr[j]), AXD_MUL(di[i], di[j])), 2.0);
+  const double gr[3] = {AXD_SUB(xp.x, xm.x), AXD_SUB(yp.x, ym.x), AXD_SUB(zp.x, zm.x)};
+  const double gi[3] = {AXD_SUB(xp.y, xm.y), AXD_SUB(yp.y, ym.y), AXD_SUB(zp.y, zm.y)};
+  gw_sources_from_diff(gr, gi, P.k.d, P.k.inv_d, P.k.d_pow2, S);
 }
 
 // one u_ij component: kick with source S, drift (FP32: Kahan with cc)
@@ -385,15 +429,8 @@ __device__ __forceinline__ void site_u(const FusedParams<float> &P, float S, flo
 __device__ __forceinline__ void site_u(const FusedParams<double> &P, double S, double uc, double uxm, double uxp,
                                        double uym, double uyp, double uzm, double uzp, double udv, double &,
                                        double &udn, double &un) {
-  double lu = AXD_ADD(uxm, uxp);
-  lu = AXD_ADD(lu, uym);
-  lu = AXD_ADD(lu, uyp);
-  lu = AXD_ADD(lu, uzm);
-  lu = AXD_ADD(lu, uzp);
-  lu = AXD_SUB(lu, AXD_MUL(6.0, uc));
-  double v = AXD_ADD(AXD_MUL(P.f1, udv), AXD_MUL(P.f2, lu));
-  udn = AXD_ADD(v, AXD_MUL(P.fsc, S));
-  un = AXD_ADD(uc, AXD_MUL(P.dtd, udn));
+  udn = u_kick64(P.k, S, uc, sum6_64(uxm, uxp, uym, uyp, uzm, uzp), udv);
+  un = drift64(P.k.h, uc, udn);
 }
 
 // One TX x TY column of zc planes starting at (x0, y0, z0): stage the
@@ -610,7 +647,7 @@ __global__ void __launch_bounds__(TX *TY, (sizeof(R) == 4 && TX * TY <= 256 ? 2 
     k_fused(const __grid_constant__ CUtensorMap tm_prow, const __grid_constant__ CUtensorMap tm_pbody,
             const __grid_constant__ CUtensorMap tm_phalo, const __grid_constant__ CUtensorMap tm_urow,
             const __grid_constant__ CUtensorMap tm_ubody, const __grid_constant__ CUtensorMap tm_uhalo,
-            const __grid_constant__ PwMaps pwm, const FusedParams<R> P) {
+            const __grid_constant__ PwMaps pwm, const __grid_constant__ FusedParams<R> P) {
   using L = StageLayout<R, TX, TY, UIJ>;
   using PL = PwLayout<R, TX, TY, UIJ>;
   extern __shared__ unsigned char smem_raw[];
@@ -648,19 +685,19 @@ __global__ void __launch_bounds__(TX *TY, (sizeof(R) == 4 && TX * TY <= 256 ? 2 
   init_stage_barriers(bars);
   const axg_ens_coef &K = coefs[step];
   FusedParams<R> P;
-  P.f1 = (R)K.f[0];
-  P.f2 = (R)K.f[1];
-  P.f3 = (R)K.f[2];
-  P.fsc = sizeof(R) == 4 ? (R)(K.f[3] * 2.0 / ((2.0 * dspa) * (2.0 * dspa))) : (R)K.f[3];
-  P.dtd = (R)K.dtd;
-  P.A = (R)K.pot[0];
-  P.B = (R)K.pot[1];
-  P.C = (R)K.pot[2];
-  P.D = (R)K.pot[3];
-  P.d = 2.0 * dspa;
-  P.inv_d = 1.0 / P.d;
-  int ex;
-  P.d_pow2 = sizeof(R) == 8 && frexp(P.d, &ex) == 0.5;
+  if constexpr (sizeof(R) == 4) {
+    P.f1 = (R)K.f[0];
+    P.f2 = (R)K.f[1];
+    P.f3 = (R)K.f[2];
+    P.fsc = (R)(K.f[3] * 2.0 / ((2.0 * dspa) * (2.0 * dspa)));
+    P.dtd = (R)K.dtd;
+    P.A = (R)K.pot[0];
+    P.B = (R)K.pot[1];
+    P.C = (R)K.pot[2];
+    P.D = (R)K.pot[3];
+  } else {
+    P.k = make_coef64(K.f, K.pot, dspa, K.dtd);
+  }
   P.zc = zc;
   P.err = err;
   uint32_t gplane = 0, gpw = 0;
@@ -702,7 +739,8 @@ __global__ void __launch_bounds__(TX *TY, (sizeof(R) == 4 && TX * TY <= 256 ? 2 
 // ------------------------------------------------------------------------
 template <typename R, bool UIJ>
 __global__ void __launch_bounds__(256) k_fused_plain(const typename V2<R>::T *__restrict__ phi_in,
-                                                     const R *__restrict__ u_in, FusedParams<R> P) {
+                                                     const R *__restrict__ u_in,
+                                                     const __grid_constant__ FusedParams<R> P) {
   using V = typename V2<R>::T;
   const int n = P.n, n2 = n * n;
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
@@ -959,8 +997,8 @@ int axg_evo_drift(axg_ctx *ctx, double h) {
                (const float *)ctx->ud, (float *)ctx->cu, n3, (float)h, uij);
   } else {
     AXG_LAUNCH(ctx, "drift_fp64", k_drift_fp64, blocks, 256, 0, (double2 *)ctx->phi[b],
-               (const double2 *)ctx->phid, (double *)ctx->u[b], (const double *)ctx->ud, n3, h,
-               uij);
+               (const double2 *)ctx->phid, (double *)ctx->u[b], (const double *)ctx->ud, n3,
+               axs_const_of(h), uij);
   }
   return AXG_OK;
 }
@@ -970,10 +1008,7 @@ int axg_evo_kick_plain(axg_ctx *ctx, double t, double dt) {
     return axg_set_error(ctx, AXG_ERR_STATE, "separate kick is the FP64 path; FP32 runs fused");
   double f[4], pot[4];
   axg_kick_coeffs(&ctx->p, t, dt, f, pot);
-  const double d = ctx->p.dspa * 2;
-  int ex;
-  const int pow2 = std::frexp(d, &ex) == 0.5;
-  KickCoeffs k{f[0], f[1], f[2], f[3], pot[0], pot[1], pot[2], pot[3], d, 1.0 / d, pow2};
+  const Coef64 k = make_coef64(f, pot, ctx->p.dspa, dt);
   const int n = (int)ctx->n;
   dim3 block(32, 8);
   dim3 grid((n + 31) / 32, (n + 7) / 8, n);
@@ -1067,9 +1102,6 @@ int axg_evo_kick_drift(axg_ctx *ctx, double t, double dt, double dtd) {
     P.B = (float)pot[1];
     P.C = (float)pot[2];
     P.D = (float)pot[3];
-    P.d = 2.0 * ctx->p.dspa;
-    P.inv_d = 1.0 / P.d;
-    P.d_pow2 = 0;
     P.err = ctx->d_err;
     if (plain && uij)
       AXG_LAUNCH(ctx, shape.suffix ? "fused_kd_fp32_uij_plain" : "fused_kd_fp32_uij",
@@ -1092,19 +1124,7 @@ int axg_evo_kick_drift(axg_ctx *ctx, double t, double dt, double dtd) {
     P.n3 = ctx->n3;
     P.n = (int)ctx->n;
     P.zc = shape.zc;
-    P.f1 = f[0];
-    P.f2 = f[1];
-    P.f3 = f[2];
-    P.fsc = f[3];
-    P.dtd = dtd;
-    P.A = pot[0];
-    P.B = pot[1];
-    P.C = pot[2];
-    P.D = pot[3];
-    P.d = 2.0 * ctx->p.dspa;
-    int ex;
-    P.d_pow2 = std::frexp(P.d, &ex) == 0.5;
-    P.inv_d = 1.0 / P.d;
+    P.k = make_coef64(f, pot, ctx->p.dspa, dtd);
     P.err = ctx->d_err;
     if (plain && uij)
       AXG_LAUNCH(ctx, shape.suffix ? "fused_kd_fp64_uij_plain" : "fused_kd_fp64_uij",

@@ -502,11 +502,11 @@ __global__ void __launch_bounds__(M) k_ff_gws_rows(const double2 *__restrict__ p
     double S0[6], S1[6];
     {
       const double2 pa[3] = {p1, pyp[x0], pzp[x0]}, pb[3] = {xm, pym[x0], pzm[x0]};
-      gw_sources_fp64(pa, pb, d, inv_d, d_pow2, S0);
+      gw_sources_fp64<false>(pa, pb, d, inv_d, d_pow2, S0);
     }
     {
       const double2 pa[3] = {xp, pyp[x0 + 1], pzp[x0 + 1]}, pb[3] = {p0, pym[x0 + 1], pzm[x0 + 1]};
-      gw_sources_fp64(pa, pb, d, inv_d, d_pow2, S1);
+      gw_sources_fp64<false>(pa, pb, d, inv_d, d_pow2, S1);
     }
 #pragma unroll
     for (int c = 0; c < 6; ++c) s[c * LP + fpad(m)] = cx(f2_from_bits(S0[c]), f2_from_bits(S1[c]));

@@ -58,7 +58,7 @@ __global__ void k_gw_source(const double2 *__restrict__ phi, int n, double d, do
     const int64_t sz1 = (int64_t)(iz == 0 ? n - 1 : iz - 1) * n2 + (int64_t)iy * n + ix;
     const double2 pa[3] = {phi[sx2], phi[sy2], phi[sz2]}, pb[3] = {phi[sx1], phi[sy1], phi[sz1]};
     double S[6];
-    gw_sources_fp64(pa, pb, d, inv_d, d_pow2, S);
+    gw_sources_fp64<true>(pa, pb, d, inv_d, d_pow2, S);
 #pragma unroll
     for (int c = 0; c < 6; ++c) src[c * n3 + s] = S[c];
   }

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import axion_grav_gb300 as ag
+from oracle import axo
 from tests.test_gpu_evolve import make_params, random_state, run_gpu
 
 pytestmark = pytest.mark.gpu
@@ -72,3 +73,28 @@ def test_plain_kernel_planes_against_fp64(n):
     for x, y in zip(a[:4], b[:4]):
         # three steps of rounding 6e-8 in fields whose Laplacian terms are a few times their size
         assert np.max(np.abs(x - y)) <= 2e-5 * np.max(np.abs(y))
+
+
+# operands the integer products refuse (zeros, subnormals, infinities, huge
+# and tiny fields) next to ones they take, for a power-of-two 2 dx and not
+@pytest.mark.parametrize("dspa", [0.5, 0.32])
+@pytest.mark.parametrize("prec", [ag.PREC_FP64_PLAIN, ag.PREC_FP64_FUSED])
+def test_fp64_products_at_the_edges_of_their_window(prec, dspa):
+    n = 12
+    p = make_params(n, prec, ag.GW_UIJ, dspa=dspa)
+    phi, phid, u, ud = random_state(n, 3, 0.05)
+    u[:, 3:6] = 0.0
+    ud[:, :, 2:4] = 0.0
+    phid[2] = 0.0
+    phi[5, 5:8] = phi[5, 5, 5]  # vanishing differences
+    u[0, 7] *= 1e-310
+    u[1, 7] = 1e300
+    u[2, 7] *= 1e-160
+    phi[8, 8, 8] = 1e-200 + 1e-320j
+    u[3, 9, 9, 9] = np.inf
+    ref = tuple(a.copy() for a in (phi, phid, u, ud))
+    with np.errstate(all="ignore"):
+        axo.leapfrog(p, *ref, None, 1.5, 0.02, 3, True, True)
+        got = run_gpu(p, (phi, phid, u, ud), lambda lat: lat.leapfrog(1.5, 0.02, 3, True, True))
+    for a, b in zip(got[:4], ref):
+        assert np.array_equal(a, b, equal_nan=True)
