@@ -6,31 +6,31 @@
 // deterministic versions of axg_detmath.h.  Cell flags, counts, plaquette
 // windings and every per-cell fit (position, direction, length, velocity,
 // wall area) are therefore bit-identical to a host evaluation of the same
-// formulas.  FP32 phases (atan2f) serve only as a filter that decides the
+// formulas.  FP32 phases serve only as a filter that decides the
 // cells whose outcome cannot change within their error bound; all other
 // cells go through the FP64 path.
 //
 // Passes (all O(N^3) passes are HBM-streaming, the fits are sparse):
-//   1. phase     : ph[s] = atan2f(Im phi, Re phi), FP32         (4 B / site)
-//   2. classify  : 8 corner phases, sort, largest circular gap -> int8 flags,
-//                  warp-aggregated counts (defects_3d.f90:67-103, 309-349).
+//   1. classify  : FP32 phases of a tile of phi in shared memory, 8 corner
+//                  phases, sort, largest circular gap -> int8 flags and
+//                  counts (defects_3d.f90:67-103, 309-349).
 //                  Filtered: the FP32 phases are within 1e-6 of the FP64
 //                  ones, and sorting moves no value by more than that, so a
 //                  cell whose every decision (wall gap against wrap gap,
 //                  largest gap against pi and 7 pi / 4) clears a 2e-5
 //                  margin has the FP64 flags; any other cell is redone from
 //                  phi with the deterministic FP64 atan2, as on the host.
-//   3. winding   : three plaquettes per site, filtered the same way (a
+//   2. winding   : three plaquettes per site, filtered the same way (a
 //                  corner difference within the margin of +-pi is redone in
 //                  FP64)
-//   4. compaction: string and wall cells listed in cell order
-//   5. fits      : string cells by groups of eight lanes -- the search
+//   3. compaction: string and wall cells listed in cell order
+//   4. fits      : string cells by groups of eight lanes -- the search
 //                  of position_string (1001 random starts, screened in FP32,
 //                  + Nelder-Mead, defects_3d.f90:435-603; the chi2 in
 //                  float-float on the FP32 pipes, axg_ffchi2.h), string_length
 //                  (1027-1056), velocity_string (605-692), position_wall
 //                  (1058-1233)
-//   6. sums      : add_string_length / add_wall_area without grouping
+//   5. sums      : add_string_length / add_wall_area without grouping
 #include <cmath>
 
 #include "axg_detmath.h"
@@ -62,25 +62,43 @@ __device__ __forceinline__ void load_c(const V *a, const V *comp, int64_t s, dou
   }
 }
 
-// FP32 phase of each site.  For an FP64 field a component outside the FP32
-// normal range (and not zero) would lose relative precision in conversion:
-// such sites get NaN and every cell touching them is classified in FP64.
-template <typename V>
-__global__ void k_phase32(const V *__restrict__ phi, float *__restrict__ ph, int64_t n3) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n3; s += stride) {
-    const V v = phi[s];
-    if constexpr (sizeof(v.x) == 4) {
-      ph[s] = atan2f(v.y, v.x);
-    } else {
-      auto in_range = [](double x) {
-        const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
-        const int e = (int)(b >> 52);
-        return b == 0 || (e >= 1023 - 126 && e <= 1023 + 127);
-      };
-      ph[s] = (in_range(v.x) && in_range(v.y)) ? atan2f((float)v.y, (float)v.x) : __int_as_float(0x7fc00000);
-    }
-  }
+// FP32 phase of a site, within 1e-6 of the FP64 one, or `unknown` (then every
+// cell touching the site is decided in FP64).  n / d, the smaller over the
+// larger component, goes through Hastings' eight-term arctangent (Abramowitz
+// and Stegun 4.4.49: 2e-8 on [0, 1]); the fast quotient, the rounding of the
+// ratio and of the quadrant sums stay below 4e-7, and 2.4e-7 more for an FP64
+// field's truncation to float.
+// About 20 instructions against some 40 of atan2f, whose care for special
+// operands the range test replaces: outside [2^-100, 2^120] of the larger
+// component, and for zeros, infinities and NaN, the phase is unknown.
+__device__ __forceinline__ float phase_fast(float re, float im, float unknown) {
+  const float ar = fabsf(re), ai = fabsf(im), d = fmaxf(ar, ai), q = __fdividef(fminf(ar, ai), d), t = q * q;
+  float p = fmaf(t, 0.0028662257f, -0.0161657367f);
+  p = fmaf(t, p, 0.0429096138f);
+  p = fmaf(t, p, -0.0752896400f);
+  p = fmaf(t, p, 0.1065626393f);
+  p = fmaf(t, p, -0.1420889944f);
+  p = fmaf(t, p, 0.1999355085f);
+  p = fmaf(t, p, -0.3333314528f);
+  p = fmaf(t * p, q, q);
+  if (ai > ar) p = 1.5707963267948966f - p;
+  if (re < 0.0f) p = 3.1415926535897932f - p;
+  return d > 7.8886091e-31f && d < 1.3292280e36f ? copysignf(p, im) : unknown;
+}
+__device__ __forceinline__ float phase_of(float2 v, float unknown) { return phase_fast(v.x, v.y, unknown); }
+// A double truncated to float on the integer pipes (the conversion and FP64
+// comparisons run on the FP64 pipe): within 2^-23 of its size, a value below
+// FP32's normal range as zero of its sign (phase_fast's range test then knows
+// whether the other component is large enough for that), above it infinite.
+__device__ __forceinline__ float f32_truncated(double x) {
+  const uint32_t h = (uint32_t)__double2hiint(x), l = (uint32_t)__double2loint(x), m = h & 0x7fffffffu;
+  uint32_t f = (m << 3 | l >> 29) - (896u << 23);
+  if (m < (897u << 20)) f = 0u;
+  if (m >= (1151u << 20)) f = m > 0x7ff00000u ? 0x7fc00000u : 0x7f800000u;
+  return __uint_as_float(f | (h & 0x80000000u));
+}
+__device__ __forceinline__ float phase_of(double2 v, float unknown) {
+  return phase_fast(f32_truncated(v.x), f32_truncated(v.y), unknown);
 }
 
 __device__ __forceinline__ void cswap(double &a, double &b) {
@@ -128,30 +146,24 @@ __device__ __forceinline__ int8_t classify_sorted(const double pht[8], int which
   return flag;
 }
 
-// Three counters per block: warps tally ballots in registers, the block
-// adds them in shared memory, and one thread adds the block's totals to the
-// global counters (3 global atomics per block instead of 3 per warp pass).
-struct BlockCount3 {
-  unsigned long long c[3] = {0, 0, 0};
-  __device__ __forceinline__ void add(bool a, bool b, bool d) {
-    c[0] += __popc(__ballot_sync(0xffffffffu, a));
-    c[1] += __popc(__ballot_sync(0xffffffffu, b));
-    c[2] += __popc(__ballot_sync(0xffffffffu, d));
+// Adds the block's three tallies (10 bits each of the threads' packed
+// counts) to dst: 3 global atomics per block.
+__device__ __forceinline__ void block_tally3(unsigned packed, unsigned long long *dst) {
+  __shared__ unsigned sh[3];
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+  if (tid < 3) sh[tid] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const unsigned c = __reduce_add_sync(0xffffffffu, (packed >> (10 * k)) & 0x3ffu);
+    if ((tid & 31) == 0 && c) atomicAdd(&sh[k], c);
   }
-  __device__ __forceinline__ void flush(unsigned long long *dst) {
-    __shared__ unsigned long long sh[3];
-    if (threadIdx.x < 3) sh[threadIdx.x] = 0;
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0)
-      for (int k = 0; k < 3; ++k)
-        if (c[k]) atomicAdd(&sh[k], c[k]);
-    __syncthreads();
-    if (threadIdx.x < 3 && sh[threadIdx.x]) atomicAdd(&dst[threadIdx.x], sh[threadIdx.x]);
-  }
-};
+  __syncthreads();
+  if (tid < 3 && sh[tid]) atomicAdd(&dst[tid], (unsigned long long)sh[tid]);
+}
 
 // >> 4 (2 x 1e-6 phase error + FP32 rounding of a gap).  The phase error
-// budget of 1e-6 covers atan2f (3 ulp) and, for an FP32-mixed field, the
+// budget of 1e-6 covers phase_fast and, for an FP32-mixed field, the
 // Kahan compensation the FP32 phase leaves out (|c| <= ulp(phi) / 2, so
 // <= 1.2e-7 rad).
 constexpr float kMargin = 2e-5f;
@@ -161,18 +173,26 @@ __device__ __forceinline__ void cswapf(float &a, float &b) {
   a = lo;
   b = hi;
 }
-__device__ __forceinline__ void sort8f(float v[8]) {
-  cswapf(v[0], v[1]); cswapf(v[2], v[3]); cswapf(v[4], v[5]); cswapf(v[6], v[7]);
-  cswapf(v[0], v[2]); cswapf(v[1], v[3]); cswapf(v[4], v[6]); cswapf(v[5], v[7]);
-  cswapf(v[1], v[2]); cswapf(v[5], v[6]); cswapf(v[0], v[4]); cswapf(v[3], v[7]);
-  cswapf(v[1], v[5]); cswapf(v[2], v[6]);
-  cswapf(v[1], v[4]); cswapf(v[3], v[6]);
+// four values in ascending order (5 comparators)
+__device__ __forceinline__ void sort4f(float v[4]) {
+  cswapf(v[0], v[1]); cswapf(v[2], v[3]);
+  cswapf(v[0], v[2]); cswapf(v[1], v[3]);
+  cswapf(v[1], v[2]);
+}
+// two sorted fours into eight (Batcher's odd-even merge, 9 comparators)
+__device__ __forceinline__ void merge44f(const float a[4], const float b[4], float v[8]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[i] = a[i];
+    v[4 + i] = b[i];
+  }
+  cswapf(v[0], v[4]); cswapf(v[1], v[5]); cswapf(v[2], v[6]); cswapf(v[3], v[7]);
   cswapf(v[2], v[4]); cswapf(v[3], v[5]);
-  cswapf(v[3], v[4]);
+  cswapf(v[1], v[2]); cswapf(v[3], v[4]); cswapf(v[5], v[6]);
 }
 
 // id_with_phase on FP32 phases; false when a decision lies inside the margin
-__device__ __forceinline__ bool classify_sorted_f(const float p[8], int which, int8_t &flag) {
+__device__ __forceinline__ bool classify_sorted_f(const float p[8], int which, int &flag) {
   flag = 0;
   const float t = p[0] - p[7] + (float)kRefTwoPi;
   float tmax = p[1] - p[0];
@@ -216,41 +236,151 @@ __global__ void k_phase64_all(const V *__restrict__ phi, const V *__restrict__ c
     ph[s] = phase64(phi, cphi, s);
 }
 
-template <typename V>
-__global__ void k_classify(const float *__restrict__ ph, const V *__restrict__ phi, const V *__restrict__ cphi, int n,
-                           int which,
-                           int8_t *__restrict__ flags, unsigned long long *__restrict__ counts) {
-  const int64_t n3 = (int64_t)n * n * n;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  BlockCount3 tally;
-  // uniform trip count so every lane reaches the ballots
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n3; base += stride) {
-    const int64_t s = base + threadIdx.x;
-    int8_t f = 0;
-    if (s < n3) {
-      const int ix = (int)(s % n), iy = (int)((s / n) % n), iz = (int)(s / ((int64_t)n * n));
-      float v[8];
-      bool known = true;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        v[c] = ph[corner(n, ix, iy, iz, c)];
-        known = known && !isnan(v[c]);
+// The cell passes.  A CTA owns 32 x kCellY columns of cells and walks zc
+// planes: each plane of (32 + 1) x (kCellY + 1) phases is formed from phi in
+// shared memory (the next two planes' phi are in flight), a thread reads the
+// four corners of its cell in that plane and keeps those of the plane below.
+// One read of phi and one write of the result; phases are never stored.
+// cell(x, y, z, lower, upper): corner dy 2 + dx of the cell's lower and upper
+// plane, returns the cell's packed counts, or a negative value when FP32
+// cannot decide it.  Those cells are queued and decided at the end by
+// exact(x, y, z, corners) from their FP64 phases, 32 cells at a time with a
+// thread per corner phase (done where they turn up, one lane of a warp at a
+// time, they took half of a 64^3 pass, and their FP64 chains held registers
+// throughout the march; with a thread per cell a single queued cell took 14 us).
+//
+// Before, the phases went through HBM (12 + 4 B a site) and each cell loaded
+// its eight corners with 64-bit index divisions, ~390 instructions a cell; now
+// it is ~155, and the issue slots bound the passes (76 and 85 % busy under
+// ncu).  512^3 FP32: classification 1.69 -> 0.66 ms, winding 1.94 -> 0.57;
+// 128^3: 66 -> 23 and 54 -> 17 us.  3 to 6 CTAs per SM measured 0.67-0.76 ms.
+constexpr int kCellX = 32, kCellY = 8, kCellZ = 32;  // at most kCellZ planes: the queue holds every cell of the CTA
+template <typename V, typename Cell, typename Exact>
+__device__ __forceinline__ unsigned cell_march(const V *__restrict__ phi, const V *__restrict__ cphi, int n, int zc,
+                                               float unknown, Cell cell, Exact exact) {
+  constexpr int W = kCellX + 1, H = kCellY + 1, NT = kCellX * kCellY;
+  __shared__ float ph[2][H * W];
+  __shared__ uint16_t queue[NT * kCellZ];
+  __shared__ double exact_ph[NT];
+  __shared__ int queued;
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kCellX + tx;
+  const int x0 = blockIdx.x * kCellX, y0 = blockIdx.y * kCellY, z0 = blockIdx.z * zc;
+  const int nz = min(zc, n - z0);
+  auto wrap = [n](int i) { return i >= n ? i - n : i; };
+  // a thread's own site and, for the first W + H - 1 threads, one of the
+  // right column and lower row; past the lattice's edge both repeat site 0
+  const int x = x0 + tx, y = y0 + ty;
+  const bool live = x < n && y < n, halo = tid < W + H - 1;
+  const int hx = tid < W ? tid : W - 1, hy = tid < W ? H - 1 : tid - W;
+  const int own = wrap(min(y, n)) * n + wrap(min(x, n)), rim = wrap(min(y0 + hy, n)) * n + wrap(min(x0 + hx, n));
+  const int64_t n2 = (int64_t)n * n;
+  // planes z0 .. z0 + nz; the last one is plane 0 when the walk ends at n
+  const V *pa = phi + z0 * n2 + own, *pb = phi + z0 * n2 + rim;
+  const int64_t last = z0 + nz == n ? -(int64_t)(n - 1) * n2 : n2;  // from plane z0 + nz - 1 to the last
+  V a = pa[0], b = a, a1, b1;
+  if (halo) b = pb[0];
+  auto advance = [&](int k) {  // a1, b1: plane z0 + k
+    const int64_t step = k == nz ? last : n2;
+    pa += step;
+    pb += step;
+    a1 = *pa;
+    if (halo) b1 = *pb;
+  };
+  b1 = b;
+  advance(1);
+  if (tid == 0) queued = 0;
+  float lo[4];
+  unsigned counts = 0;
+  const int slot = ty * W + tx, hslot = hy * W + hx;
+#pragma unroll 2
+  for (int k = 0; k <= nz; ++k) {
+    float *s = ph[k & 1];
+    s[slot] = phase_of(a, unknown);
+    if (halo) s[hslot] = phase_of(b, unknown);
+    a = a1;
+    b = b1;
+    if (k + 2 <= nz) advance(k + 2);
+    __syncthreads();
+    const float *c = s + slot;
+    const float hi[4] = {c[0], c[1], c[W], c[W + 1]};
+    if (k > 0 && live) {
+      const int r = cell(x, y, z0 + k - 1, lo, hi);
+      if (r >= 0) {
+        counts += (unsigned)r;
+      } else {
+        queue[atomicAdd(&queued, 1)] = (uint16_t)((k - 1) * NT + tid);
       }
-      if (known) {
-        sort8f(v);
-        known = classify_sorted_f(v, which, f);
-      }
-      if (!known) {  // the FP64 classification of the host
-        double d[8];
-        for (int c = 0; c < 8; ++c) d[c] = phase64(phi, cphi, corner(n, ix, iy, iz, c));
-        sort8(d);
-        f = classify_sorted(d, which);
-      }
-      flags[s] = f;
     }
-    tally.add((f & 1) != 0, (f & 2) != 0, (f & 4) != 0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) lo[i] = hi[i];
   }
-  tally.flush(counts);
+  __syncthreads();
+  for (int q0 = 0; q0 < queued; q0 += NT / 8) {
+    auto site = [&](int q, int &cx, int &cy, int &cz) {
+      const int e = queue[q];
+      cx = x0 + e % kCellX;
+      cy = y0 + e / kCellX % kCellY;
+      cz = z0 + e / NT;
+    };
+    int cx, cy, cz;
+    if (q0 + tid / 8 < queued) {
+      site(q0 + tid / 8, cx, cy, cz);
+      exact_ph[tid] = phase64(phi, cphi, corner(n, cx, cy, cz, tid & 7));
+    }
+    __syncthreads();
+    if (tid < NT / 8 && q0 + tid < queued) {
+      site(q0 + tid, cx, cy, cz);
+      double d[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) d[c] = exact_ph[8 * tid + c];
+      counts += exact(cx, cy, cz, d);
+    }
+    __syncthreads();
+  }
+  static_assert(NT >= W + H - 1, "one halo site per thread");
+  static_assert(NT * kCellZ <= 65536, "queue entries of 16 bits");
+  return counts;
+}
+
+// WHICH: the flags asked for, or -1 for those of `flags_wanted`
+template <typename V, int WHICH>
+__global__ void __launch_bounds__(kCellX *kCellY, 5) k_classify(const V *__restrict__ phi,
+                                                                const V *__restrict__ cphi, int n, int zc,
+                                                                int flags_wanted,
+                                                                int8_t *__restrict__ flags,
+                                                                unsigned long long *__restrict__ counts) {
+  const int which = WHICH >= 0 ? WHICH : flags_wanted;
+  constexpr float kUnknown = 1e30f;  // sorts last
+  float sorted[4];                   // the lower plane's corners in order, from the cell below
+  const int64_t n2 = (int64_t)n * n;
+  int8_t *dst = flags + ((int64_t)blockIdx.z * zc * n + blockIdx.y * kCellY + threadIdx.y) * n + blockIdx.x * kCellX +
+                threadIdx.x;
+  auto pack = [](int flag) { return (flag & 1) | (flag & 2) << 9 | (flag & 4) << 18; };
+  const int zfirst = blockIdx.z * zc;
+  auto cell = [&](int, int, int z, const float lo[4], const float hi[4]) {
+    if (z == zfirst) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sorted[i] = lo[i];
+      sort4f(sorted);
+    }
+    float up[4] = {hi[0], hi[1], hi[2], hi[3]}, v[8];
+    sort4f(up);
+    merge44f(sorted, up, v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sorted[i] = up[i];
+    int f;
+    const bool sure = classify_sorted_f(v, which, f) && v[7] < 4.0f;
+    *dst = (int8_t)f;
+    dst += n2;
+    return sure ? pack(f) : -1;
+  };
+  auto exact = [&](int x, int y, int z, double d[8]) {  // the FP64 classification of the host
+    sort8(d);
+    const int f = classify_sorted(d, which);
+    flags[((int64_t)z * n + y) * n + x] = (int8_t)f;
+    return (unsigned)pack(f);
+  };
+  block_tally3(cell_march(phi, cphi, n, zc, kUnknown, cell, exact), counts);
 }
 
 __device__ __forceinline__ double wrapd(double d) {
@@ -267,51 +397,57 @@ __device__ __forceinline__ bool pierced(double a, double b, double c, double d) 
   return w > AXD_PI_HI || w < -AXD_PI_HI;
 }
 
-// plaquette a-b-c-d on FP32 phases; false when a corner difference lies
-// within the margin of the +-pi wrap or a phase is unknown
-__device__ __forceinline__ bool pierced_f(float a, float b, float c, float d, bool &hit) {
-  const float kPi = (float)AXD_PI_HI;
-  const float ds[4] = {b - a, c - b, d - c, a - d};
-  float w = 0.0f;
-  bool sure = true;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float x = ds[k];
-    sure = sure && fabsf(fabsf(x) - kPi) >= kMargin;  // false for NaN too
-    w += x > kPi ? x - 2 * kPi : (x <= -kPi ? x + 2 * kPi : x);
-  }
-  hit = w > kPi || w < -kPi;
-  return sure;
-}
-
+// Plaquette winding.  The raw phase differences around a plaquette sum to
+// zero, so the wrapped ones sum to -2 pi times the sum of the links' wrap
+// numbers rint(d / 2 pi), and the plaquette is pierced when those do not
+// cancel.  A link's number is the FP64 one unless |d| lies within kMargin of
+// pi; then, or with a phase unknown, the site's plaquettes are redone in FP64.
 template <typename V>
-__global__ void k_winding(const float *__restrict__ ph, const V *__restrict__ phi, const V *__restrict__ cphi, int n,
-                          unsigned long long *__restrict__ counts) {
-  const int64_t n2 = (int64_t)n * n, n3 = n2 * n;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  BlockCount3 tally;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n3; base += stride) {
-    const int64_t s = base + threadIdx.x;
-    bool hit[3] = {false, false, false};
-    if (s < n3) {
-      const int ix = (int)(s % n), iy = (int)((s / n) % n), iz = (int)(s / n2);
-      const int x1 = ix + 1 == n ? 0 : ix + 1, y1 = iy + 1 == n ? 0 : iy + 1,
-                z1 = iz + 1 == n ? 0 : iz + 1;
-      auto S = [&](int x, int y, int z) { return ((int64_t)z * n + y) * n + x; };
-      // corners of the x, y, z plaquettes (counts[0..2] = px, py, pz)
-      const int64_t q[3][4] = {{S(ix, iy, iz), S(ix, y1, iz), S(ix, y1, z1), S(ix, iy, z1)},
-                               {S(ix, iy, iz), S(ix, iy, z1), S(x1, iy, z1), S(x1, iy, iz)},
-                               {S(ix, iy, iz), S(x1, iy, iz), S(x1, y1, iz), S(ix, y1, iz)}};
+__global__ void __launch_bounds__(kCellX *kCellY, 5) k_winding(const V *__restrict__ phi,
+                                                               const V *__restrict__ cphi, int n, int zc,
+                                                               unsigned long long *__restrict__ counts) {
+  constexpr float kInv = 0.15915494309189534f, kBig = 12582912.0f;  // 1 / 2 pi; 1.5 2^23: adding it rounds to an integer
+  constexpr float kSure = 0.5f - kMargin * kInv;
+  float kx[2] = {0.f, 0.f}, ky[2] = {0.f, 0.f};  // the lower plane's links: x at y, y + 1; y at x, x + 1
+  float far = 0.f;                               // the largest |d / 2 pi - rint| among them
+  const int zfirst = blockIdx.z * zc;
+  auto pack = [](unsigned hit) { return (int)((hit & 1u) | (hit & 2u) << 9 | (hit & 4u) << 18); };
+  auto link = [&](float a, float b, float &m) {
+    const float t = (b - a) * kInv, k = (t + kBig) - kBig;
+    m = fmaxf(m, fabsf(t - k));
+    return k;
+  };
+  auto plane = [&](const float p[4], float lx[2], float ly[2]) {
+    float m = 0.f;
+    lx[0] = link(p[0], p[1], m);
+    lx[1] = link(p[2], p[3], m);
+    ly[0] = link(p[0], p[2], m);
+    ly[1] = link(p[1], p[3], m);
+    return m;
+  };
+  auto cell = [&](int, int, int z, const float lo[4], const float hi[4]) {
+    if (z == zfirst) far = plane(lo, kx, ky);
+    float ux[2], uy[2];
+    const float up = plane(hi, ux, uy);
+    float m = fmaxf(far, up);
+    const float kz = link(lo[0], hi[0], m), kzx = link(lo[1], hi[1], m), kzy = link(lo[2], hi[2], m);
+    const float wx = (ky[0] + kzy) - (uy[0] + kz), wy = (kz + ux[0]) - (kzx + kx[0]), wz = (kx[0] + ky[1]) - (kx[1] + ky[0]);
+    const unsigned hit = (wx != 0.f ? 1u : 0u) | (wy != 0.f ? 2u : 0u) | (wz != 0.f ? 4u : 0u);
+    const float s = (wx + wy) + wz;  // NaN where a phase is
+    const bool sure = m <= kSure && s == s;
+    far = up;
 #pragma unroll
-      for (int o = 0; o < 3; ++o) {
-        if (!pierced_f(ph[q[o][0]], ph[q[o][1]], ph[q[o][2]], ph[q[o][3]], hit[o]))
-          hit[o] = pierced(phase64(phi, cphi, q[o][0]), phase64(phi, cphi, q[o][1]), phase64(phi, cphi, q[o][2]),
-                           phase64(phi, cphi, q[o][3]));
-      }
+    for (int i = 0; i < 2; ++i) {
+      kx[i] = ux[i];
+      ky[i] = uy[i];
     }
-    tally.add(hit[0], hit[1], hit[2]);
-  }
-  tally.flush(counts);
+    return sure ? pack(hit) : -1;
+  };
+  auto exact = [&](int, int, int, const double p[8]) {  // corner c = dx + 2 dy + 4 dz
+    return (unsigned)pack((pierced(p[0], p[2], p[6], p[4]) ? 1u : 0u) | (pierced(p[0], p[4], p[5], p[1]) ? 2u : 0u) |
+                          (pierced(p[0], p[1], p[3], p[2]) ? 4u : 0u));
+  };
+  block_tally3(cell_march(phi, cphi, n, zc, __int_as_float(0x7fc00000), cell, exact), counts);
 }
 
 // ---------------- compaction in cell order ----------------
@@ -1708,22 +1844,14 @@ int grid_for(int64_t count, int per = 256) {
   return (int)(b < 1 ? 1 : b);
 }
 
-int ensure_scratch(axg_ctx *ctx) {
-  if (!ctx->phase) AXG_TRY(axg_alloc(ctx, (void **)&ctx->phase, (size_t)ctx->n3 * 4, "phase"));
-  if (!ctx->flags) AXG_TRY(axg_alloc(ctx, (void **)&ctx->flags, (size_t)ctx->n3, "defect flags"));
-  return AXG_OK;
-}
-
-int compute_phases(axg_ctx *ctx) {
-  AXG_TRY(ensure_scratch(ctx));
-  const void *phi = ctx->phi[ctx->cur];
-  if (ctx->p.precision == AXG_PREC_FP32_MIXED)
-    AXG_LAUNCH(ctx, "defect_phase_fp32", k_phase32<float2>, grid_for(ctx->n3), 256, 0,
-               (const float2 *)phi, ctx->phase, ctx->n3);
-  else
-    AXG_LAUNCH(ctx, "defect_phase_fp64", k_phase32<double2>, grid_for(ctx->n3), 256, 0,
-               (const double2 *)phi, ctx->phase, ctx->n3);
-  return AXG_OK;
+// planes a CTA of the cell passes walks: 32 (one extra plane of phases in 32),
+// fewer on small lattices so that about four CTAs per SM remain
+dim3 cell_grid(int n, int *zc) {
+  const unsigned gx = (unsigned)((n + kCellX - 1) / kCellX), gy = (unsigned)((n + kCellY - 1) / kCellY);
+  int c = kCellZ;
+  while (c > 2 && (int64_t)gx * gy * ((n + c - 1) / c) < 4 * 152) c /= 2;
+  *zc = c;
+  return dim3(gx, gy, (unsigned)((n + c - 1) / c));
 }
 
 // grouping_strings / grouping_walls + the grouped branch of add_string_length
@@ -1782,16 +1910,25 @@ double group_threshold(double wid, double hor) {
 }  // namespace
 
 int axg_def_classify(axg_ctx *ctx, int which, int64_t counts[3]) {
-  AXG_TRY(compute_phases(ctx));
+  if (!ctx->flags) AXG_TRY(axg_alloc(ctx, (void **)&ctx->flags, (size_t)ctx->n3, "defect flags"));
   AXG_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_cnt, 0, 3 * sizeof(unsigned long long), ctx->stream));
-  if (ctx->p.precision == AXG_PREC_FP32_MIXED)
-    AXG_LAUNCH(ctx, "defect_classify", k_classify<float2>, grid_for(ctx->n3), 256, 0, ctx->phase,
-               (const float2 *)ctx->phi[ctx->cur], (const float2 *)ctx->cphi, (int)ctx->n, which, ctx->flags,
-               ctx->d_cnt);
+  const int n = (int)ctx->n;
+  int zc;
+  const dim3 grid = cell_grid(n, &zc), block(kCellX, kCellY);
+  const bool f32 = ctx->p.precision == AXG_PREC_FP32_MIXED;
+  const auto *c32 = (const float2 *)ctx->cphi;
+  if (f32 && which == 7)
+    AXG_LAUNCH(ctx, "defect_classify", (k_classify<float2, 7>), grid, block, 0, (const float2 *)ctx->phi[ctx->cur], c32,
+               n, zc, which, ctx->flags, ctx->d_cnt);
+  else if (f32)
+    AXG_LAUNCH(ctx, "defect_classify", (k_classify<float2, -1>), grid, block, 0, (const float2 *)ctx->phi[ctx->cur], c32,
+               n, zc, which, ctx->flags, ctx->d_cnt);
+  else if (which == 7)
+    AXG_LAUNCH(ctx, "defect_classify", (k_classify<double2, 7>), grid, block, 0, (const double2 *)ctx->phi[ctx->cur],
+               (const double2 *)nullptr, n, zc, which, ctx->flags, ctx->d_cnt);
   else
-    AXG_LAUNCH(ctx, "defect_classify", k_classify<double2>, grid_for(ctx->n3), 256, 0, ctx->phase,
-               (const double2 *)ctx->phi[ctx->cur], (const double2 *)nullptr, (int)ctx->n, which, ctx->flags,
-               ctx->d_cnt);
+    AXG_LAUNCH(ctx, "defect_classify", (k_classify<double2, -1>), grid, block, 0, (const double2 *)ctx->phi[ctx->cur],
+               (const double2 *)nullptr, n, zc, which, ctx->flags, ctx->d_cnt);
   unsigned long long h[3];
   AXG_CUDA_TRY(ctx, cudaMemcpyAsync(h, ctx->d_cnt, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
   AXG_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1804,14 +1941,16 @@ int axg_def_classify(axg_ctx *ctx, int which, int64_t counts[3]) {
 }
 
 int axg_def_winding(axg_ctx *ctx, int64_t counts[3]) {
-  AXG_TRY(compute_phases(ctx));
   AXG_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_cnt + 3, 0, 3 * sizeof(unsigned long long), ctx->stream));
+  const int n = (int)ctx->n;
+  int zc;
+  const dim3 grid = cell_grid(n, &zc), block(kCellX, kCellY);
   if (ctx->p.precision == AXG_PREC_FP32_MIXED)
-    AXG_LAUNCH(ctx, "string_winding", k_winding<float2>, grid_for(ctx->n3), 256, 0, ctx->phase,
-               (const float2 *)ctx->phi[ctx->cur], (const float2 *)ctx->cphi, (int)ctx->n, ctx->d_cnt + 3);
+    AXG_LAUNCH(ctx, "string_winding", k_winding<float2>, grid, block, 0, (const float2 *)ctx->phi[ctx->cur],
+               (const float2 *)ctx->cphi, n, zc, ctx->d_cnt + 3);
   else
-    AXG_LAUNCH(ctx, "string_winding", k_winding<double2>, grid_for(ctx->n3), 256, 0, ctx->phase,
-               (const double2 *)ctx->phi[ctx->cur], (const double2 *)nullptr, (int)ctx->n, ctx->d_cnt + 3);
+    AXG_LAUNCH(ctx, "string_winding", k_winding<double2>, grid, block, 0, (const double2 *)ctx->phi[ctx->cur],
+               (const double2 *)nullptr, n, zc, ctx->d_cnt + 3);
   unsigned long long h[3];
   AXG_CUDA_TRY(ctx, cudaMemcpyAsync(h, ctx->d_cnt + 3, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
   AXG_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));

@@ -1040,8 +1040,9 @@ struct StepShape {
 //    4.2 / 12.4 at 32^3, 36.5 / 40 at 160^3, 88.5 / 92 at 224^3, 129 / 126 at
 //    256^3, 1000 / 927 at 512^3;
 //  * FP64 is bound by the FP64 pipe; the plain kernel's many small CTAs fill
-//    it best (14.5 against 107 at 32^3, 598 / 720 at 128^3, 4.76 / 4.79 ms at
-//    256^3);
+//    it best (12.4 against 109 at 32^3, 415 / 487 at 128^3) until lattices
+//    outgrow the L2 (3.26 / 3.18 ms at 256^3, 26.3 / 25.2 at 512^3, tile
+//    32 x 4 x 32; phi alone 6.62 / 6.68);
 //  * TMA needs rows of a multiple of 16 bytes: N a multiple of 4;
 //  * of the TMA tiles 32 x 8 x 32 moves the fewest halo bytes (3.90 against
 //    4.08 ms at 512^3) unless its larger CTAs leave the last of their waves
@@ -1060,8 +1061,9 @@ StepShape step_shape(const axg_ctx *ctx) {
   if (asked) return plain;
   if (ctx->tile_cfg >= 0 && axg_evo_tile_supported(ctx, ctx->tile_cfg))
     return {ctx->tile_cfg, kTiles[ctx->tile_cfg].zc, false};
+  constexpr int kTile8 = 8, kTile4 = 10, kTile64 = 7;  // 32 x 8 x 32, 32 x 4 x 16, 32 x 4 x 32, pointwise fields by TMA
+  if (!fp32 && uij && n >= 256 && n % 32 == 0) return {kTile64, kTiles[kTile64].zc, false};
   if (!fp32 || (n & 3) || n <= (uij ? 80 : 224)) return plain;
-  constexpr int kTile8 = 8, kTile4 = 10;  // 32 x 8 x 32 and 32 x 4 x 16, pointwise fields by TMA
   const double waves = (double)((n + 31) / 32) * ((n + 7) / 8) * ((n + 31) / 32) / (2 * 152);
   const int cfg = uij && waves > 0.83 * std::ceil(waves) ? kTile8 : kTile4;
   const int chunks = (n + kTiles[cfg].zc - 1) / kTiles[cfg].zc;
