@@ -519,7 +519,7 @@ int axg_destroy(axg_ctx *ctx) {
                    &ctx->ud, &ctx->cu, (void **)&ctx->acc, (void **)&ctx->gsrc, (void **)&ctx->gw_omega,
                    (void **)&ctx->gw_pol, (void **)&ctx->ff_tw, (void **)&ctx->gsrcF, (void **)&ctx->flags,
                    (void **)&ctx->phase64, (void **)&ctx->d_strings, (void **)&ctx->d_walls, (void **)&ctx->spec_mat,
-                   (void **)&ctx->spec_largeq0, (void **)&ctx->spec_dq, (void **)&ctx->spec_buf,
+                   (void **)&ctx->spec_largeq0, (void **)&ctx->spec_dq, (void **)&ctx->spec_modes, (void **)&ctx->spec_range, (void **)&ctx->spec_buf,
                    &ctx->ubuf, (void **)&ctx->d_red, (void **)&ctx->d_cnt, (void **)&ctx->d_err})
     axg_free(ctx, q);
   if (ctx->plan_gsrc_ok) cufftDestroy(ctx->plan_gsrc);

@@ -111,8 +111,14 @@ __device__ __forceinline__ T c_zero() {
   return z;
 }
 
-// a complex float-float from two doubles (re, im)
-__device__ __forceinline__ float4 c_from(double2 x) { return cx(f2_from(x.x), f2_from(x.y)); }
+// a complex float-float from two doubles (re, im), split on the integer
+// pipes (zeros, common in masked fields, past f2_from_bits' FP64 branch): by
+// conversions, 8 FP64-pipe operations, the complex row pass was bound by the
+// FP64 pipe, 254 us at 256^3
+__device__ __forceinline__ F2 f2_split(double x) {
+  return (__double_as_longlong(x) << 1) == 0 ? F2{0.f, 0.f} : f2_from_bits(x);
+}
+__device__ __forceinline__ float4 c_from(double2 x) { return cx(f2_split(x.x), f2_split(x.y)); }
 
 // In-register DFTs of 2, 4 and 8 points, natural order in and out; INV uses
 // exp(+2 pi i / R).  The 8-point one is two 4-point DFTs of the even and odd
@@ -330,10 +336,46 @@ constexpr int kFfRows = 8;   // rows per CTA of the float-float real row pass
 constexpr int kFfCRows = 4;  // rows per CTA of the float-float complex row pass
 constexpr int kFfCols = 4;   // kx columns per CTA of the float-float column passes (64 bytes)
 
+// What a row pass transforms: element pair m (real rows) or element x (complex
+// rows) of row r.  Doubles from memory, the window of the field spectrum
+// (dv on cells whose flag bit 4 is clear), or the field masked by the flags,
+// formed here so that neither is stored first.
+struct LoadReals {
+  const double *in;
+  __device__ __forceinline__ float4 pair(int64_t r, int n, int m) const {
+    return c_from(reinterpret_cast<const double2 *>(in + r * n)[m]);
+  }
+};
+struct LoadWindow {
+  const int8_t *flags;
+  float hi, lo;  // dv
+  __device__ __forceinline__ float4 pair(int64_t r, int n, int m) const {
+    const char2 f = reinterpret_cast<const char2 *>(flags + r * n)[m];
+    const bool a = f.x & 4, b = f.y & 4;
+    return make_float4(a ? 0.f : hi, a ? 0.f : lo, b ? 0.f : hi, b ? 0.f : lo);
+  }
+};
+struct LoadComplex {
+  const double2 *in;
+  __device__ __forceinline__ float4 at(int64_t r, int n, int x) const { return c_from(in[r * n + x]); }
+};
+template <typename V>
+struct LoadMasked {
+  const V *in;
+  const int8_t *flags;
+  __device__ __forceinline__ float4 at(int64_t r, int n, int x) const {
+    const int64_t i = r * n + x;
+    const V v = in[i];
+    if (flags[i] & 4) return make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (sizeof(v.x) == 4) return make_float4(v.x, 0.f, v.y, 0.f);
+    else return c_from(v);
+  }
+};
+
 // Row pass: kFfRows rows of N = 2M reals -> M + 1 complex each (float-float).
-template <int M>
-__global__ void __launch_bounds__(kFfRows * M / 8) k_ff_rows(const double *__restrict__ in, float4 *__restrict__ out,
-                                                             int64_t rows, const float4 *__restrict__ twff) {
+template <int M, typename Load>
+__global__ void __launch_bounds__(kFfRows * M / 8) k_ff_rows(const Load in, float4 *__restrict__ out, int64_t rows,
+                                                             const float4 *__restrict__ twff) {
   constexpr int N = 2 * M, NH = M + 1, TH = M / 8, LP = M + M / 8;
   __shared__ float4 s[kFfRows * LP];
   __shared__ float4 tw[N];  // W_N^k, k < N
@@ -341,10 +383,9 @@ __global__ void __launch_bounds__(kFfRows * M / 8) k_ff_rows(const double *__res
   const int64_t r0 = (int64_t)blockIdx.x * kFfRows;
   const int ln = threadIdx.x / TH, j = threadIdx.x % TH;
   const bool ok = r0 + ln < rows;
-  const double2 *x = reinterpret_cast<const double2 *>(in + (r0 + ln) * N);
   float4 v[8];
 #pragma unroll
-  for (int r = 0; r < 8; ++r) v[r] = ok ? c_from(x[j + r * TH]) : c_zero<float4>();
+  for (int r = 0; r < 8; ++r) v[r] = ok ? in.pair(r0 + ln, N, j + r * TH) : c_zero<float4>();
   __syncthreads();  // twiddles
   float4 *line = s + ln * LP;
   f_stockham<M, 1, false>(v, j, line, 1, tw, 2, [&](int i, float4 z) { line[fpad(i)] = z; });  // W_M = W_N^2
@@ -355,11 +396,11 @@ __global__ void __launch_bounds__(kFfRows * M / 8) k_ff_rows(const double *__res
   }
 }
 
-// Complex row pass: kFfCRows contiguous rows of L complex doubles -> L
-// float-float points each, transformed in place of the input (each CTA
+// Complex row pass: kFfCRows contiguous rows of L complex values -> L
+// float-float points each; the output may take the input's place (each CTA
 // reads all of its rows before it writes).
-template <int L, bool INV>
-__global__ void __launch_bounds__(kFfCRows * L / 8) k_ff_rows_c2c(double2 *__restrict__ data, int64_t rows,
+template <int L, bool INV, typename Load>
+__global__ void __launch_bounds__(kFfCRows * L / 8) k_ff_rows_c2c(const Load in, float4 *data, int64_t rows,
                                                                   const float4 *__restrict__ twff) {
   constexpr int TH = L / 8, LP = L + L / 8;
   __shared__ float4 s[kFfCRows * LP];
@@ -370,9 +411,9 @@ __global__ void __launch_bounds__(kFfCRows * L / 8) k_ff_rows_c2c(double2 *__res
   const bool ok = r0 + ln < rows;
   float4 v[8];
 #pragma unroll
-  for (int r = 0; r < 8; ++r) v[r] = ok ? c_from(data[(r0 + ln) * L + j + r * TH]) : c_zero<float4>();
+  for (int r = 0; r < 8; ++r) v[r] = ok ? in.at(r0 + ln, L, j + r * TH) : c_zero<float4>();
   __syncthreads();
-  float4 *out = reinterpret_cast<float4 *>(data) + (r0 + ln) * L;
+  float4 *out = data + (r0 + ln) * L;
   f_stockham<L, 1, INV>(v, j, s + ln * LP, 1, tw, 1, [&](int i, float4 z) {
     if (ok) out[i] = z;
   });
@@ -434,18 +475,18 @@ int launch_cols(axg_ctx *ctx, const char *name, int64_t blocks, T *data, int nh,
   return AXG_OK;
 }
 
-template <int L, bool INV>
-int z2z_t(axg_ctx *ctx, double2 *data, const float4 *tw) {
+template <int L, bool INV, typename Load>
+int z2z_t(axg_ctx *ctx, const Load &in, double2 *data, const float4 *tw, bool keep_ff) {
   constexpr int n = L;
   const int64_t rows = (int64_t)n * n, plane = (int64_t)n * n, vol = plane * n;
   float4 *f = reinterpret_cast<float4 *>(data);
-  AXG_LAUNCH(ctx, "fft_ff_rows_c2c", (k_ff_rows_c2c<L, INV>), (unsigned)((rows + kFfCRows - 1) / kFfCRows),
-             kFfCRows * L / 8, 0, data, rows, tw);
+  AXG_LAUNCH(ctx, "fft_ff_rows_c2c", (k_ff_rows_c2c<L, INV, Load>), (unsigned)((rows + kFfCRows - 1) / kFfCRows),
+             kFfCRows * L / 8, 0, in, f, rows, tw);
   const int nkb = n / kFfCols;
   AXG_TRY((launch_cols<float4, L, kFfCols, INV>(ctx, "fft_ff_y", (int64_t)n * nkb, f, n, n, vol, plane, (int64_t)n,
                                                  tw, 0)));
   AXG_TRY((launch_cols<float4, L, kFfCols, INV>(ctx, "fft_ff_z", (int64_t)n * nkb, f, n, n, vol, (int64_t)n, plane,
-                                                 tw, 1)));
+                                                 tw, keep_ff ? 0 : 1)));
   return AXG_OK;
 }
 
@@ -463,13 +504,13 @@ int d2z_cols_t(axg_ctx *ctx, float4 *f, int batch, const float4 *tw, bool keep_f
   return AXG_OK;
 }
 
-template <int L>
-int d2z_t(axg_ctx *ctx, const double *in, double2 *out, int batch, const float4 *tw, bool keep_ff) {
+template <int L, typename Load>
+int d2z_t(axg_ctx *ctx, const Load &in, double2 *out, int batch, const float4 *tw, bool keep_ff) {
   constexpr int n = L;
   const int64_t rows = (int64_t)batch * n * n;
   float4 *f = reinterpret_cast<float4 *>(out);
-  AXG_LAUNCH(ctx, "fft_ff_rows", k_ff_rows<L / 2>, (unsigned)((rows + kFfRows - 1) / kFfRows), kFfRows * L / 16, 0,
-             in, f, rows, tw);
+  AXG_LAUNCH(ctx, "fft_ff_rows", (k_ff_rows<L / 2, Load>), (unsigned)((rows + kFfRows - 1) / kFfRows),
+             kFfRows * L / 16, 0, in, f, rows, tw);
   return d2z_cols_t<L>(ctx, f, batch, tw, keep_ff);
 }
 
@@ -921,12 +962,15 @@ int ensure_twiddles(axg_ctx *ctx, int n) {
 }
 }  // namespace
 
-int axg_ff_z2z(axg_ctx *ctx, double2 *data, int n, int inverse) {
+namespace {
+template <typename Load>
+int z2z_n(axg_ctx *ctx, const Load &in, double2 *data, int n, int inverse, bool keep_ff) {
   if (!axg_ff_fft_supported(n)) return axg_set_error(ctx, AXG_ERR_UNSUPPORTED, "float-float FFT size");
   AXG_TRY(ensure_twiddles(ctx, n));
   const float4 *tw = reinterpret_cast<const float4 *>(ctx->ff_tw);
-#define AXG_FF_Z2Z(L) \
-  case L: return inverse ? z2z_t<L, true>(ctx, data, tw) : z2z_t<L, false>(ctx, data, tw);
+#define AXG_FF_Z2Z(L)                                                              \
+  case L:                                                                          \
+    return inverse ? z2z_t<L, true, Load>(ctx, in, data, tw, keep_ff) : z2z_t<L, false, Load>(ctx, in, data, tw, keep_ff);
   switch (n) {
     AXG_FF_Z2Z(16)
     AXG_FF_Z2Z(32)
@@ -939,7 +983,8 @@ int axg_ff_z2z(axg_ctx *ctx, double2 *data, int n, int inverse) {
 #undef AXG_FF_Z2Z
 }
 
-int axg_ff_d2z(axg_ctx *ctx, const double *in, double2 *out, int n, int batch, bool keep_ff) {
+template <typename Load>
+int d2z_n(axg_ctx *ctx, const Load &in, double2 *out, int n, int batch, bool keep_ff) {
   if (!axg_ff_fft_supported(n)) return axg_set_error(ctx, AXG_ERR_UNSUPPORTED, "float-float FFT size");
   AXG_TRY(ensure_twiddles(ctx, n));
   const float4 *tw = reinterpret_cast<const float4 *>(ctx->ff_tw);
@@ -952,6 +997,26 @@ int axg_ff_d2z(axg_ctx *ctx, const double *in, double2 *out, int n, int batch, b
     case 512: return d2z_t<512>(ctx, in, out, batch, tw, keep_ff);
     default: return axg_set_error(ctx, AXG_ERR_UNSUPPORTED, "float-float FFT size");
   }
+}
+}  // namespace
+
+int axg_ff_z2z(axg_ctx *ctx, double2 *data, int n, int inverse, bool keep_ff) {
+  return z2z_n(ctx, LoadComplex{data}, data, n, inverse, keep_ff);
+}
+
+int axg_ff_z2z_masked(axg_ctx *ctx, const void *field, bool fp32, const int8_t *flags, double2 *out, int n,
+                      int inverse) {
+  if (fp32) return z2z_n(ctx, LoadMasked<float2>{(const float2 *)field, flags}, out, n, inverse, true);
+  return z2z_n(ctx, LoadMasked<double2>{(const double2 *)field, flags}, out, n, inverse, true);
+}
+
+int axg_ff_d2z(axg_ctx *ctx, const double *in, double2 *out, int n, int batch, bool keep_ff) {
+  return d2z_n(ctx, LoadReals{in}, out, n, batch, keep_ff);
+}
+
+int axg_ff_d2z_window(axg_ctx *ctx, const int8_t *flags, double dv, double2 *out, int n) {
+  const float hi = (float)dv;
+  return d2z_n(ctx, LoadWindow{flags, hi, (float)(dv - (double)hi)}, out, n, 1, true);
 }
 
 int axg_gw_source_r2c_f32(axg_ctx *ctx, const float2 *phi, float2 *out, int n, float scale) {

@@ -642,60 +642,53 @@ __global__ void __launch_bounds__(256, 4) k_gw_accumulate_f32(const float2 *__re
 // ---------------- shell histograms ----------------
 constexpr int kMaxBins = 256;
 
-// |A|^2 of one accumulator entry: FP64, or float-float (FP32-mixed)
-__device__ __forceinline__ double acc_norm2(double2 z) { return z.x * z.x + z.y * z.y; }
-__device__ __forceinline__ double acc_norm2(float4 z) {
-  const double re = (double)z.x + (double)z.y, im = (double)z.z + (double)z.w;
-  return re * re + im * im;
+// sum of |A|^2 over the four accumulators of an entry: FP64, or float-float
+__device__ __forceinline__ double acc_norm2(const double2 *__restrict__ acc, int64_t astride, int64_t h) {
+  double v = 0.0;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const double2 z = acc[a * astride + h];
+    v += z.x * z.x + z.y * z.y;
+  }
+  return v;
 }
-
+__device__ __forceinline__ F2 acc_norm2(const float4 *__restrict__ acc, int64_t astride, int64_t h) {
+  F2 v = {0.f, 0.f};
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const float4 z = acc[a * astride + h];
+    const F2 r = {z.x, z.y}, i = {z.z, z.w};
+    v = f2_add(v, f2_dot2(r, r, i, i, 1.f));
+  }
+  return v;
+}
 // Green accumulators -> numer / denom per bin (bin of |k|^2 from the table).
 // A stored entry with 0 < hx < n/2 stands for k and -k (the same |k|): its
 // |A|^2 counts twice, or once plus the Nyquist-row mirror's own entry.
+// Float-float accumulators are squared and summed as such: with 16
+// conversions and 16 FP64 operations an entry the FP64 pipe took 4.19 ms at
+// 512^3, now 0.77 (64 B an entry: 0.83 of the copy peak).
 template <typename A>
-__global__ void k_gw_bin_green(const A *__restrict__ acc, int n, int64_t astride, const int16_t *__restrict__ tab,
-                               int nb, double *__restrict__ numer, double *__restrict__ denom) {
-  __shared__ double sn[kMaxBins], sd[kMaxBins];
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) sn[b] = sd[b] = 0.0;
-  __syncthreads();
+__global__ void __launch_bounds__(256) k_gw_bin_green(const A *__restrict__ acc, int n, int64_t astride, int rows,
+                                                      const int16_t *__restrict__ tab, int nb, int copies,
+                                                      double *__restrict__ numer, double *__restrict__ denom) {
+  BlockBins bins(nb, copies);
   const int nh = n / 2 + 1;
   const int64_t nhalf = (int64_t)n * n * nh;
-  BinRun run;
-  for (int64_t h0 = run_start(); h0 < nhalf; h0 += run_stride()) {
-    for (int64_t h = h0; h < h0 + kRun && h < nhalf; ++h) {
-      const int hx = (int)(h % nh), hy = (int)((h / nh) % n), hz = (int)(h / ((int64_t)nh * n));
-      const int kx = kint(hx, n), ky = kint(hy, n), kz = kint(hz, n);
-      const int b = tab[kx * kx + ky * ky + kz * kz];
-      const bool mirror = hx > 0 && hx < n / 2;
-      double v = 0.0;
-      if (b >= 0) {
-        double v1 = 0.0;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) v1 += acc_norm2(acc[a * astride + h]);
-        v = v1;
-        if (mirror) {
-          if (hy == n / 2 || hz == n / 2) {
-            const int64_t e = nhalf + gw_nyq_extra(hx, hy, hz, n);
-            double v2 = 0.0;
-#pragma unroll
-            for (int a = 0; a < 4; ++a) v2 += acc_norm2(acc[a * astride + e]);
-            v += v2;
-          } else {
-            v += v1;
-          }
-        }
-      }
-      run.add(sn, sd, b, v, mirror ? 2u : 1u);
-    }
-  }
-  run.flush(sn, sd);
-  __syncthreads();
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    if (sd[b] != 0.0) {
-      atomicAdd(&numer[b], sn[b]);
-      atomicAdd(&denom[b], sd[b]);
-    }
-  }
+  BinRun<decltype(acc_norm2(acc, astride, 0))> run;
+  walk_spectrum(n, nh, rows, [&](int hx, int hy, int hz) {
+    const int kx = kint(hx, n), ky = kint(hy, n), kz = kint(hz, n);
+    const int b = tab[kx * kx + ky * ky + kz * kz];
+    if (b < 0) return;
+    const bool mirror = hx > 0 && hx < n / 2;
+    const auto v1 = acc_norm2(acc, astride, ((int64_t)hz * n + hy) * nh + hx);
+    auto v = v1;
+    if (mirror)
+      v = run_sum(v1, hy == n / 2 || hz == n / 2 ? acc_norm2(acc, astride, nhalf + gw_nyq_extra(hx, hy, hz, n)) : v1);
+    run.add(bins, b, v, mirror ? 2u : 1u);
+  });
+  run.flush(bins);
+  bins.finish(numer, denom);
 }
 
 // u_ij: one of the 12 real fields (f < 6: tau u_f; else u_c + tau u'_c,
@@ -717,102 +710,83 @@ __global__ void k_uij_prepare(const R *__restrict__ u, const R *__restrict__ ud,
   }
 }
 
-// TT power of a complex symmetric 3x3 (components 11,21,22,31,32,33)
-// |Lambda U|^2 of the TT projection; R = float for FP32 spectra (the shell
-// sums stay FP64)
+// The TT part of a symmetric tensor spectrum U (components 11, 21, 22, 31, 32,
+// 33) in the basis (m, l) normal to k: m = (-s, c, 0) with (c, s) the azimuth
+// of k, l = k x m / |k|.  |Lambda U|^2 = |U_mm - U_ll|^2 / 2 + 2 |U_ml|^2 with
+// U_mm - U_ll = sum a_c U_c and |k| U_ml = sum b_c U_c; a and b are rational
+// in the integers k:
+//   a_11 = s^2 - q^2 c^2,  a_21 = -2 s c (1 + q^2),  a_22 = c^2 - q^2 s^2,
+//   a_31 = 2 kz kx / k^2,  a_32 = 2 kz ky / k^2,     a_33 = -(a_11 + a_22),
+//   b_11 = kz s c,  b_21 = kz (s^2 - c^2),  b_22 = -b_11,  b_31 = -ky,  b_32 = kx
+// with c^2 = kx^2 / p^2, s^2 = ky^2 / p^2, s c = kx ky / p^2, q = kz / k.
+// a_33 that way, the trace drops out of the differences U_11 - U_33 and
+// U_22 - U_33 exactly.  20 multiply-adds a tensor where P U P - P tr(P U) / 2,
+// P = 1 - k k, and its squared norm took ~200 operations.
 template <typename R>
-__device__ R tt_power(const R Ur[6], const R Ui[6], const R kh[3]) {
-  const int idx[3][3] = {{0, 1, 3}, {1, 2, 4}, {3, 4, 5}};
-  R P[3][3], Tr[3][3], Ti[3][3], Rr[3][3], Ri[3][3];
-  for (int a = 0; a < 3; ++a)
-    for (int b = 0; b < 3; ++b) P[a][b] = (a == b ? R(1) : R(0)) - kh[a] * kh[b];
-  for (int a = 0; a < 3; ++a)
-    for (int b = 0; b < 3; ++b) {
-      R sr = 0, si = 0;
-      for (int c = 0; c < 3; ++c) {
-        sr += P[a][c] * Ur[idx[c][b]];
-        si += P[a][c] * Ui[idx[c][b]];
-      }
-      Tr[a][b] = sr;
-      Ti[a][b] = si;
-    }
-  for (int a = 0; a < 3; ++a)
-    for (int b = 0; b < 3; ++b) {
-      R sr = 0, si = 0;
-      for (int c = 0; c < 3; ++c) {
-        sr += Tr[a][c] * P[c][b];
-        si += Ti[a][c] * P[c][b];
-      }
-      Rr[a][b] = sr;
-      Ri[a][b] = si;
-    }
-  const R trr = Rr[0][0] + Rr[1][1] + Rr[2][2], tri = Ri[0][0] + Ri[1][1] + Ri[2][2];
-  R s = 0;
-  for (int a = 0; a < 3; ++a)
-    for (int b = 0; b < 3; ++b) {
-      const R vr = Rr[a][b] - R(0.5) * P[a][b] * trr, vi = Ri[a][b] - R(0.5) * P[a][b] * tri;
-      s += vr * vr + vi * vi;
-    }
-  return s;
+struct TTBasis {
+  R a11, a21, a22, a31, a32, b11, b21, b31, b32, ik2;
+};
+template <typename R>
+__device__ __forceinline__ TTBasis<R> tt_basis(int kx, int ky, int kz, int k2) {
+  const int p2 = kx * kx + ky * ky;
+  const R ik2 = R(1) / (R)k2, ip2 = p2 ? R(1) / (R)p2 : R(0);
+  const R cc = p2 ? (R)(kx * kx) * ip2 : R(1), ss = (R)(ky * ky) * ip2, sc = (R)(kx * ky) * ip2;
+  const R qq = (R)(kz * kz) * ik2;
+  TTBasis<R> t;
+  t.a11 = ss - qq * cc;
+  t.a21 = R(-2) * sc * (R(1) + qq);
+  t.a22 = cc - qq * ss;
+  t.a31 = (R)(2 * kz * kx) * ik2;
+  t.a32 = (R)(2 * kz * ky) * ik2;
+  t.b11 = (R)kz * sc;
+  t.b21 = (R)kz * (ss - cc);
+  t.b31 = (R)-ky;
+  t.b32 = (R)kx;
+  t.ik2 = ik2;
+  return t;
+}
+template <typename R, typename CV>
+__device__ __forceinline__ R tt_power(const TTBasis<R> &t, const CV *__restrict__ F, int64_t stride, int64_t h) {
+  const CV u11 = F[h], u21 = F[stride + h], u22 = F[2 * stride + h], u31 = F[3 * stride + h], u32 = F[4 * stride + h],
+           u33 = F[5 * stride + h];
+  auto plus = [&](R x11, R x21, R x22, R x31, R x32, R x33) {
+    return t.a11 * (x11 - x33) + t.a22 * (x22 - x33) + t.a21 * x21 + t.a31 * x31 + t.a32 * x32;
+  };
+  auto cross = [&](R x11, R x21, R x22, R x31, R x32) {
+    return t.b11 * (x11 - x22) + t.b21 * x21 + t.b31 * x31 + t.b32 * x32;
+  };
+  const R pr = plus(u11.x, u21.x, u22.x, u31.x, u32.x, u33.x), pi = plus(u11.y, u21.y, u22.y, u31.y, u32.y, u33.y);
+  const R xr = cross(u11.x, u21.x, u22.x, u31.x, u32.x), xi = cross(u11.y, u21.y, u22.y, u31.y, u32.y);
+  return R(0.5) * (pr * pr + pi * pi) + R(2) * t.ik2 * (xr * xr + xi * xi);
 }
 
-// F: the twelve half spectra, kx rows of sp entries
+// F: the twelve half spectra, kx rows of sp entries.  The TT power in the
+// precision of the spectrum (FP32 for FP32-mixed), the shell sums in FP64;
+// numer comes without its factor dv^2.  512^3 FP32 1.44 -> 0.83 ms (96 B an
+// entry: the copy peak allows 0.96 for what misses the L2); 256^3 FP64, bound
+// by the FP64 pipe, 4.41 -> 1.15.
 template <typename CV>
-__global__ void k_uij_bin(const CV *__restrict__ F, int sp, int n, double dwav, double dv,
-                          const int16_t *__restrict__ tab, int nb, double *__restrict__ numer,
-                          double *__restrict__ denom) {
-  __shared__ double sn[kMaxBins], sd[kMaxBins];
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) sn[b] = sd[b] = 0.0;
-  __syncthreads();
+__global__ void __launch_bounds__(256) k_uij_bin(const CV *__restrict__ F, int sp, int n, int rows, double dwav,
+                                                 const int16_t *__restrict__ tab, int nb, int copies,
+                                                 double *__restrict__ numer, double *__restrict__ denom) {
+  using R = decltype(F[0].x);
+  BlockBins bins(nb, copies);
   const int nh = n / 2 + 1;
-  const int64_t nhalf = (int64_t)n * n * nh, nspec = (int64_t)n * n * sp;
-  const double dv2 = dv * dv, dwav2 = dwav * dwav;
-  BinRun run;
-  for (int64_t h0 = run_start(); h0 < nhalf; h0 += run_stride()) {
-    for (int64_t h = h0; h < h0 + kRun && h < nhalf; ++h) {
-      const int ix = (int)(h % nh), iy = (int)((h / nh) % n), iz = (int)(h / ((int64_t)nh * n));
-      const int kx = kint(ix, n), ky = kint(iy, n), kz = kint(iz, n);
-      const int k2 = kx * kx + ky * ky + kz * kz;
-      const int b = tab[k2];
-      double v = 0.0;
-      unsigned wgt = 0;
-      if (b >= 0) {
-        // the TT projection in the precision of the spectrum (FP32 for FP32-mixed)
-        using R = decltype(F[0].x);
-        const R iq = R(1) / sqrt((R)k2);
-        const R kh[3] = {(R)kx * iq, (R)ky * iq, (R)kz * iq};
-        R Ur[6], Ui[6], Dr[6], Di[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-          const int64_t hs = (h / nh) * sp + ix;
-          const CV a = F[c * nspec + hs], d = F[(6 + c) * nspec + hs];
-          Ur[c] = a.x;
-          Ui[c] = a.y;
-          Dr[c] = d.x;
-          Di[c] = d.y;
-        }
-        wgt = (ix == 0 || 2 * ix == n) ? 1u : 2u;  // Hermitian partner of the half spectrum
-        if constexpr (sizeof(R) == 4) {
-          // FP32 spectra: the entry's energy in FP32, one conversion to the
-          // FP64 shell sums (a handful of FP64 operations fewer per entry)
-          const float e = tt_power<R>(Dr, Di, kh) + (float)k2 * (float)dwav2 * tt_power<R>(Ur, Ui, kh);
-          v = (double)e * (wgt * dv2);
-        } else {
-          const double e0 = (double)tt_power<R>(Dr, Di, kh) * dv2, e1 = (double)tt_power<R>(Ur, Ui, kh) * dv2;
-          v = wgt * (e0 + (double)k2 * dwav2 * e1);
-        }
-      }
-      run.add(sn, sd, b, v, wgt);
-    }
-  }
-  run.flush(sn, sd);
-  __syncthreads();
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    if (sd[b] != 0.0) {
-      atomicAdd(&numer[b], sn[b]);
-      atomicAdd(&denom[b], sd[b]);
-    }
-  }
+  const int64_t nspec = (int64_t)n * n * sp;
+  const R dwav2 = (R)(dwav * dwav);
+  BinRun<double> run;
+  walk_spectrum(n, nh, rows, [&](int ix, int iy, int iz) {
+    const int kx = kint(ix, n), ky = kint(iy, n), kz = kint(iz, n), k2 = kx * kx + ky * ky + kz * kz;
+    const int b = tab[k2];
+    if (b < 0) return;
+    const int64_t h = ((int64_t)iz * n + iy) * sp + ix;
+    const TTBasis<R> t = tt_basis<R>(kx, ky, kz, k2);
+    const unsigned wgt = (ix == 0 || 2 * ix == n) ? 1u : 2u;  // Hermitian partner of the half spectrum
+    const R e = tt_power(t, F + 6 * nspec, nspec, h) + (R)k2 * dwav2 * tt_power(t, F, nspec, h);
+    run.add(bins, b, (double)((R)wgt * e), wgt);
+  });
+  run.flush(bins);
+  bins.finish(numer, denom);
 }
 
 // grav_waves.f90:265-267 on an n^3 grid of spacing dspa (the GW grid of
@@ -1029,18 +1003,23 @@ int axg_gw_spec(axg_ctx *ctx, double tau, int log_bins, double *wave, double *po
   AXG_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, sizeof(double) * 2 * nb, ctx->stream));
   const int16_t *tab = nullptr;
   AXG_TRY(axg_bin_table(ctx, AXG_BIN_GW, n, dwav, dq, nb, log_bins, edges.data(), &tab));
+  const int brows = walk_rows(n, n / 2 + 1), bgrid = walk_grid(n, n / 2 + 1, brows);
+  const int copies = bin_copies(nb);
+  const size_t bsm = bin_smem(nb);
+  double scale = 1.0;  // of numer
   if (ctx->p.gw_mode == AXG_GW_GREEN) {
     if (ctx->acc_ff)
-      AXG_LAUNCH(ctx, "gw_bin_green", k_gw_bin_green<float4>, 152 * 4, 256, 0, (const float4 *)ctx->acc, n,
-                 ctx->acc_stride, tab, nb, d_num, d_den);
+      AXG_LAUNCH(ctx, "gw_bin_green", k_gw_bin_green<float4>, bgrid, 256, bsm, (const float4 *)ctx->acc, n,
+                 ctx->acc_stride, brows, tab, nb, copies, d_num, d_den);
     else
-      AXG_LAUNCH(ctx, "gw_bin_green", k_gw_bin_green<double2>, 152 * 4, 256, 0, ctx->acc, n, ctx->acc_stride, tab, nb,
-                 d_num, d_den);
+      AXG_LAUNCH(ctx, "gw_bin_green", k_gw_bin_green<double2>, bgrid, 256, bsm, ctx->acc, n, ctx->acc_stride,
+                 brows, tab, nb, copies, d_num, d_den);
   } else if (ctx->p.gw_mode == AXG_GW_UIJ) {
     AXG_TRY(ensure_uij_fft(ctx));
     const bool fp32 = ctx->p.precision == AXG_PREC_FP32_MIXED;
     const int64_t nhalf = (int64_t)n * n * (n / 2 + 1);
     const double dv = ctx->p.dspa * ctx->p.dspa * ctx->p.dspa;
+    scale = dv * dv;
     if (fp32) {
       float *w = (float *)ctx->ubuf;
       float2 *F = ctx->uij_own_fft ? (float2 *)ctx->ubuf : (float2 *)(w + ctx->n3);
@@ -1055,8 +1034,8 @@ int axg_gw_spec(axg_ctx *ctx, double tau, int log_bins, double *wave, double *po
           AXG_CUFFT_TRY(ctx, cufftExecR2C(ctx->plan_u, w, (cufftComplex *)F + f * nhalf));
         }
       }
-      AXG_LAUNCH(ctx, "uij_bin_fp32", k_uij_bin<float2>, 152 * 4, 256, 0, F, ctx->u_pitch, n, dwav, dv, tab, nb,
-                 d_num, d_den);
+      AXG_LAUNCH(ctx, "uij_bin_fp32", k_uij_bin<float2>, bgrid, 256, bsm, F, ctx->u_pitch, n, brows, dwav, tab, nb,
+                 copies, d_num, d_den);
     } else {
       double *w = (double *)ctx->ubuf;
       double2 *F = ctx->uij_own_fft ? (double2 *)ctx->ubuf : (double2 *)(w + ctx->n3);
@@ -1070,8 +1049,8 @@ int axg_gw_spec(axg_ctx *ctx, double tau, int log_bins, double *wave, double *po
           AXG_CUFFT_TRY(ctx, cufftExecD2Z(ctx->plan_u, w, (cufftDoubleComplex *)F + f * nhalf));
         }
       }
-      AXG_LAUNCH(ctx, "uij_bin_fp64", k_uij_bin<double2>, 152 * 4, 256, 0, F, ctx->u_pitch, n, dwav, dv, tab, nb,
-                 d_num, d_den);
+      AXG_LAUNCH(ctx, "uij_bin_fp64", k_uij_bin<double2>, bgrid, 256, bsm, F, ctx->u_pitch, n, brows, dwav, tab, nb,
+                 copies, d_num, d_den);
     }
   } else {
     return axg_set_error(ctx, AXG_ERR_STATE, "gw_mode is NONE");
@@ -1084,7 +1063,7 @@ int axg_gw_spec(axg_ctx *ctx, double tau, int log_bins, double *wave, double *po
   const double fact = gw_fact(ctx->p, n, dspa);
   for (int k = 0; k < nb; ++k) {
     const double qc = log_bins ? std::sqrt(edges[k] * edges[k + 1]) : (edges[k + 1] + edges[k]) / 2;
-    numer[k] = h[k];
+    numer[k] = h[k] * scale;
     denom[k] = h[nb + k];
     power[k] = denom[k] > 0 ? numer[k] / denom[k] * (qc * qc * qc) * fact : 0.0;
     if (wave) {

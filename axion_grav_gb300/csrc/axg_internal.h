@@ -125,7 +125,9 @@ struct axg_ctx {
   // spectra
   double *spec_mat = nullptr;  // mat_spec [num_cov][501]
   double *spec_largeq0 = nullptr, *spec_dq = nullptr;  // per ij
-  std::vector<double> h_mat_spec, h_largeq, h_dq, h_wav;
+  double *spec_modes = nullptr;      // per ij: sum over the lattice's modes of the pair's table
+  long long *spec_range = nullptr;   // per ij: first and last |k|^2 inside the pair's table
+  std::vector<double> h_wav;         // bin edges
   std::vector<double> last_power;
   std::vector<double> last_mat_div;  // deconvolution matrix after the division by mode counts
   std::vector<double> last_cov;      // MC covariance of the last spectrum (num_cov)
@@ -274,7 +276,11 @@ bool axg_ff_use(int n);
 // keep_ff: the output stays float-float, (re hi, re lo, im hi, im lo) per
 // complex value in the same 16 bytes, for a consumer that reads it so
 int axg_ff_d2z(axg_ctx *ctx, const double *in, double2 *out, int n, int batch, bool keep_ff = false);
-int axg_ff_z2z(axg_ctx *ctx, double2 *data, int n, int inverse);  // in place, one n^3 volume
+int axg_ff_z2z(axg_ctx *ctx, double2 *data, int n, int inverse, bool keep_ff = false);  // in place, one n^3 volume
+// the same of a field that the defect flags mask (zero where bit 4 is set)
+// into out, kept float-float; and the D2Z of the window, dv where it is clear
+int axg_ff_z2z_masked(axg_ctx *ctx, const void *field, bool fp32, const int8_t *flags, double2 *out, int n, int inverse);
+int axg_ff_d2z_window(axg_ctx *ctx, const int8_t *flags, double dv, double2 *out, int n);
 // The Green accumulators hold the stored half spectrum only: component a of
 // the entry h = (hz n + hy) (n/2 + 1) + hx is acc[a acc_stride + h], and the
 // site of -k is its conjugate (real sources, and e+(-k) = conj e+(k)).  On

@@ -1,7 +1,7 @@
 // axg_spectrum.cu -- masked field spectrum with window deconvolution
 // (spectrum.f90:23-171, 242-567, 736-954) on the GPU.
 //
-//   init (host, once): mode-coupling table mat_spec(0:500, num_cov) by the
+//   init (once): mode-coupling table mat_spec(0:500, num_cov) by the
 //        reference's 200-point quadrature (spectrum.f90:74-98, 117-171);
 //   conv spectrum: k_spec_degrade box-averages phidot over deg^3 and zeroes
 //        coarse cells that hold a masked cell (flag bit 4 of the last
@@ -11,8 +11,8 @@
 //        each of the num_cov = nb(nb+1)/2 bin pairs (O(num_cov N^3),
 //        spectrum.f90:385-428).  Here |W|^2 and the mode count are first
 //        histogrammed by integer |k|^2 (k_spec_w2_hist), an exact regrouping,
-//        and k_spec_mat sums the histogram against the interpolation table
-//        (O(num_cov * 3(N/2)^2));
+//        and k_spec_mat sums prefix sums of the histogram against the cells
+//        of the interpolation table (O(num_cov * 500));
 //   packed Cholesky inverse (dpptrf/dpptri) and dspmv on the host (nb x nb).
 #include <cmath>
 #include <vector>
@@ -61,37 +61,26 @@ __global__ void k_spec_degrade(const V *__restrict__ phid, const int8_t *__restr
   }
 }
 
-// |F dv_spa|^2 dv_wav per k-site into the bins of |k|^2: the two scalings
-// are one factor, scale = dv_spa^2 dv_wav (three FP64 operations per site
-// instead of six)
-__global__ void k_spec_bin(const double2 *__restrict__ F, int m, const int16_t *__restrict__ tab, double scale,
-                           int nb, double *__restrict__ conv, double *__restrict__ count) {
-  extern __shared__ double sh[];
-  double *sc = sh, *sn = sh + nb;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) sc[b] = sn[b] = 0.0;
-  __syncthreads();
-  const int64_t m3 = (int64_t)m * m * m;
-  BinRun run;
-  for (int64_t s0 = run_start(); s0 < m3; s0 += run_stride()) {
-    for (int64_t s = s0; s < s0 + kRun && s < m3; ++s) {
-      const int kx = kint(s % m, m), ky = kint((s / m) % m, m), kz = kint(s / ((int64_t)m * m), m);
-      const int b = tab[kx * kx + ky * ky + kz * kz];
-      double v = 0.0;
-      if (b >= 0) {
-        const double2 f = F[s];
-        v = (f.x * f.x + f.y * f.y) * scale;
-      }
-      run.add(sc, sn, b, v, 1u);
-    }
-  }
-  run.flush(sc, sn);
-  __syncthreads();
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    if (sn[b] != 0.0) {
-      atomicAdd(&conv[b], sc[b]);
-      atomicAdd(&count[b], sn[b]);
-    }
-  }
+// |F|^2 per k-site into the bins of |k|^2, F in FP64 (cuFFT, the Monte-Carlo
+// fields) or float-float; the sums are scaled on the host
+__device__ __forceinline__ double norm2(double2 w) { return w.x * w.x + w.y * w.y; }
+__device__ __forceinline__ F2 norm2(float4 w) {
+  const F2 r = {w.x, w.y}, i = {w.z, w.w};
+  return f2_dot2(r, r, i, i, 1.f);
+}
+template <typename V>
+__global__ void __launch_bounds__(256) k_spec_bin(const V *__restrict__ F, int m, int rows,
+                                                  const int16_t *__restrict__ tab, int nb, int copies,
+                                                  double *__restrict__ conv, double *__restrict__ count) {
+  BlockBins bins(nb, copies);
+  BinRun<decltype(norm2(F[0]))> run;
+  walk_spectrum(m, m, rows, [&](int ix, int iy, int iz) {
+    const int kx = kint(ix, m), ky = kint(iy, m), kz = kint(iz, m);
+    const int b = tab[kx * kx + ky * ky + kz * kz];
+    if (b >= 0) run.add(bins, b, norm2(F[((int64_t)iz * m + iy) * m + ix]), 1u);
+  });
+  run.flush(bins);
+  bins.finish(conv, count);
 }
 
 // the real window of compute_matrix_deconv: dx^3 on unmasked coarse cells
@@ -115,99 +104,209 @@ __global__ void k_spec_window(const int8_t *__restrict__ flags, int n, int deg, 
   }
 }
 
-// |W|^2 and mode counts per integer |k|^2 from the half spectrum of the real
-// window (|W(-k)| = |W(k)|: interior kx planes count twice)
-__global__ void k_spec_w2_hist(const double2 *__restrict__ W, int m, double *__restrict__ h,
-                               double *__restrict__ cnt) {
+// |W|^2 per integer |k|^2 from the half spectrum of the real window
+// (|W(-k)| = |W(k)|: interior kx planes count twice)
+template <typename V>
+__global__ void k_spec_w2_hist(const V *__restrict__ W, int m, double *__restrict__ h) {
+  const int mh = m / 2 + 1;
+  walk_spectrum(m, mh, 1, [&](int ix, int iy, int iz) {
+    const int kx = kint(ix, m), ky = kint(iy, m), kz = kint(iz, m);
+    auto v = norm2(W[((int64_t)iz * m + iy) * mh + ix]);
+    if (ix != 0 && 2 * ix != m) v = run_sum(v, v);
+    atomicAdd(&h[kx * kx + ky * ky + kz * kz], run_value(v));
+  });
+}
+
+// The window matrix of bin pair ij (spectrum.f90:385-428) is the sum over all
+// k of |W(k)|^2 u_ij(|k|), divided by the sum of u_ij alone, with u_ij linear
+// between the 501 nodes of its table.  Regrouped by |k|^2 and then by table
+// cell: with the prefix sums of |W|^2 and of |W|^2 |k|, a cell [q_a, q_a + dq)
+// adds
+//   tab_a (S0 - D) + tab_(a+1) D,  S0 = sum h,  D = (sum h q - S0 q_a) / dq
+// from two prefix differences.  The sums are double-double (T. J. Dekker,
+// Numer. Math. 18 (1971) 224): S0 q_a cancels sum h q to a few thousandths.
+// 1275 pairs x 500 cells instead of 1275 pairs x every |k|^2, ~14 FP64
+// operations each on a pipe at 1/64 of the FP32 rate: 870 -> 154 us at 256^3
+// with the scans, 3.4 ms -> 270 us at 512^3.  The sums of u_ij alone (h = the
+// number of modes) belong to the lattice and are formed once.
+struct DD {
+  double h, l;
+};
+__device__ __forceinline__ DD dd_add(DD a, DD b) {
+  const double s = AXD_ADD(a.h, b.h), v = AXD_SUB(s, a.h);
+  double e = AXD_ADD(AXD_SUB(a.h, AXD_SUB(s, v)), AXD_SUB(b.h, v));
+  e = AXD_ADD(e, AXD_ADD(a.l, b.l));
+  const double h = AXD_ADD(s, e);
+  return {h, AXD_SUB(e, AXD_SUB(h, s))};
+}
+__device__ __forceinline__ DD dd_sub(DD a, DD b) { return dd_add(a, DD{-b.h, -b.l}); }
+__device__ __forceinline__ DD dd_prod(double a, double b) {
+  const double p = AXD_MUL(a, b);
+  return {p, AXD_FMA(a, b, -p)};
+}
+struct Sums {
+  DD h, hq;
+};
+__device__ __forceinline__ Sums sums_add(Sums a, Sums b) { return {dd_add(a.h, b.h), dd_add(a.hq, b.hq)}; }
+__device__ __forceinline__ Sums sums_shfl(Sums a, int lane) {
+  auto f = [lane](double x) { return __shfl_sync(0xffffffffu, x, lane); };
+  return {{f(a.h.h), f(a.h.l)}, {f(a.hq.h), f(a.hq.l)}};
+}
+// inclusive scan over the lanes of a warp
+__device__ __forceinline__ Sums warp_scan(Sums x) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const Sums y = sums_shfl(x, lane >= o ? lane - o : 0);
+    if (lane >= o) x = sums_add(y, x);
+  }
+  return x;
+}
+constexpr int kScan = 128;  // |k|^2 values per CTA of the scan, a chunk
+
+// q = |k| = sqrt(iq2) dwav; pre[iq2 + 1]: the sums of iq2's chunk up to and
+// with iq2; tot[chunk]: the chunk's
+__global__ void __launch_bounds__(kScan) k_spec_scan(const double *__restrict__ h, int64_t count, double dwav,
+                                                     Sums *__restrict__ pre, Sums *__restrict__ tot) {
+  const int64_t i = (int64_t)blockIdx.x * kScan + threadIdx.x;
+  Sums x{};
+  if (i < count) {
+    x.h = {h[i], 0.0};
+    x.hq = dd_prod(h[i], AXD_MUL(sqrt((double)i), dwav));
+  }
+  x = warp_scan(x);
+  __shared__ Sums warp[kScan / 32];
+  const int w = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 31) warp[w] = x;
+  __syncthreads();
+  Sums before{};
+  for (int k = 0; k < w; ++k) before = sums_add(before, warp[k]);
+  if (w > 0) x = sums_add(before, x);
+  if (i < count) pre[i + 1] = x;
+  if (threadIdx.x == kScan - 1) tot[blockIdx.x] = x;
+}
+
+// the chunks' totals into the sums before each chunk: one warp, each lane a
+// run of chunks (more warps would only queue for one SM's FP64 pipe)
+__global__ void k_spec_scan_chunks(Sums *__restrict__ tot, int chunks) {
+  const int lane = threadIdx.x, per = (chunks + 31) / 32, c0 = min(lane * per, chunks), c1 = min(c0 + per, chunks);
+  Sums run{};
+  for (int c = c0; c < c1; ++c) run = sums_add(run, tot[c]);
+  Sums before = sums_shfl(warp_scan(run), lane > 0 ? lane - 1 : 0);
+  if (lane == 0) before = Sums{};
+  for (int c = c0; c < c1; ++c) {
+    const Sums own = tot[c];
+    tot[c] = before;
+    before = sums_add(before, own);
+  }
+}
+
+__global__ void __launch_bounds__(kScan) k_spec_scan_add(Sums *__restrict__ pre, const Sums *__restrict__ before,
+                                                         int64_t count) {
+  const int64_t i = (int64_t)blockIdx.x * kScan + threadIdx.x;
+  if (i < count) pre[i + 1] = sums_add(before[blockIdx.x], pre[i + 1]);
+  if (i == 0) pre[0] = Sums{};
+}
+
+// pre[k]: the sums over |k|^2 < k.  One CTA per bin pair, thread a the first
+// |k|^2 of table cell a (a = 500: the end) and the sums up to it.
+constexpr int kMatThreads = 512;
+static_assert(kMatThreads > kNumLargeq, "a thread per node of the table");
+__global__ void __launch_bounds__(kMatThreads) k_spec_mat(const Sums *__restrict__ pre,
+                                                          const double *__restrict__ mat_spec,
+                                                          const double *__restrict__ largeq0,
+                                                          const double *__restrict__ dq_spec,
+                                                          const long long *__restrict__ range, double dwav,
+                                                          double *__restrict__ out) {
+  const int ij = blockIdx.x, a = threadIdx.x, lane = a & 31;
+  const long long lo = range[2 * ij], hi = range[2 * ij + 1];
+  const double *tab = mat_spec + (int64_t)ij * (kNumLargeq + 1);
+  const double lq0 = largeq0[ij], dq = dq_spec[ij], idq = 1.0 / dq, iw = 1.0 / dwav;
+  auto first = [&](int c) -> long long {  // within [lo, hi + 1]
+    if (c == 0 || hi < lo) return lo;
+    if (c >= kNumLargeq) return hi + 1;
+    const double e = (lq0 + dq * c) * iw;
+    const long long k = (long long)ceil(e * e);
+    return k < lo ? lo : (k > hi + 1 ? hi + 1 : k);
+  };
+  const long long k0 = first(a);
+  const Sums p0 = pre[k0];
+  long long k1 = __shfl_down_sync(0xffffffffu, k0, 1);
+  Sums p1 = sums_shfl(p0, lane < 31 ? lane + 1 : 31);
+  if (lane == 31) {
+    k1 = first(a + 1);
+    p1 = pre[k1];
+  }
+  double v = 0.0;
+  if (a < kNumLargeq && k1 > k0) {
+    const double qa = lq0 + dq * a;
+    const DD s0 = dd_sub(p1.h, p0.h);
+    DD sq = dd_prod(s0.h, qa);
+    sq.l = AXD_FMA(s0.l, qa, sq.l);
+    const double D = dd_sub(dd_sub(p1.hq, p0.hq), sq).h * idq;
+    v = tab[a] * (s0.h - D) + tab[a + 1] * D;
+  }
+  __shared__ double sum[kMatThreads / 32];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane == 0) sum[a >> 5] = v;
+  __syncthreads();
+  if (a == 0) {
+    for (int w = 1; w < kMatThreads / 32; ++w) v += sum[w];
+    out[ij] = v;
+  }
+}
+
+// modes per integer |k|^2
+__global__ void k_spec_modes(int m, double *__restrict__ cnt) {
   const int mh = m / 2 + 1;
   const int64_t nhalf = (int64_t)m * m * mh;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < nhalf; s += stride) {
     const int ix = (int)(s % mh), iy = (int)((s / mh) % m), iz = (int)(s / ((int64_t)mh * m));
     const int kx = kint(ix, m), ky = kint(iy, m), kz = kint(iz, m);
-    const int iq2 = kx * kx + ky * ky + kz * kz;
-    const double wgt = (ix == 0 || 2 * ix == m) ? 1.0 : 2.0;
-    const double2 w = W[s];
-    atomicAdd(&h[iq2], wgt * (w.x * w.x + w.y * w.y));
-    atomicAdd(&cnt[iq2], wgt);
+    atomicAdd(&cnt[kx * kx + ky * ky + kz * kz], (ix == 0 || 2 * ix == m) ? 1.0 : 2.0);
   }
 }
 
-// one block per bin pair ij (spectrum.f90:385-428 regrouped by |k|^2)
-// |k| = sqrt(iq2) dwav for every integer |k|^2 up to iq2max, formed once and
-// shared by all the (i, j) pairs of k_spec_mat instead of an FP64 square
-// root per pair and |k|^2 (FP64 runs at 1/64 of the FP32 rate on GB300)
-__global__ void k_spec_qtab(int64_t iq2max, double dwav, double *__restrict__ q) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= iq2max; i += (int64_t)gridDim.x * blockDim.x)
-    q[i] = sqrt((double)i) * dwav;
-}
-
-__global__ void k_spec_mat(const double *__restrict__ h, const double *__restrict__ cnt,
-                           const double *__restrict__ mat_spec, const double *__restrict__ largeq0,
-                           const double *__restrict__ dq_spec, const long long *__restrict__ range,
-                           const double *__restrict__ qtab, double *__restrict__ mat0, double *__restrict__ tat0) {
-  const int ij = blockIdx.x;
-  const long long lo = range[2 * ij], hi = range[2 * ij + 1];
-  const double *tab = mat_spec + (int64_t)ij * (kNumLargeq + 1);
-  const double lq0 = largeq0[ij], idq = 1.0 / dq_spec[ij];  // one division per pair
-  double a = 0.0, b = 0.0;
-  for (long long iq2 = lo + threadIdx.x; iq2 <= hi; iq2 += blockDim.x) {
-    const double c = cnt[iq2];
-    if (c == 0.0) continue;
-    const double q = qtab[iq2];
-    double d = (q - lq0) * idq;
-    const double fl = floor(d);
-    double u = 0.0;
-    if (fl < kNumLargeq && fl >= 0) {
-      const int iq = (int)fl;
-      d = d - iq;
-      u = (1 - d) * tab[iq] + d * tab[iq + 1];
-    }
-    a += h[iq2] * u;
-    b += c * u;
-  }
-  __shared__ double sa[256], sb[256];
-  sa[threadIdx.x] = a;
-  sb[threadIdx.x] = b;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) {
-      sa[threadIdx.x] += sa[threadIdx.x + o];
-      sb[threadIdx.x] += sb[threadIdx.x + o];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    mat0[ij] = sa[0];
-    tat0[ij] = sb[0];
-  }
-}
-
-// spectrum.f90:117-171
-double integrate_p_check(int num, double li, double si, double lj, double sj, double q) {
-  double maxp = lj < q + li ? lj : q + li;
-  double a = q - li, b = si - q;
+// spectrum.f90:117-171, every operation rounded once in the reference's order
+__device__ double integrate_p_check(int num, double li, double si, double lj, double sj, double q) {
+  const double qli = AXD_ADD(q, li);
+  const double maxp = lj < qli ? lj : qli;
+  const double a = AXD_SUB(q, li), b = AXD_SUB(si, q);
   double minp = a > b ? a : b;
   minp = minp > sj ? minp : sj;
-  double dp = (maxp - minp) / num;
+  const double dp = AXD_DIV(AXD_SUB(maxp, minp), (double)num);
   double x = 0.0;
   if (dp > 0) {
+    const double qq = AXD_MUL(q, q), l2 = AXD_MUL(li, li), s2 = AXD_MUL(si, si);
     for (int ip = 1; ip <= num; ++ip) {
-      double p = dp * (ip - 0.5) + minp;
-      double maxmu, minmu;
-      if (q == 0.0) {
-        maxmu = 1.0;
-        minmu = -1.0;
-      } else {
-        maxmu = (li * li - p * p - q * q) / 2 / p / q;
-        minmu = (si * si - p * p - q * q) / 2 / p / q;
+      const double p = AXD_ADD(AXD_MUL(dp, ip - 0.5), minp);
+      double maxmu = 1.0, minmu = -1.0;
+      if (q != 0.0) {
+        const double pp = AXD_MUL(p, p);
+        maxmu = AXD_DIV(AXD_DIV(AXD_MUL(AXD_SUB(AXD_SUB(l2, pp), qq), 0.5), p), q);
+        minmu = AXD_DIV(AXD_DIV(AXD_MUL(AXD_SUB(AXD_SUB(s2, pp), qq), 0.5), p), q);
         maxmu = maxmu < 1.0 ? maxmu : 1.0;
         minmu = minmu > -1.0 ? minmu : -1.0;
       }
-      x = x + p * p * dp * (maxmu - minmu);
+      x = AXD_ADD(x, AXD_MUL(AXD_MUL(AXD_MUL(p, p), dp), AXD_SUB(maxmu, minmu)));
     }
   }
-  return x * kRefTwoPi;
+  return AXD_MUL(x, kRefTwoPi);
+}
+
+// mat_spec(0:500, ij) (spectrum.f90:74-98): the 200-point quadrature of every
+// table node, a node per thread.  On one host thread it was most of a
+// context's first spectrum: 530 ms for 50 bins.
+__global__ void k_spec_table(int num_cov, const double *__restrict__ wav, const double *__restrict__ largeq0,
+                             const double *__restrict__ dq_spec, double *__restrict__ mat_spec) {
+  const int ij = blockIdx.x + 1;
+  int i = (int)lround(sqrt(2.0 * ij));
+  const int j = ij - i * (i - 1) / 2;
+  for (int iq = threadIdx.x; iq <= kNumLargeq; iq += blockDim.x)
+    mat_spec[(int64_t)(ij - 1) * (kNumLargeq + 1) + iq] =
+        integrate_p_check(kNumInt, wav[i], wav[i - 1], wav[j], wav[j - 1],
+                          AXD_ADD(largeq0[ij - 1], AXD_MUL(dq_spec[ij - 1], (double)iq)));
 }
 
 // reference LAPACK dpptrf + dpptri ('U'), packed upper
@@ -336,7 +435,25 @@ int grid_for(int64_t count) {
 
 }  // namespace
 
-// init_spectrum (spectrum.f90:23-103): tables on the host, copied to the device
+namespace {
+// scratch of window_sums for |k|^2 <= iq2max, in Sums
+size_t window_sums_scratch(int64_t iq2max) { return (size_t)(iq2max + 2) + (size_t)((iq2max + kScan) / kScan); }
+
+// out[ij] = sum over |k|^2 of h u_ij(|k|) for every bin pair
+int window_sums(axg_ctx *ctx, const double *h, int64_t iq2max, double dwav, Sums *scratch, double *out) {
+  const int nb = ctx->p.num_bin, num_cov = nb * (nb + 1) / 2;
+  const int chunks = (int)((iq2max + kScan) / kScan);
+  Sums *pre = scratch, *tot = scratch + iq2max + 2;
+  AXG_LAUNCH(ctx, "spec_scan", k_spec_scan, chunks, kScan, 0, h, iq2max + 1, dwav, pre, tot);
+  AXG_LAUNCH(ctx, "spec_scan_chunks", k_spec_scan_chunks, 1, 32, 0, tot, chunks);
+  AXG_LAUNCH(ctx, "spec_scan_add", k_spec_scan_add, chunks, kScan, 0, pre, tot, iq2max + 1);
+  AXG_LAUNCH(ctx, "spec_mat", k_spec_mat, num_cov, kMatThreads, 0, pre, ctx->spec_mat, ctx->spec_largeq0, ctx->spec_dq,
+             ctx->spec_range, dwav, out);
+  return AXG_OK;
+}
+}  // namespace
+
+// init_spectrum (spectrum.f90:23-103): bin pairs on the host, tables on the device
 int axg_spec_init(axg_ctx *ctx) {
   if (ctx->spec_mat) return AXG_OK;
   const int nb = ctx->p.num_bin;
@@ -349,9 +466,10 @@ int axg_spec_init(axg_ctx *ctx) {
   const double qmax = kRefPi / dspa_spec;
   const double dq = qmax / nb;
   for (int iq = 1; iq <= nb; ++iq) wav[iq] = wav[iq - 1] + dq;
-  ctx->h_mat_spec.assign((size_t)num_cov * 501, 0.0);
-  ctx->h_largeq.assign((size_t)num_cov * 501, 0.0);
-  ctx->h_dq.assign(num_cov, 0.0);
+  const double dwav = kRefTwoPi / dspa_spec / m;
+  const int64_t iq2max = 3LL * (m / 2) * (m / 2);
+  std::vector<double> l0(num_cov), hdq(num_cov);
+  std::vector<long long> hr(2 * (size_t)num_cov);  // the |k|^2 inside each pair's table
   for (int ij = 1; ij <= num_cov; ++ij) {
     int i = (int)std::lround(std::sqrt(2.0 * ij));
     int j = ij - i * (i - 1) / 2;
@@ -361,21 +479,38 @@ int axg_spec_init(axg_ctx *ctx) {
     if (minq < 0) minq = 0.0;
     double d = maxq - minq;
     d = d / kNumLargeq;
-    ctx->h_dq[ij - 1] = d;
-    for (int iq = 0; iq <= kNumLargeq; ++iq) {
-      double q = minq + d * iq;
-      ctx->h_largeq[(size_t)(ij - 1) * 501 + iq] = q;
-      ctx->h_mat_spec[(size_t)(ij - 1) * 501 + iq] = integrate_p_check(kNumInt, li, si, lj, sj, q);
-    }
+    hdq[ij - 1] = d;
+    l0[ij - 1] = minq;
+    double e = (minq + d * kNumLargeq) / dwav;
+    long long imax2 = (long long)std::ceil(e * e) - 1;
+    e = minq / dwav;
+    long long imin2 = (long long)std::ceil(e * e);
+    hr[2 * (ij - 1)] = std::max(imin2, 0LL);
+    hr[2 * (ij - 1) + 1] = std::min(imax2, (long long)iq2max);
   }
-  std::vector<double> l0(num_cov);
-  for (int ij = 0; ij < num_cov; ++ij) l0[ij] = ctx->h_largeq[(size_t)ij * 501];
-  AXG_TRY(axg_alloc(ctx, (void **)&ctx->spec_mat, ctx->h_mat_spec.size() * 8, "mat_spec"));
+  AXG_TRY(axg_alloc(ctx, (void **)&ctx->spec_mat, (size_t)num_cov * (kNumLargeq + 1) * 8, "mat_spec"));
   AXG_TRY(axg_alloc(ctx, (void **)&ctx->spec_largeq0, (size_t)num_cov * 8, "largeq"));
   AXG_TRY(axg_alloc(ctx, (void **)&ctx->spec_dq, (size_t)num_cov * 8, "dq_spec"));
-  AXG_CUDA_TRY(ctx, cudaMemcpy(ctx->spec_mat, ctx->h_mat_spec.data(), ctx->h_mat_spec.size() * 8, cudaMemcpyHostToDevice));
-  AXG_CUDA_TRY(ctx, cudaMemcpy(ctx->spec_largeq0, l0.data(), (size_t)num_cov * 8, cudaMemcpyHostToDevice));
-  AXG_CUDA_TRY(ctx, cudaMemcpy(ctx->spec_dq, ctx->h_dq.data(), (size_t)num_cov * 8, cudaMemcpyHostToDevice));
+  AXG_TRY(axg_alloc(ctx, (void **)&ctx->spec_range, (size_t)num_cov * 16, "pair ranges"));
+  AXG_TRY(axg_alloc(ctx, (void **)&ctx->spec_modes, (size_t)num_cov * 8, "pair mode sums"));
+  double *d_wav = nullptr;  // bin edges, then the modes per |k|^2 and the scratch of their sums
+  auto cleanup = axg_on_exit([&] {
+    cudaStreamSynchronize(ctx->stream);
+    axg_free(ctx, (void **)&d_wav);
+  });
+  const size_t edges = (wav.size() + 1) & ~(size_t)1, modes = ((size_t)iq2max + 2) & ~(size_t)1;
+  AXG_TRY(axg_alloc(ctx, (void **)&d_wav, (edges + modes) * 8 + window_sums_scratch(iq2max) * sizeof(Sums),
+                    "spectrum tables"));
+  AXG_CUDA_TRY(ctx, cudaMemcpyAsync(d_wav, wav.data(), wav.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
+  AXG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->spec_largeq0, l0.data(), (size_t)num_cov * 8, cudaMemcpyHostToDevice, ctx->stream));
+  AXG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->spec_dq, hdq.data(), (size_t)num_cov * 8, cudaMemcpyHostToDevice, ctx->stream));
+  AXG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->spec_range, hr.data(), hr.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
+  AXG_LAUNCH(ctx, "spec_table", k_spec_table, num_cov, 128, 0, num_cov, d_wav, ctx->spec_largeq0, ctx->spec_dq,
+             ctx->spec_mat);
+  double *cnt = d_wav + edges;
+  AXG_CUDA_TRY(ctx, cudaMemsetAsync(cnt, 0, modes * 8, ctx->stream));
+  AXG_LAUNCH(ctx, "spec_modes", k_spec_modes, grid_for((int64_t)m * m * (m / 2 + 1)), 256, 0, m, cnt);
+  AXG_TRY(window_sums(ctx, cnt, iq2max, dwav, (Sums *)(cnt + modes), ctx->spec_modes));
   ctx->ns_spec = m;
   // m^3 complex; the window pass uses it as m^3 reals followed by the D2Z
   // half spectrum m^2 (m/2 + 1), which needs 16 m^2 bytes more
@@ -408,60 +543,61 @@ int axg_spec_estimation(axg_ctx *ctx, double tau, double *wave, double *power, d
   const double dv_wav = std::pow(dwav / kRefTwoPi, 3);
   const bool fp32 = ctx->p.precision == AXG_PREC_FP32_MIXED;
   const int64_t iq2max = 3LL * (m / 2) * (m / 2);
-  // scratch: histogram + counts + mat0/tat0 + bin sums + pair ranges
+  // scratch: histogram, pair sums, bin sums, and what window_sums needs
   double *scratch = nullptr;
-  long long *range = nullptr;
-  const size_t nscr = (size_t)(3 * (iq2max + 1) + 2 * num_cov + 2 * nb);
-  AXG_TRY(axg_alloc(ctx, (void **)&scratch, nscr * 8, "spectrum scratch"));
+  const size_t nscr = (((size_t)(iq2max + 1 + num_cov + 2 * nb)) + 1) & ~(size_t)1;
+  AXG_TRY(axg_alloc(ctx, (void **)&scratch, nscr * 8 + window_sums_scratch(iq2max) * sizeof(Sums), "spectrum scratch"));
   int rc = AXG_OK;
   do {
-    if ((rc = axg_alloc(ctx, (void **)&range, (size_t)num_cov * 16, "pair ranges"))) break;
-    double *h = scratch, *cnt = scratch + iq2max + 1, *mat0 = cnt + iq2max + 1, *tat0 = mat0 + num_cov,
-           *d_conv = tat0 + num_cov, *d_cnt = d_conv + nb, *qtab = d_cnt + nb;
+    double *h = scratch, *mat0 = h + iq2max + 1, *d_conv = mat0 + num_cov, *d_cnt = d_conv + nb;
     AXG_CUDA_TRY(ctx, cudaMemsetAsync(scratch, 0, nscr * 8, ctx->stream));
     // ---- compute_matrix_deconv (spectrum.f90:344-444) ----
     // the window is real: D2Z half spectrum (|W|^2 is the same for either sign)
     double *wreal = (double *)ctx->spec_buf;
     double2 *whalf = (double2 *)(((uintptr_t)(wreal + m3) + 255) & ~(uintptr_t)255);
-    AXG_LAUNCH(ctx, "spec_window", k_spec_window, grid_for(m3), 256, 0, ctx->flags, n, deg, dv_spa, wreal);
-    if (axg_ff_use(m))
-      AXG_TRY(axg_ff_d2z(ctx, wreal, whalf, m, 1));
-    else
-      AXG_CUFFT_TRY(ctx, cufftExecD2Z(ctx->plan_window, wreal, (cufftDoubleComplex *)whalf));
-    AXG_LAUNCH(ctx, "spec_w2_hist", k_spec_w2_hist, grid_for((int64_t)m * m * (m / 2 + 1)), 256, 0, whalf, m, h,
-               cnt);
-    std::vector<long long> hr(2 * (size_t)num_cov);
-    for (int ij = 0; ij < num_cov; ++ij) {
-      double e = ctx->h_largeq[(size_t)ij * 501 + kNumLargeq] / dwav;
-      long long imax2 = (long long)std::ceil(e * e) - 1;
-      e = ctx->h_largeq[(size_t)ij * 501] / dwav;
-      long long imin2 = (long long)std::ceil(e * e);
-      hr[2 * ij] = std::max(imin2, 0LL);
-      hr[2 * ij + 1] = std::min(imax2, (long long)iq2max);
+    // (our own transforms of an undegraded field read the flags in their row pass)
+    const bool ff = axg_ff_use(m), direct = ff && deg == 1;
+    const int wgrid = walk_grid(m, m / 2 + 1, 1);
+    if (direct) {
+      AXG_TRY(axg_ff_d2z_window(ctx, ctx->flags, dv_spa, whalf, m));
+    } else {
+      AXG_LAUNCH(ctx, "spec_window", k_spec_window, grid_for(m3), 256, 0, ctx->flags, n, deg, dv_spa, wreal);
+      if (ff) AXG_TRY(axg_ff_d2z(ctx, wreal, whalf, m, 1, true));
+      else AXG_CUFFT_TRY(ctx, cufftExecD2Z(ctx->plan_window, wreal, (cufftDoubleComplex *)whalf));
     }
-    AXG_CUDA_TRY(ctx, cudaMemcpyAsync(range, hr.data(), hr.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
-    AXG_LAUNCH(ctx, "spec_qtab", k_spec_qtab, grid_for(iq2max + 1), 256, 0, iq2max, dwav, qtab);
-    AXG_LAUNCH(ctx, "spec_mat", k_spec_mat, num_cov, 256, 0, h, cnt, ctx->spec_mat, ctx->spec_largeq0,
-               ctx->spec_dq, range, qtab, mat0, tat0);
+    if (ff) AXG_LAUNCH(ctx, "spec_w2_hist", k_spec_w2_hist<float4>, wgrid, 256, 0, (const float4 *)whalf, m, h);
+    else AXG_LAUNCH(ctx, "spec_w2_hist", k_spec_w2_hist<double2>, wgrid, 256, 0, whalf, m, h);
+    AXG_TRY(window_sums(ctx, h, iq2max, dwav, (Sums *)(scratch + nscr), mat0));
     // ---- compute_conv_spec (spectrum.f90:466-567) ----
-    if (fp32)
-      AXG_LAUNCH(ctx, "spec_degrade", k_spec_degrade<float2>, grid_for(m3), 256, 0, (const float2 *)ctx->phid,
-                 ctx->flags, n, deg, 1.0 / ((double)deg * deg * deg), 0, dv_spa, ctx->spec_buf);
-    else
-      AXG_LAUNCH(ctx, "spec_degrade", k_spec_degrade<double2>, grid_for(m3), 256, 0, (const double2 *)ctx->phid,
-                 ctx->flags, n, deg, 1.0 / ((double)deg * deg * deg), 0, dv_spa, ctx->spec_buf);
-    if (axg_ff_use(m))
-      AXG_TRY(axg_ff_z2z(ctx, (double2 *)ctx->spec_buf, m, 1));
-    else
-      AXG_CUFFT_TRY(ctx, cufftExecZ2Z(ctx->plan_spec, (cufftDoubleComplex *)ctx->spec_buf,
-                                      (cufftDoubleComplex *)ctx->spec_buf, CUFFT_INVERSE));
+    if (direct) {
+      AXG_TRY(axg_ff_z2z_masked(ctx, ctx->phid, fp32, ctx->flags, (double2 *)ctx->spec_buf, m, 1));
+    } else {
+      if (fp32)
+        AXG_LAUNCH(ctx, "spec_degrade", k_spec_degrade<float2>, grid_for(m3), 256, 0, (const float2 *)ctx->phid,
+                   ctx->flags, n, deg, 1.0 / ((double)deg * deg * deg), 0, dv_spa, ctx->spec_buf);
+      else
+        AXG_LAUNCH(ctx, "spec_degrade", k_spec_degrade<double2>, grid_for(m3), 256, 0, (const double2 *)ctx->phid,
+                   ctx->flags, n, deg, 1.0 / ((double)deg * deg * deg), 0, dv_spa, ctx->spec_buf);
+      if (ff)
+        AXG_TRY(axg_ff_z2z(ctx, (double2 *)ctx->spec_buf, m, 1, true));
+      else
+        AXG_CUFFT_TRY(ctx, cufftExecZ2Z(ctx->plan_spec, (cufftDoubleComplex *)ctx->spec_buf,
+                                        (cufftDoubleComplex *)ctx->spec_buf, CUFFT_INVERSE));
+    }
     const double dq = ctx->h_wav[1] - ctx->h_wav[0];
     const int16_t *tab = nullptr;
     AXG_TRY(axg_bin_table(ctx, AXG_BIN_SPECTRUM, m, dwav, dq, nb, 0, nullptr, &tab));
-    AXG_LAUNCH(ctx, "spec_bin", k_spec_bin, 152 * 4, 256, 2 * nb * sizeof(double), ctx->spec_buf, m, tab,
-               dv_spa * dv_spa * dv_wav, nb, d_conv, d_cnt);
+    const int brows = walk_rows(m, m), bgrid = walk_grid(m, m, brows);
+    if (ff)
+      AXG_LAUNCH(ctx, "spec_bin", k_spec_bin<float4>, bgrid, 256, bin_smem(nb),
+                 (const float4 *)ctx->spec_buf, m, brows, tab, nb, bin_copies(nb), d_conv, d_cnt);
+    else
+      AXG_LAUNCH(ctx, "spec_bin", k_spec_bin<double2>, bgrid, 256, bin_smem(nb),
+                 (const double2 *)ctx->spec_buf, m, brows, tab, nb, bin_copies(nb), d_conv, d_cnt);
     std::vector<double> hm(2 * num_cov), hb(2 * nb);
-    AXG_CUDA_TRY(ctx, cudaMemcpyAsync(hm.data(), mat0, hm.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    AXG_CUDA_TRY(ctx, cudaMemcpyAsync(hm.data(), mat0, (size_t)num_cov * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    AXG_CUDA_TRY(ctx, cudaMemcpyAsync(hm.data() + num_cov, ctx->spec_modes, (size_t)num_cov * 8, cudaMemcpyDeviceToHost,
+                                      ctx->stream));
     AXG_CUDA_TRY(ctx, cudaMemcpyAsync(hb.data(), d_conv, hb.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
     AXG_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     std::vector<double> mat(num_cov);
@@ -471,7 +607,7 @@ int axg_spec_estimation(axg_ctx *ctx, double tau, double *wave, double *power, d
       break;
     }
     // ---- spectrum_estimation (spectrum.f90:267-285) ----
-    const double t2 = tau * tau;
+    const double t2 = tau * tau * (dv_spa * dv_spa * dv_wav);  // |F dv_spa|^2 dv_wav tau^2
     std::vector<double> cv(nb), ct(nb), pw(nb, 0.0);
     for (int i = 1; i <= nb; ++i) {
       cv[i - 1] = hb[i - 1] * t2;
@@ -506,7 +642,6 @@ int axg_spec_estimation(axg_ctx *ctx, double tau, double *wave, double *power, d
   } while (0);
   cudaStreamSynchronize(ctx->stream);
   axg_free(ctx, (void **)&scratch);
-  axg_free(ctx, (void **)&range);
   return rc;
 }
 
@@ -575,12 +710,17 @@ int axg_spec_covariance(axg_ctx *ctx, int min_mc, int max_mc, double tol, double
                                       (cufftDoubleComplex *)ctx->spec_buf, CUFFT_FORWARD));
     AXG_LAUNCH(ctx, "mc_mask", k_mc_mask, grid_for(m3), 256, 0, ctx->spec_buf, ctx->flags, n, deg);
     if (ff)
-      AXG_TRY(axg_ff_z2z(ctx, (double2 *)ctx->spec_buf, m, 1));
+      AXG_TRY(axg_ff_z2z(ctx, (double2 *)ctx->spec_buf, m, 1, true));
     else
       AXG_CUFFT_TRY(ctx, cufftExecZ2Z(ctx->plan_spec, (cufftDoubleComplex *)ctx->spec_buf,
                                       (cufftDoubleComplex *)ctx->spec_buf, CUFFT_INVERSE));
-    AXG_LAUNCH(ctx, "mc_bin", k_spec_bin, 152 * 4, 256, 2 * nb * sizeof(double), ctx->spec_buf, m, tab, 1.0, nb,
-               d_pow, d_cnt);
+    const int brows = walk_rows(m, m), bgrid = walk_grid(m, m, brows);
+    if (ff)
+      AXG_LAUNCH(ctx, "mc_bin", k_spec_bin<float4>, bgrid, 256, bin_smem(nb),
+                 (const float4 *)ctx->spec_buf, m, brows, tab, nb, bin_copies(nb), d_pow, d_cnt);
+    else
+      AXG_LAUNCH(ctx, "mc_bin", k_spec_bin<double2>, bgrid, 256, bin_smem(nb),
+                 (const double2 *)ctx->spec_buf, m, brows, tab, nb, bin_copies(nb), d_pow, d_cnt);
     AXG_CUDA_TRY(ctx, cudaMemcpyAsync(pw0.data(), d_pow, sizeof(double) * nb, cudaMemcpyDeviceToHost, ctx->stream));
     AXG_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     // pow = mat_deconv pow0 - power (dspmv, beta = 1)
