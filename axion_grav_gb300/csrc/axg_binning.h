@@ -26,7 +26,10 @@ int axg_bin_table(axg_ctx *ctx, int kind, int m, double dwav, double dq, int nb,
 #ifdef __CUDACC__
 #include "axg_ff.h"
 
-// The block's bins in dynamic shared memory: sums in `copies` copies, spread
+// the integer wave vector of index j
+__device__ __forceinline__ int kint(int j, int n) { return (j + n / 2) % n - n / 2; }
+
+// The block's bins in shared memory (bin_smem bytes at mem): sums in `copies` copies, spread
 // over a warp's lanes, and counts.  A shared double is added to by a
 // compare-and-swap loop, and neighbouring lanes, whose |k| is nearly the same,
 // leave a bin together: with one copy the 256^3 field spectrum was binned in
@@ -35,9 +38,7 @@ struct BlockBins {
   double *v;
   unsigned *w;
   int nb, copies;
-  __device__ BlockBins(int nb_, int copies_) : nb(nb_), copies(copies_) {
-    extern __shared__ double axg_bins_sm[];
-    v = axg_bins_sm;
+  __device__ BlockBins(double *mem, int nb_, int copies_) : v(mem), nb(nb_), copies(copies_) {
     w = reinterpret_cast<unsigned *>(v + nb * copies);
     for (int i = threadIdx.x; i < nb * copies; i += blockDim.x) v[i] = 0.0;
     for (int i = threadIdx.x; i < nb; i += blockDim.x) w[i] = 0u;
@@ -59,6 +60,11 @@ struct BlockBins {
       }
   }
 };
+// the start of a kernel's dynamic shared memory
+__device__ __forceinline__ double *bins_mem() {
+  extern __shared__ double axg_bins_sm[];
+  return axg_bins_sm;
+}
 inline int bin_copies(int nb) {
   int c = 32;
   while (c > 1 && nb * c > 2048) c /= 2;

@@ -22,9 +22,10 @@
 //   y, z    : n-point FFTs along y and along z, a few adjacent kx columns per
 //             CTA so every row of the tile is one 64-byte segment.
 // The complex-float transforms (FP32-mixed Green sources and u_ij fields)
-// store their half spectra with kx rows padded to a multiple of 4 complex
-// values (axg_f32_spec_pitch): their y pass reads 32-byte rows on sector
-// boundaries, and their z pass moves its tiles by TMA (k_cols_z_tma).
+// store their half spectra with padded kx rows (axg_f32_spec_pitch); their y
+// pass moves its tiles by TMA (k_cols_tma), and the z pass hands its outputs to
+// what reads them, the TT power's shell sums or the Green accumulation, instead
+// of storing them (k_z_sink).
 // Each line is a Stockham radix-8 FFT in registers (f_stockham): a 512-point
 // line takes two shared-memory exchanges, the first pass reads its inputs
 // from global memory and the column passes' last pass writes there.
@@ -35,7 +36,9 @@
 #include <cstdlib>
 #include <vector>
 
+#include "axg_binning.h"
 #include "axg_ff.h"
+#include "axg_gw_site.h"
 #include "axg_gw_source.h"
 #include "axg_internal.h"
 #include "axg_tma.h"
@@ -248,14 +251,6 @@ __device__ __forceinline__ void load_tw(float4 *tw, const float4 *__restrict__ t
     tw[k + half] = c_neg(w);
   }
 }
-__device__ __forceinline__ void load_tw(float2 *tw, const float4 *__restrict__ twff, int half) {
-  for (int k = threadIdx.x; k < half; k += blockDim.x) {
-    const float4 w = twff[k];
-    tw[k] = make_float2(w.x, w.z);
-    tw[k + half] = make_float2(-w.x, -w.z);
-  }
-}
-
 // The split of an M-point FFT Z of packed reals into X[k], k <= M:
 // X[k] = E[k] + W_N^k O[k], E = (Z[k] + conj Z[M-k]) / 2,
 // O = (Z[k] - conj Z[M-k]) / 2i (W_N^M = -1).
@@ -589,8 +584,8 @@ int ff_gws_d2z_t(axg_ctx *ctx, const double2 *phi, double d, double inv_d, int d
 // central differences of phi: the row kernel forms S_ij for its rows from
 // phi (the stencil rows come through L1 / L2) and runs the real-to-half x
 // transform of all six at once, so the real sources never reach HBM; the y
-// and z passes are the column passes in complex float.  Output as cuFFT's
-// R2C: [6][n][n][n/2+1] complex float.  Twiddles are the high parts of the
+// and z passes are the TMA passes.  Output as cuFFT's R2C, rows padded:
+// [6][n][n][pitch] complex float.  Twiddles are the high parts of the
 // float-float table, i.e. W_n^k rounded to float.
 
 constexpr int kSrcRows = 2;  // x-rows per CTA of the source row pass (6 x 2 lines)
@@ -686,13 +681,15 @@ __global__ void __launch_bounds__(6 * kSrcRows * M / 8) k_gws_rows(const float2 
   });
 }
 
-// The u_ij spectrum's twelve real fields, tau u_c and u_c + tau u'_c (c =
+// The u_ij spectrum's twelve real fields, tau u_c and u_c + tau u'_c (tau with
+// taul, what a float of it drops; c =
 // 11, 21, 22, 31, 32, 33; FP32-mixed subtracts the Kahan compensation from
 // u first), formed inside the row pass as the Green sources are: one CTA per
 // x-row, twelve lines.  Output [12][n][n][n/2+1] complex float.
 template <int M>
 __global__ void __launch_bounds__(12 * M / 8) k_uij_rows(const float *__restrict__ u, const float *__restrict__ ud,
                                                          const float *__restrict__ cu, int64_t n3, float tau,
+                                                         float taul,
                                                          float2 *__restrict__ out, int sp,
                                                          const float4 *__restrict__ twff) {
   constexpr int N = 2 * M, TH = M / 8, LP = rowline_pitch<M>();
@@ -711,8 +708,9 @@ __global__ void __launch_bounds__(12 * M / 8) k_uij_rows(const float *__restrict
       uv.y -= cv.y;
     }
     const float2 dv = *reinterpret_cast<const float2 *>(ud + x);
-    s[c * LP + fswz(m)] = make_float2(tau * uv.x, tau * uv.y);
-    s[(6 + c) * LP + fswz(m)] = make_float2(uv.x + tau * dv.x, uv.y + tau * dv.y);
+    s[c * LP + fswz(m)] = make_float2(fmaf(taul, uv.x, tau * uv.x), fmaf(taul, uv.y, tau * uv.y));
+    s[(6 + c) * LP + fswz(m)] =
+        make_float2(fmaf(taul, dv.x, uv.x + tau * dv.x), fmaf(taul, dv.y, uv.y + tau * dv.y));
   }
   __syncthreads();
   {
@@ -775,136 +773,595 @@ __global__ void __launch_bounds__(M) k_ff_uij_rows(const double *__restrict__ u,
   }
 }
 
-// z pass of the complex-float half spectra through TMA.  Persistent CTAs
-// walk tiles of kFzCols kx columns x L z-points (one ky row of one field);
-// a tile arrives by cp.async.bulk.tensor in one of kFzStages shared-memory
-// stages while the CTA transforms the one before, and leaves by a bulk
-// tensor store from its own stage.  The spectra's rows are padded
-// (axg_f32_spec_pitch) so that their byte stride suits TMA; the last kx
-// block reaches past the pitch, where TMA loads zeros and drops the stores.
-// Each z-line is 64 bytes wide in 512 planes a megabyte apart: the plain
-// column kernel reached 0.53 of the DRAM peak on it, limited by the loads in
-// flight.  A stage wait that runs out raises AXG_KERR_MBAR_TIMEOUT.
-constexpr int kFzCols = 8;    // kx columns per tile: 64-byte boxes
-constexpr int kFzStages = 2;  // 3 and 4 stages at one CTA per SM measured slower
-constexpr int kFyCols = 4;    // kx columns per CTA of the y pass (32-byte rows, sector aligned at the padded pitch)
+constexpr int kFzCols = 8;  // kx columns per tile of the TMA passes: 64-byte boxes
 
+// The z pass of the complex-float half spectra with its consumer: the
+// transforms of a kx column's tensor components are contracted as they come
+// out, in the registers that hold them, and never stored.
+//
+// A persistent CTA takes items of kFzCols kx columns x L z-points at one ky;
+// the tiles of an item's fields follow each other through a ring of
+// shared-memory stages filled by cp.async.bulk.tensor, and so do chunks of what
+// the sink updates in memory.  The exchanges alternate between two line
+// buffers, so that each needs one barrier; the first one also frees the stage.
+// 128 registers a thread (16 warps an SM) hold the sums of a thread's eight
+// outputs.
+//
+// 512^3: u_ij z pass and shell sums 3.04 + 0.83 -> 2.70 ms (the lines alone 1.6,
+// the tiles' arrival 1.1); Green z pass and accumulation 1.34 + 2.31 -> 2.21 ms
+// (10.9 GB, 0.73 of the copy peak); 128^3 40 + 44 -> 48 and 23 + 39 -> 41 us.
+// With the accumulators read and written by the threads instead of through the
+// ring the Green form took 3.92 ms, its 16 warps waiting on them, and with
+// polarisations and TT coefficients over |k| (division, square root and 8 more
+// registers an output) the u_ij form 3.79.
 template <int L>
-constexpr size_t zt_smem() {
-  return (size_t)(kFzStages * L * kFzCols + (L + L / 8) * kFzCols + L) * sizeof(float2) + 8 * kFzStages + 16 + 128;
+constexpr int zs_stages() {
+  return L >= 512 ? 4 : 3;
+}
+template <int L>
+constexpr int zs_blocks() {  // CTAs per SM: 512 threads, at most 16
+  return L < 32 ? 16 : 4096 / (kFzCols * L);
+}
+template <int L>
+constexpr size_t zs_smem() {  // without the sink's
+  return (size_t)(zs_stages<L>() * L * kFzCols + 2 * (L + L / 8) * kFzCols + L) * sizeof(float2) + 8 * zs_stages<L>() +
+         128 + 16;
+}
+// the last pass of an L-point line: its stride (L / its radix), and the z index
+// of thread j's output in slot s less j
+template <int L>
+constexpr int z_last_ns() {
+  int ns = 1;
+  while (L / ns > 8) ns *= 8;
+  return ns;
+}
+template <int L>
+__host__ __device__ constexpr int z_off(int s) {
+  constexpr int NS = z_last_ns<L>(), R = L / NS;
+  return (s / R) * (L / 8) + (s % R) * NS;
+}
+// ... its wave number, from j as a float: outputs r >= R / 2 are the negative ones
+template <int L>
+__device__ __forceinline__ float z_wave(float jf, int s) {
+  constexpr int R = L / z_last_ns<L>();
+  return jf + (float)(z_off<L>(s) - (s % R >= R / 2 ? L : 0));
 }
 
+// j as a float the compiler knows nothing of: what depends on it is formed where
+// it is used, not ahead of the loop over an item's fields (where the values of
+// all eight outputs and six components spilled 300 bytes a thread)
+__device__ __forceinline__ float fresh(int j) {
+  asm volatile("" : "+r"(j));
+  return (float)j;
+}
+
+// Twiddles of the passes NS = 8, 64 of an L-point line: W_(NS R)^(r k) at
+// (r - 1) NS + k after those of the pass before, consecutive k on consecutive
+// banks.
 template <int L>
-__global__ void __launch_bounds__(kFzCols * L / 8, (1024 / (kFzCols * L / 8)) < 32 ? 1024 / (kFzCols * L / 8) : 32)
-    k_cols_z_tma(const __grid_constant__ CUtensorMap tm, int nkb, int ny, int ntiles,
-                 const float4 *__restrict__ twff, int *err) {
+__device__ __forceinline__ void load_tw_z(float2 *tw, const float4 *__restrict__ twff) {
+  int at = 0;
+  for (int ns = 8; ns < L; ns *= 8) {
+    const int R = L / ns >= 8 ? 8 : L / ns;
+    for (int e = threadIdx.x; e < (R - 1) * ns; e += blockDim.x) {
+      const int r = 1 + e / ns, k = e % ns, i = r * k * (L / (ns * R));  // < L
+      const float4 w = twff[i & (L / 2 - 1)];
+      tw[at + e] = i < L / 2 ? make_float2(w.x, w.z) : make_float2(-w.x, -w.z);
+    }
+    at += (R - 1) * ns;
+  }
+}
+
+// fpad(i + s) - fpad(i) for the passes' offsets s: multiples of 8, or i + s % 8 < 8
+constexpr int z_pad(int s) { return (s + s / 8) * kFzCols; }
+
+// one exchange and the passes NS >= 8 after it: outputs of the pass before in v,
+// element i + r NS0 of the line in v[r]; the outputs stay in v.  sync: the
+// barrier of this exchange; buf: the buffers, swapped at each exchange.
+template <int L, int NS, typename Sync>
+__device__ __forceinline__ void z_passes(float2 v[8], int j, float2 *&b0, float2 *&b1, const float2 *tw, Sync sync) {
+  constexpr int NS0 = NS / 8, R = L / NS >= 8 ? 8 : L / NS, NI = 8 / R, TH = L / 8;
+  {
+    const int d = (j / NS0) * NS + (j & (NS0 - 1));
+    float2 *w = b0 + fpad(d) * kFzCols;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) w[NS0 == 1 ? r * kFzCols : z_pad(r * NS0)] = v[r];
+  }
+  sync();
+  {
+    const float2 *p = b0 + fpad(j) * kFzCols;
+#pragma unroll
+    for (int q = 0; q < NI; ++q)
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[q * R + r] = p[z_pad(q * TH + r * (L / R))];
+  }
+  float2 *const t = b0;
+  b0 = b1;
+  b1 = t;
+#pragma unroll
+  for (int q = 0; q < NI; ++q) {
+    const int k = (j + q * TH) & (NS - 1);
+#pragma unroll
+    for (int r = 1; r < R; ++r) v[q * R + r] = c_mul(v[q * R + r], tw[(r - 1) * NS + k]);
+    c_dft<R, false>(&v[q * R]);
+  }
+  if constexpr (NS * R < L) z_passes<L, NS * 8>(v, j, b0, b1, tw + (R - 1) * NS, [] { __syncthreads(); });
+}
+
+// y pass of the complex-float half spectra (Z: z pass): persistent CTAs walk
+// tiles of kFzCols kx columns x L points (one z plane of one field; one ky)
+// through the ring of stages; a tile is transformed into its own stage and leaves by a bulk
+// tensor store.  A wait that runs out raises AXG_KERR_MBAR_TIMEOUT.  512^3, six
+// spectra: 1.30 ms by one CTA per 4 columns from the threads' loads (32-byte
+// rows), 1.09 so (0.90 of the copy peak).
+template <int L, bool Z>
+__global__ void __launch_bounds__(kFzCols *L / 8, zs_blocks<L>())
+    k_cols_tma(const __grid_constant__ CUtensorMap tm, int nkb, int ntiles_all, const float4 *__restrict__ twff, int *err) {
   using namespace axg_tma;
-  constexpr int TH = L / 8, LP = L + L / 8, TILE = L * kFzCols, BOX = L < 256 ? L : 256, S = kFzStages;
-  constexpr uint32_t BYTES = TILE * sizeof(float2);
+  constexpr int TH = L / 8, LP = L + L / 8, TILE = L * kFzCols, BOX = L < 256 ? L : 256, S = zs_stages<L>();
   extern __shared__ unsigned char zt_raw[];
   unsigned char *sm =
       reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(zt_raw) + 127) & ~uintptr_t(127));
-  float2 *tile = reinterpret_cast<float2 *>(sm);  // [S][L][kFzCols], dense as the TMA box
-  float2 *xb = tile + S * TILE;                    // exchange lines, element i of column c at fpad(i) kFzCols + c
-  float2 *tw = xb + LP * kFzCols;                  // W_L^k, k < L
+  float2 *tile = reinterpret_cast<float2 *>(sm);
+  float2 *xb = tile + S * TILE;
+  float2 *tw = xb + 2 * LP * kFzCols;
   uint64_t *bars = reinterpret_cast<uint64_t *>(tw + L);
-  int &fail = *reinterpret_cast<int *>(bars + S);
-  load_tw(tw, twff, L / 2);
+  load_tw_z<L>(tw, twff);
   const uint32_t bar0 = smem_u32(bars);
   if (threadIdx.x == 0) {
     for (int q = 0; q < S; ++q) mbar_init(bar0 + 8 * q, 1);
     fence_barrier_init();
-    fail = 0;
   }
   __syncthreads();
-  auto issue = [&](int t, int st) {  // tile t: (field, ky) = o, kx block kb
-    const int o = t / nkb, kb = t % nkb;
-    const uint32_t dst = smem_u32(tile + st * TILE), bar = bar0 + 8 * st;
-    mbar_expect_tx(bar, BYTES);
-#pragma unroll
-    for (int h = 0; h < L / BOX; ++h)
-      tma_load_4d(dst + h * BOX * kFzCols * (int)sizeof(float2), &tm, kb * kFzCols, o % ny, h * BOX, o / ny, bar);
+  const int ntiles = (ntiles_all - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  int next = 0;  // thread 0: the CTA's next tile to load
+  auto at = [&](int t, int &kb, int &z, int &f) {
+    const int i = blockIdx.x + t * (int)gridDim.x, o = i / nkb;
+    kb = i - o * nkb;
+    f = o / L;
+    z = o & (L - 1);
   };
-  if (threadIdx.x == 0)
-    for (int q = 0; q < S - 1; ++q)
-      if (blockIdx.x + q * (int)gridDim.x < ntiles) issue(blockIdx.x + q * gridDim.x, q);
-  const int c = threadIdx.x % kFzCols, j = threadIdx.x / kFzCols;
-  int i = 0;
-  for (int t = blockIdx.x; t < ntiles; ++i, t += gridDim.x) {
-    const int st = i % S;
-    const int tn = t + (S - 1) * (int)gridDim.x;
-    if (threadIdx.x == 0 && tn < ntiles) {
-      bulk_wait_read0();  // the store of the previous tile, from the stage about to be refilled, has read it
-      issue(tn, (i + S - 1) % S);
+  auto load_to = [&](int limit) {
+    for (; next < limit && next < ntiles; ++next) {
+      int kb, z, f;
+      at(next, kb, z, f);
+      const uint32_t dst = smem_u32(tile + next % S * TILE), bar = bar0 + 8 * (next % S);
+      mbar_expect_tx(bar, TILE * sizeof(float2));
+#pragma unroll
+      for (int h = 0; h < L / BOX; ++h)
+        tma_load_4d(dst + h * BOX * kFzCols * (int)sizeof(float2), &tm, kb * kFzCols, Z ? z : h * BOX,
+                    Z ? h * BOX : z, f, bar);
     }
-    if (!mbar_wait_bounded(bar0 + 8 * st, (i / S) & 1)) fail = 1;
-    __syncthreads();
-    if (fail) break;
-    float2 *tl = tile + st * TILE;
+  };
+  if (threadIdx.x == 0) load_to(S);
+  const int c = threadIdx.x % kFzCols, j = threadIdx.x / kFzCols;
+  float2 *b0 = xb + c, *b1 = b0 + LP * kFzCols;
+  int t = 0, bad = 0;
+  for (; t < ntiles; ++t) {
+    const int late = !mbar_wait_bounded(bar0 + 8 * (t % S), (t / S) & 1);
+    float2 *tl = tile + t % S * TILE;
     float2 v[8];
 #pragma unroll
     for (int r = 0; r < 8; ++r) v[r] = tl[(j + r * TH) * kFzCols + c];
-    f_stockham<L, 1, false>(v, j, xb + c, kFzCols, tw, 1, [&](int ii, float2 z) { tl[ii * kFzCols + c] = z; });
+    c_dft<8, false>(v);
+    z_passes<L, 8>(v, j, b0, b1, tw, [&] {
+      bad = __syncthreads_or(late);  // every thread has read the stage
+      if (threadIdx.x == 0 && !bad && t > 0 && next < ntiles) {
+        bulk_wait_read0();  // the store of the tile before has, too
+        load_to(t + S);
+      }
+    });
+    if (bad) break;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) tl[(j + z_off<L>(s)) * kFzCols + c] = v[s];
     fence_proxy_async();
     __syncthreads();
     if (threadIdx.x == 0) {
-      const int o = t / nkb, kb = t % nkb;
+      int kb, z, f;
+      at(t, kb, z, f);
       const uint32_t src = smem_u32(tl);
 #pragma unroll
       for (int h = 0; h < L / BOX; ++h)
-        tma_store_4d(&tm, src + h * BOX * kFzCols * (int)sizeof(float2), kb * kFzCols, o % ny, h * BOX, o / ny);
+        tma_store_4d(&tm, src + h * BOX * kFzCols * (int)sizeof(float2), kb * kFzCols, Z ? z : h * BOX,
+                     Z ? h * BOX : z, f);
       bulk_commit();
     }
   }
   if (threadIdx.x == 0) {
-    if (fail) {
+    if (bad) {
       atomicCAS(err, 0, AXG_KERR_MBAR_TIMEOUT);
-      for (int q = 1; q < S; ++q) mbar_wait_bounded(bar0 + 8 * ((i + q) % S), ((i + q) / S) & 1, 100000000LL);
+      for (int q = t + 1; q < next; ++q) mbar_wait_bounded(bar0 + 8 * (q % S), (q / S) & 1, 100000000LL);
     }
     bulk_wait0();
   }
 }
 
-// y and z passes in complex float of `batch` half spectra, rows of pitch sp
-// (axg_f32_spec_pitch): the y pass by k_cols (kFyCols columns, 32-byte
-// rows on sector boundaries), the z pass by k_cols_z_tma
+// A sink: kFields tiles an item, field(f) the spectrum of tile f, then kChunks
+// chunks of rows that it updates; begin, take (tile f's outputs in v, slot s
+// at z = j + z_off(s)), chunk and end of an item; finish.
+template <int L, typename Sink>
+__global__ void __launch_bounds__(kFzCols *L / 8, zs_blocks<L>())
+    k_z_sink(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tc, int nkb, int nitems,
+             const float4 *__restrict__ twff, const typename Sink::Args args, int *err) {
+  using namespace axg_tma;
+  constexpr int TH = L / 8, LP = L + L / 8, TILE = L * kFzCols, BOX = L < 256 ? L : 256, S = zs_stages<L>(),
+                NF = Sink::kFields, NT = NF + Sink::kChunks;
+  constexpr uint32_t BYTES = TILE * sizeof(float2);
+  extern __shared__ unsigned char zt_raw[];
+  unsigned char *sm =
+      reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(zt_raw) + 127) & ~uintptr_t(127));
+  float2 *tile = reinterpret_cast<float2 *>(sm);  // [S][L][kFzCols], dense as the TMA box
+  float2 *xb = tile + S * TILE;                    // two sets of exchange lines
+  float2 *tw = xb + 2 * LP * kFzCols;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(tw + L);
+  load_tw_z<L>(tw, twff);
+  const uint32_t bar0 = smem_u32(bars);
+  if (threadIdx.x == 0) {
+    for (int q = 0; q < S; ++q) mbar_init(bar0 + 8 * q, 1);
+    fence_barrier_init();
+  }
+  Sink sink(args, reinterpret_cast<double *>(bars + S));
+  __syncthreads();
+  const int ntiles = (nitems - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * NT;
+  int next = 0;                      // thread 0: the CTA's next tile to load
+  auto load_to = [&](int limit) {
+    for (; next < limit && next < ntiles; ++next) {
+      const int item = blockIdx.x + (next / NT) * (int)gridDim.x, o = item / nkb, kb = item % nkb, f = next % NT;
+      const uint32_t dst = smem_u32(tile + next % S * TILE), bar = bar0 + 8 * (next % S);
+      if (f < NF) {
+        mbar_expect_tx(bar, BYTES);
+#pragma unroll
+        for (int h = 0; h < L / BOX; ++h)
+          tma_load_4d(dst + h * BOX * kFzCols * (int)sizeof(float2), &tm, kb * kFzCols, o, h * BOX, Sink::field(f),
+                      bar);
+      } else {
+        sink.load_chunk(&tc, dst, bar, kb, o, f - NF);
+      }
+    }
+  };
+  if (threadIdx.x == 0) load_to(S);
+  const int c = threadIdx.x % kFzCols, j = threadIdx.x / kFzCols;
+  float2 *b0 = xb + c, *b1 = b0 + LP * kFzCols;
+  int t = 0, bad = 0;
+  for (int item = blockIdx.x; item < nitems && !bad; item += gridDim.x) {
+    const int ky = item / nkb, kb = item % nkb;
+    sink.begin(kb * kFzCols + c, ky);
+#pragma unroll 1
+    for (int f = 0; f < NF; ++f, ++t) {
+      const int late = !mbar_wait_bounded(bar0 + 8 * (t % S), (t / S) & 1);
+      const float2 *tl = tile + t % S * TILE + j * kFzCols + c;
+      float2 v[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) v[r] = tl[r * TH * kFzCols];
+      c_dft<8, false>(v);
+      z_passes<L, 8>(v, j, b0, b1, tw, [&] {
+        bad = __syncthreads_or(late);  // every thread has read the stage
+        if (threadIdx.x == 0 && !bad) {
+          if (Sink::kChunks && next < ntiles) bulk_wait_read0();  // the last chunk's store has, too
+          load_to(t + 1 + S);
+        }
+      });
+      if (bad) break;
+      sink.take(f, v, j);
+    }
+    if constexpr (Sink::kChunks > 0) {
+#pragma unroll
+      for (int f = 0; f < Sink::kChunks; ++f) {
+        if (bad) break;
+        const int late = !mbar_wait_bounded(bar0 + 8 * (t % S), (t / S) & 1);
+        float2 *tl = tile + t % S * TILE;
+        if (!late) sink.chunk(f, reinterpret_cast<float4 *>(tl), j, c);
+        fence_proxy_async();
+        bad = __syncthreads_or(late);
+        if (bad) break;
+        if (threadIdx.x == 0) {
+          if (next < ntiles) bulk_wait_read0();  // the store before this one has read its stage
+          load_to(t + S);
+          sink.store_chunk(&tc, smem_u32(tl), kb, ky, f);
+          bulk_commit();
+        }
+        ++t;
+      }
+    }
+    if (!bad) sink.end(j, c, b0, b1);
+  }
+  if (threadIdx.x == 0) {
+    if (bad) {
+      atomicCAS(err, 0, AXG_KERR_MBAR_TIMEOUT);
+      for (int q = t + 1; q < next; ++q) mbar_wait_bounded(bar0 + 8 * (q % S), (q / S) & 1, 100000000LL);
+    }
+    bulk_wait0();
+  }
+  sink.finish();
+}
+
+// TT power of u_ij into shell sums: tt_basis times k^2, whose coefficients are
+// polynomials in kz, U_mm - U_ll in A and |k| U_ml in B.  The trace drops out
+// through the differences to component 33, so that one and 11 come first.
 template <int L>
-int f_cols_t(axg_ctx *ctx, float2 *out, int batch, int sp, const float4 *tw) {
-  constexpr int n = L, nh = L / 2 + 1;
-  const int64_t plane = (int64_t)n * sp, vol = plane * n;
-  const int nky = (nh + kFyCols - 1) / kFyCols;
-  AXG_TRY((launch_cols<float2, L, kFyCols, false>(ctx, "fft_f32_y", (int64_t)batch * n * nky, out, nh, n, vol, plane,
-                                                   (int64_t)sp, tw, 0)));
-  CUtensorMap m;
-  constexpr int BOX = L < 256 ? L : 256;
-  const cuuint64_t dims[4] = {(cuuint64_t)sp, (cuuint64_t)n, (cuuint64_t)n, (cuuint64_t)batch};
-  const cuuint64_t str[3] = {(cuuint64_t)sp * 8, (cuuint64_t)plane * 8, (cuuint64_t)vol * 8};
-  const cuuint32_t box[4] = {kFzCols, 1, BOX, 1};
-  AXG_TRY(axg_encode_tmap(ctx, &m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, out, dims, str, box));  // (re, im) float pairs
-  constexpr size_t smem = zt_smem<L>();
+struct UijSink {
+  static constexpr int kFields = 12, kChunks = 0;  // 33, 11, 22, 21, 31, 32 of w', then of w
+  struct Args {
+    const int16_t *tab;
+    int nb, copies;
+    float dwav2, dwavl;  // and what a float of it drops
+    double *numer, *denom;
+  };
+  __device__ __forceinline__ static int field(int f) {
+    const int g = f % 6;
+    return (f < 6 ? 6 : 0) + (g == 0 ? 5 : g == 1 ? 0 : g == 2 ? 2 : g == 3 ? 1 : g - 1);
+  }
+  __device__ __forceinline__ void load_chunk(const CUtensorMap *, uint32_t, uint32_t, int, int, int) {}
+  __device__ __forceinline__ void store_chunk(const CUtensorMap *, uint32_t, int, int, int) {}
+  const Args &a;
+  BlockBins bins;
+  BinRun<F2> run;
+  int ix;
+  float kx, ky, sc, df;  // s c and s^2 - c^2 of the azimuth
+  float e[8];
+  float2 A[8], B[8];
+  __device__ UijSink(const Args &args, double *mem) : a(args), bins(mem, args.nb, args.copies) {}
+  __device__ __forceinline__ void begin(int hx, int hy) {
+    ix = hx;
+    kx = (float)(hx < L / 2 ? hx : hx - L);
+    ky = (float)(hy < L / 2 ? hy : hy - L);
+    const float p2 = kx * kx + ky * ky, ip2 = p2 > 0.f ? 1.f / p2 : 0.f;
+    sc = kx * ky * ip2;
+    df = p2 > 0.f ? (ky * ky - kx * kx) * ip2 : -1.f;
+  }
+  __device__ __forceinline__ void take(int f, const float2 v[8], int j) {
+    const int g = f < 6 ? f : f - 6;
+    const float jf = fresh(j);
+    if (g == 0) {
+#pragma unroll
+      for (int s = 0; s < 8; ++s) A[s] = v[s];
+    } else if (g == 1) {
+#pragma unroll
+      for (int s = 0; s < 8; ++s) B[s] = v[s];
+    } else if (g == 2) {
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        // k^2 (s^2 - q^2 c^2) = ky^2 + kz^2 (s^2 - c^2), and 22 with kx, -
+        const float kz = z_wave<L>(jf, s), kd = kz * kz * df;
+        const float a11 = fmaf(ky, ky, kd), a22 = fmaf(kx, kx, -kd), b11 = kz * sc;
+        const float2 x33 = A[s], x11 = B[s];
+        A[s].x = a11 * (x11.x - x33.x) + a22 * (v[s].x - x33.x);
+        A[s].y = a11 * (x11.y - x33.y) + a22 * (v[s].y - x33.y);
+        B[s].x = b11 * (x11.x - v[s].x);
+        B[s].y = b11 * (x11.y - v[s].y);
+      }
+    } else if (g == 3) {
+      const float m2 = -2.f * kx * ky, m4 = -4.f * sc;  // -2 s c (k^2 + kz^2)
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const float kz = z_wave<L>(jf, s);
+        add(s, fmaf(kz * kz, m4, m2), kz * df, v[s]);
+      }
+    } else {
+      const float ka = 2.f * (g == 4 ? kx : ky), kb = g == 4 ? -ky : kx;
+#pragma unroll
+      for (int s = 0; s < 8; ++s) add(s, z_wave<L>(jf, s) * ka, kb, v[s]);
+      if (g == 5) {
+        const float p2 = kx * kx + ky * ky;
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          const float kz = z_wave<L>(jf, s), k2 = fmaf(kz, kz, p2), ik = gw_rsqrt(k2), i2 = ik * ik;
+          const float px = A[s].x * i2, py = A[s].y * i2, cx = B[s].x * ik, cy = B[s].y * ik;
+          const float p = 0.5f * (px * px + py * py) + 2.f * (cx * cx + cy * cy);
+          e[s] = f < 6 ? p : fmaf(fmaf(k2, a.dwavl, k2 * a.dwav2), p, e[s]);
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ void add(int s, float ca, float cb, float2 v) {
+    A[s].x = fmaf(ca, v.x, A[s].x);
+    A[s].y = fmaf(ca, v.y, A[s].y);
+    B[s].x = fmaf(cb, v.x, B[s].x);
+    B[s].y = fmaf(cb, v.y, B[s].y);
+  }
+  // The item's powers to the bins: through an exchange buffer, so that a thread
+  // sums runs of |kz| (kz and -kz share their bin) before it adds to the shared
+  // bins; added as they lie, 8 values in 8 bins, they took 0.6 ms at 512^3.
+  __device__ __forceinline__ void end(int j, int c, float2 *&b0, float2 *&b1) {
+    constexpr int TH = L / 8, PER = L / 2 / TH;
+    float *x = reinterpret_cast<float *>(b0 - c) + c;
+    auto at = [](int z) { return (z + z / 4) * kFzCols; };
+#pragma unroll
+    for (int s = 0; s < 8; ++s) x[at(j + z_off<L>(s))] = e[s];
+    __syncthreads();
+    if (ix <= L / 2) {
+      const unsigned wgt = (ix == 0 || ix == L / 2) ? 1u : 2u;  // Hermitian partner of the half spectrum
+      const int p2 = (int)(kx * kx + ky * ky);
+      auto put = [&](int z, F2 v, unsigned w) {
+        const int b = a.tab[p2 + z * z];
+        if (b >= 0) run.add(bins, b, F2{(float)wgt * v.h, (float)wgt * v.l}, wgt * w);
+      };
+      if (j == 0) put(0, F2{x[0], 0.f}, 1u);
+#pragma unroll
+      for (int i = 1; i <= PER; ++i) {
+        const int z = j * PER + i;
+        const F2 v = {x[at(z)], 0.f};
+        if (z < L / 2) put(z, f2_add(v, F2{x[at(L - z)], 0.f}), 2u);
+        else put(z, v, 1u);
+      }
+      run.flush(bins);
+    }
+    float2 *const t = b0;
+    b0 = b1;
+    b1 = t;
+  }
+  __device__ __forceinline__ void finish() { bins.finish(a.numer, a.denom); }
+};
+
+// The Green accumulation.  With e+ times k^2, the contractions split into sums
+// whose coefficients are polynomials in kz:
+//   Sa = sum k^2 Re(e) Re(S), Se = sum k^2 Re(e) Im(S),
+//   Sb = sum |k| Im(e) Im(S), Sg = sum |k| Im(e) Re(S)   (S conjugated),
+// X+ = (Sa - Sb', Se + Sg'), X- = (Sa + Sb', Se - Sg') over k^2.  A chunk is the
+// accumulators of one output slot of every thread.
+template <int L>
+struct GreenSink {
+  static constexpr int kFields = 6, kChunks = 8;
+  static constexpr int NH = L / 2 + 1, TH = L / 8, SP = axg_f32_spec_pitch(L);
+  struct Args {
+    float2 *srcF;
+    int ref_compat;
+    float Th, Tl, dw, dwl;
+  };
+  __device__ __forceinline__ static int field(int f) { return f; }
+  const Args &a;
+  int ix, iy;
+  float kx, ky, cs, df;  // c s and c^2 - s^2 of the azimuth
+  float2 R[8], I[8];     // (Sa, Se), (Sb, Sg)
+  float2 last[8];        // the source 33
+  __device__ GreenSink(const Args &args, double *) : a(args) {}
+  // the chunk in a stage: [4][TH][kFzCols] float4
+  __device__ __forceinline__ void load_chunk(const CUtensorMap *tc, uint32_t dst, uint32_t bar, int kb, int o, int f) {
+    constexpr uint32_t ONE = TH * kFzCols * sizeof(float4);
+    axg_tma::mbar_expect_tx(bar, (a.ref_compat ? 3 : 4) * ONE);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (q != 1 || !a.ref_compat) axg_tma::tma_load_4d(dst + q * ONE, tc, kb * kFzCols * 2, o, z_off<L>(f), q, bar);
+  }
+  __device__ __forceinline__ void store_chunk(const CUtensorMap *tc, uint32_t src, int kb, int o, int f) {
+    constexpr uint32_t ONE = TH * kFzCols * sizeof(float4);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) axg_tma::tma_store_4d(tc, src + q * ONE, kb * kFzCols * 2, o, z_off<L>(f), q);
+  }
+  __device__ __forceinline__ void begin(int hx, int hy) {
+    ix = hx;
+    iy = hy;
+    kx = (float)(hx < L / 2 ? hx : hx - L);
+    ky = (float)(hy < L / 2 ? hy : hy - L);
+    const float p2 = kx * kx + ky * ky, ip2 = p2 > 0.f ? 1.f / p2 : 0.f;
+    cs = kx * ky * ip2;
+    df = p2 > 0.f ? (kx * kx - ky * ky) * ip2 : 1.f;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) R[s] = I[s] = make_float2(0.f, 0.f);
+  }
+  __device__ __forceinline__ void add(int s, float pr, float pi, float2 v) {
+    R[s].x = fmaf(pr, v.x, R[s].x);
+    R[s].y = fmaf(-pr, v.y, R[s].y);
+    I[s].x = fmaf(-pi, v.y, I[s].x);
+    I[s].y = fmaf(pi, v.x, I[s].y);
+  }
+  __device__ __forceinline__ void take(int f, const float2 v[8], int j) {
+    const float jf = fresh(j);
+    // e+_ij = p_i p_j, halved on the diagonal, |k| p = (kz c - i |k| s, kz s + i |k| c, -p)
+    if (f == 0 || f == 2) {
+      const float h = (f == 0 ? 0.5f : -0.5f) * df, k = f == 0 ? ky : kx, g = -0.5f * k * k, t = f == 0 ? -cs : cs;
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const float kz = z_wave<L>(jf, s);
+        add(s, fmaf(kz * kz, h, g), kz * t, v[s]);
+      }
+    } else if (f == 1) {
+      const float h = 2.f * cs, g = kx * ky;
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const float kz = z_wave<L>(jf, s);
+        add(s, fmaf(kz * kz, h, g), kz * df, v[s]);
+      }
+    } else if (f < 5) {
+      const float k = f == 3 ? -kx : -ky, t = f == 3 ? ky : -kx;  // p s = ky, p c = kx
+#pragma unroll
+      for (int s = 0; s < 8; ++s) add(s, z_wave<L>(jf, s) * k, t, v[s]);
+    } else {
+#pragma unroll
+      for (int s = 0; s < 8; ++s) last[s] = v[s];
+    }
+    // the rows whose mirrors are entries of their own keep their transforms
+    constexpr int ny = L / 2 / z_last_ns<L>();  // the slot of z = n/2, thread j = 0
+    if (ix > 0 && ix < L / 2 && (iy == L / 2 || j == 0)) {
+      float2 *o = a.srcF + ((int64_t)(f * L + j) * L + iy) * SP + ix;
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (iy == L / 2 || s == ny) o[(int64_t)z_off<L>(s) * L * SP] = v[s];
+    }
+  }
+  __device__ __forceinline__ void chunk(int s, float4 *tl, int j, int c) {
+    float4 *t = tl + j * kFzCols + c;
+    constexpr int ONE = TH * kFzCols;
+    const float kz = z_wave<L>(fresh(j), s), p2 = kx * kx + ky * ky, k2 = fmaf(kz, kz, p2);
+    F32Acc ac;
+    ac.load(t, ONE, 0, a.ref_compat);
+    if (k2 > 0.f) {
+      const float ik = gw_rsqrt(k2), i2 = ik * ik;
+      // e33 = p^2 / 2: its part of X-, and its parts of Sa and Se
+      const float h = 0.5f * p2, lr = h * last[s].x, li = h * -last[s].y;
+      const float Ra = (R[s].x + lr) * i2, Re = (R[s].y + li) * i2, Ib = I[s].x * ik, Ig = I[s].y * ik;
+      const float x[2] = {Ra - Ib, Re + Ig}, m[2] = {Ra + Ib, Re - Ig}, l[2] = {lr * i2, li * i2};
+      float sq, cq;
+      gw_cos_sin(k2, ik, a.Th, a.Tl, &cq, &sq);
+      ac.update(fmaf(a.dwl, cq, a.dw * cq), fmaf(a.dwl, sq, a.dw * sq), x, m, l, a.ref_compat);
+    } else if (a.ref_compat) {
+      ac.a21 = ac.a12;
+    }
+    ac.store(t, ONE, 0);
+  }
+  __device__ __forceinline__ void end(int, int, float2 *&, float2 *&) {}
+  __device__ __forceinline__ void finish() {}
+};
+
+// a persistent TMA pass: as many CTAs as fit, at most `items`
+template <int L, typename K, typename... A>
+int launch_persistent(axg_ctx *ctx, const char *name, K kern, int items, size_t smem, const A &...args) {
+  AXG_TRY(allow_smem(ctx, kern, smem));
+  AXG_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   constexpr int threads = kFzCols * L / 8;
-  AXG_TRY(allow_smem(ctx, k_cols_z_tma<L>, smem));
-  AXG_CUDA_TRY(ctx, cudaFuncSetAttribute(k_cols_z_tma<L>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   int per_sm = 0, sms = 0;
-  AXG_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cols_z_tma<L>, threads, smem));
-  if (per_sm < 1) return axg_set_error(ctx, AXG_ERR_CUDA, "z-pass kernel does not fit on an SM");
+  AXG_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
+  if (per_sm < 1) return axg_set_error(ctx, AXG_ERR_CUDA, "transform kernel does not fit on an SM");
   AXG_CUDA_TRY(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-  const int nkb = (nh + kFzCols - 1) / kFzCols, ntiles = batch * n * nkb;
-  const int grid = std::min(ntiles, sms * per_sm);
-  AXG_LAUNCH(ctx, "fft_f32_z", k_cols_z_tma<L>, (unsigned)grid, threads, smem, m, nkb, n, ntiles, tw, ctx->d_err);
+  AXG_LAUNCH(ctx, name, kern, (unsigned)std::min(items, sms * per_sm), threads, smem, args...);
   return AXG_OK;
 }
 
+// The tensor maps of `batch` half spectra, (re, im) float pairs, by tiles along
+// y and along z
 template <int L>
-int uij_r2c_t(axg_ctx *ctx, const float *u, const float *ud, const float *cu, float tau, float2 *out,
-              const float4 *tw) {
+int spec_tmaps(axg_ctx *ctx, float2 *F, int batch, CUtensorMap *my, CUtensorMap *mz) {
+  constexpr int n = L, sp = axg_f32_spec_pitch(L), BOX = L < 256 ? L : 256;
+  const cuuint64_t dims[4] = {(cuuint64_t)sp, (cuuint64_t)n, (cuuint64_t)n, (cuuint64_t)batch};
+  const cuuint64_t str[3] = {(cuuint64_t)sp * 8, (cuuint64_t)n * sp * 8, (cuuint64_t)n * n * sp * 8};
+  const cuuint32_t ybox[4] = {kFzCols, BOX, 1, 1}, zbox[4] = {kFzCols, 1, BOX, 1};
+  AXG_TRY(axg_encode_tmap(ctx, my, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, F, dims, str, ybox));
+  return axg_encode_tmap(ctx, mz, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, F, dims, str, zbox);
+}
+
+// the y pass in complex float of a sink's half spectra and their z pass into it
+template <int L, typename Sink>
+int f_cols_sink(axg_ctx *ctx, const char *name, float2 *F, const float4 *tw, const typename Sink::Args &args,
+                size_t sink_smem) {
+  constexpr int n = L, nh = L / 2 + 1, batch = Sink::kFields, nkb = (nh + kFzCols - 1) / kFzCols;
+  CUtensorMap my, mz;
+  AXG_TRY(spec_tmaps<L>(ctx, F, batch, &my, &mz));
+  CUtensorMap mc = mz;
+  if (Sink::kChunks) {
+    const cuuint64_t adims[4] = {(cuuint64_t)2 * nh, (cuuint64_t)n, (cuuint64_t)n, 4};
+    const cuuint64_t astr[3] = {(cuuint64_t)nh * 16, (cuuint64_t)n * nh * 16, (cuuint64_t)ctx->acc_stride * 16};
+    const cuuint32_t abox[4] = {2 * kFzCols, 1, L / 8, 1};
+    AXG_TRY(axg_encode_tmap(ctx, &mc, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, ctx->acc, adims, astr, abox));
+  }
+  AXG_TRY((launch_persistent<L>(ctx, "fft_f32_y", k_cols_tma<L, false>, batch * n * nkb, zs_smem<L>(), my, nkb,
+                                batch * n * nkb, tw, ctx->d_err)));
+  return launch_persistent<L>(ctx, name, k_z_sink<L, Sink>, n * nkb, zs_smem<L>() + sink_smem, mz, mc, nkb, n * nkb,
+                              tw, args, ctx->d_err);
+}
+
+template <int L>
+int uij_power_t(axg_ctx *ctx, const float *u, const float *ud, const float *cu, double tau, float2 *F, double dwav,
+                const int16_t *tab, int nb, double *numer, double *denom, const float4 *tw) {
   constexpr int n = L, M = L / 2;
   const int sp = axg_f32_spec_pitch(n);
   constexpr size_t smem = rows_f32_smem<M>(12);
   AXG_TRY(allow_smem(ctx, k_uij_rows<M>, smem));
   AXG_LAUNCH(ctx, "uij_rows_fp32", k_uij_rows<M>, (unsigned)((int64_t)n * n), 12 * M / 8, smem, u, ud, cu,
-             (int64_t)n * n * n, tau, out, sp, tw);
-  return f_cols_t<L>(ctx, out, 12, sp, tw);
+             (int64_t)n * n * n, (float)tau, (float)(tau - (double)(float)tau), F, sp, tw);
+  const double q2 = dwav * dwav;
+  const typename UijSink<L>::Args args = {tab,  nb,   bin_copies(nb), (float)q2, (float)(q2 - (double)(float)q2),
+                                          numer, denom};
+  return f_cols_sink<L, UijSink<L>>(ctx, "uij_z_bin_fp32", F, tw, args, bin_smem(nb));
 }
 
 template <int L>
@@ -916,16 +1373,33 @@ int ff_uij_d2z_t(axg_ctx *ctx, const double *u, const double *ud, double tau, do
   return d2z_cols_t<L>(ctx, f, 12, tw, false);
 }
 
+// Up to 64^3 a step is its kernels' latencies: an item's chain of fourteen tiles
+// in the sink takes 9 us there, storing the transforms and accumulating from
+// them 5 (Green step at 64^3 33 and 27 us); at 128^3 41 + 3 and 62.
+constexpr int kGreenUnfused = 64;
+
 template <int L>
-int gws_r2c_t(axg_ctx *ctx, const float2 *phi, float2 *out, float scale, const float4 *tw) {
+int gws_accumulate_t(axg_ctx *ctx, const float2 *phi, float2 *srcF, float scale, double phase1, float dw,
+                     float dwl, int ref_compat, const float4 *tw) {
   constexpr int n = L, M = L / 2;
   const int64_t rows = (int64_t)n * n;
-  const int sp = axg_f32_spec_pitch(n);
   constexpr size_t smem = rows_f32_smem<M>(6 * kSrcRows);
   AXG_TRY(allow_smem(ctx, k_gws_rows<M>, smem));
   AXG_LAUNCH(ctx, "gw_source_rows_fp32", k_gws_rows<M>, (unsigned)(rows / kSrcRows), 6 * kSrcRows * M / 8, smem,
-             phi, scale, out, sp, tw);
-  return f_cols_t<L>(ctx, out, 6, sp, tw);
+             phi, scale, srcF, axg_f32_spec_pitch(n), tw);
+  if constexpr (L <= kGreenUnfused) {
+    constexpr int items = 6 * n * ((n / 2 + kFzCols) / kFzCols), nkb = (n / 2 + kFzCols) / kFzCols;
+    CUtensorMap my, mz;
+    AXG_TRY(spec_tmaps<L>(ctx, srcF, 6, &my, &mz));
+    AXG_TRY((launch_persistent<L>(ctx, "fft_f32_y", k_cols_tma<L, false>, items, zs_smem<L>(), my, nkb, items, tw,
+                                  ctx->d_err)));
+    return launch_persistent<L>(ctx, "fft_f32_z", k_cols_tma<L, true>, items, zs_smem<L>(), mz, nkb, items, tw,
+                                ctx->d_err);
+  } else {
+    const float th = (float)phase1;
+    const typename GreenSink<L>::Args args = {srcF, ref_compat, th, (float)(phase1 - (double)th), dw, dwl};
+    return f_cols_sink<L, GreenSink<L>>(ctx, "gw_z_accumulate_fp32", srcF, tw, args, 0);
+  }
 }
 
 }  // namespace
@@ -1019,17 +1493,20 @@ int axg_ff_d2z_window(axg_ctx *ctx, const int8_t *flags, double dv, double2 *out
   return d2z_n(ctx, LoadWindow{flags, hi, (float)(dv - (double)hi)}, out, n, 1, true);
 }
 
-int axg_gw_source_r2c_f32(axg_ctx *ctx, const float2 *phi, float2 *out, int n, float scale) {
+bool axg_gw_fused_f32(int n) { return axg_ff_fft_supported(n) && n > kGreenUnfused; }
+
+int axg_gw_source_accumulate_f32(axg_ctx *ctx, const float2 *phi, float2 *srcF, int n, float scale, double phase1,
+                                 float dw, float dwl, int ref_compat) {
   if (!axg_ff_fft_supported(n)) return axg_set_error(ctx, AXG_ERR_UNSUPPORTED, "FP32 source transform size");
   AXG_TRY(ensure_twiddles(ctx, n));
   const float4 *tw = reinterpret_cast<const float4 *>(ctx->ff_tw);
   switch (n) {
-    case 16: return gws_r2c_t<16>(ctx, phi, out, scale, tw);
-    case 32: return gws_r2c_t<32>(ctx, phi, out, scale, tw);
-    case 64: return gws_r2c_t<64>(ctx, phi, out, scale, tw);
-    case 128: return gws_r2c_t<128>(ctx, phi, out, scale, tw);
-    case 256: return gws_r2c_t<256>(ctx, phi, out, scale, tw);
-    case 512: return gws_r2c_t<512>(ctx, phi, out, scale, tw);
+    case 16: return gws_accumulate_t<16>(ctx, phi, srcF, scale, phase1, dw, dwl, ref_compat, tw);
+    case 32: return gws_accumulate_t<32>(ctx, phi, srcF, scale, phase1, dw, dwl, ref_compat, tw);
+    case 64: return gws_accumulate_t<64>(ctx, phi, srcF, scale, phase1, dw, dwl, ref_compat, tw);
+    case 128: return gws_accumulate_t<128>(ctx, phi, srcF, scale, phase1, dw, dwl, ref_compat, tw);
+    case 256: return gws_accumulate_t<256>(ctx, phi, srcF, scale, phase1, dw, dwl, ref_compat, tw);
+    case 512: return gws_accumulate_t<512>(ctx, phi, srcF, scale, phase1, dw, dwl, ref_compat, tw);
     default: return axg_set_error(ctx, AXG_ERR_UNSUPPORTED, "FP32 source transform size");
   }
 }
@@ -1050,17 +1527,18 @@ int axg_gw_source_d2z_ff(axg_ctx *ctx, const double2 *phi, double d, double inv_
   }
 }
 
-int axg_uij_r2c_f32(axg_ctx *ctx, const float *u, const float *ud, const float *cu, float tau, float2 *out, int n) {
+int axg_uij_power_f32(axg_ctx *ctx, const float *u, const float *ud, const float *cu, double tau, float2 *F, int n,
+                      double dwav, const int16_t *tab, int nb, double *numer, double *denom) {
   if (!axg_ff_fft_supported(n)) return axg_set_error(ctx, AXG_ERR_UNSUPPORTED, "FP32 u_ij transform size");
   AXG_TRY(ensure_twiddles(ctx, n));
   const float4 *tw = reinterpret_cast<const float4 *>(ctx->ff_tw);
   switch (n) {
-    case 16: return uij_r2c_t<16>(ctx, u, ud, cu, tau, out, tw);
-    case 32: return uij_r2c_t<32>(ctx, u, ud, cu, tau, out, tw);
-    case 64: return uij_r2c_t<64>(ctx, u, ud, cu, tau, out, tw);
-    case 128: return uij_r2c_t<128>(ctx, u, ud, cu, tau, out, tw);
-    case 256: return uij_r2c_t<256>(ctx, u, ud, cu, tau, out, tw);
-    case 512: return uij_r2c_t<512>(ctx, u, ud, cu, tau, out, tw);
+    case 16: return uij_power_t<16>(ctx, u, ud, cu, tau, F, dwav, tab, nb, numer, denom, tw);
+    case 32: return uij_power_t<32>(ctx, u, ud, cu, tau, F, dwav, tab, nb, numer, denom, tw);
+    case 64: return uij_power_t<64>(ctx, u, ud, cu, tau, F, dwav, tab, nb, numer, denom, tw);
+    case 128: return uij_power_t<128>(ctx, u, ud, cu, tau, F, dwav, tab, nb, numer, denom, tw);
+    case 256: return uij_power_t<256>(ctx, u, ud, cu, tau, F, dwav, tab, nb, numer, denom, tw);
+    case 512: return uij_power_t<512>(ctx, u, ud, cu, tau, F, dwav, tab, nb, numer, denom, tw);
     default: return axg_set_error(ctx, AXG_ERR_UNSUPPORTED, "FP32 u_ij transform size");
   }
 }

@@ -17,8 +17,9 @@
 //                    cross-wired (2,1)/(1,2) updates through their closed form
 //                    over the six components.  FP64 for the FP64 paths; the
 //                    FP32-mixed path contracts in FP32 (sources, transforms,
-//                    polarisation, sin/cos of the FP64-reduced phase) and
-//                    accumulates in FP64.
+//                    polarisation, sin/cos of the float-float phase) and
+//                    accumulates in float-float, inside the z pass of its own
+//                    transforms (axg_fft_ff.cu, k_z_sink) above 64^3.
 // Spectra: shell histograms in FP64 (grav_waves.f90:257-321), 25 linear bins
 // or log bins; the u_ij path (AXG_GW_UIJ) FFTs w = tau u and w' = u + tau u'
 // (R2C, FP32 for the FP32-mixed path), TT-projects per k and accumulates
@@ -31,6 +32,7 @@
 #include "axg_binning.h"
 #include "axg_detmath.h"
 #include "axg_ff.h"
+#include "axg_gw_site.h"
 #include "axg_gw_source.h"
 #include "axg_internal.h"
 
@@ -40,8 +42,6 @@ constexpr double kRefPi = 3.14159265359;
 constexpr double kRefTwoPi = 2 * kRefPi;
 // potential.f90:13-23
 constexpr double kBigHInMstar = 2.1332e-42 / 2.435e18;
-
-__device__ __forceinline__ int kint(int j, int n) { return (j + n / 2) % n - n / 2; }
 
 // FP64 sources in the reference's operation order (gw_sources_fp64)
 __global__ void k_gw_source(const double2 *__restrict__ phi, int n, double d, double inv_d, int d_pow2,
@@ -162,53 +162,6 @@ __global__ void k_gw_source_degrade_f32(const float2 *__restrict__ phi, int n, i
 #pragma unroll
       for (int j = 0; j <= i; ++j, ++k) src[k * m3 + c] = scale * (xr[i] * xr[j] + xi[i] * xi[j]);
   }
-}
-
-// |k| dwav per stored half-spectrum entry as a float-float pair, the phase
-// rate of the FP32 Green accumulation
-__global__ void k_gw_omega(int n, double dwav, float2 *__restrict__ om) {
-  const int nh = n / 2 + 1;
-  const int64_t nhalf = (int64_t)n * n * nh;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; h < nhalf; h += stride) {
-    const double kx = kint((int)(h % nh), n), ky = kint((int)((h / nh) % n), n), kz = kint((int)(h / ((int64_t)nh * n)), n);
-    const double w = sqrt(kx * kx + ky * ky + kz * kz) * dwav;
-    const float hi = (float)w;
-    om[h] = make_float2(hi, (float)(w - (double)hi));
-  }
-}
-
-// get_comwav_grav (grav_waves.f90:157-191): p = (qz c - i s, qz s + i c, -r)
-// for the unit vector q of k, (c, s) its azimuth; e+_ij = p_i p_j, halved on
-// the diagonal, in the component order (1,1),(2,1),(2,2),(3,1),(3,2),(3,3).
-// Divisions are reciprocal multiplies (one rounding more than the reference).
-template <typename R>
-__device__ __forceinline__ bool gw_polarisation(R kx, R ky, R kz, R qq, R pr[6], R pi[6]) {
-  if (!(qq > 0)) return false;
-  const R iq = R(1) / qq;
-  const R qx = kx * iq, qy = ky * iq, qz = kz * iq;
-  const R r = sqrt(qx * qx + qy * qy);
-  R c = 1, sn = 0;
-  if (r > 0) {
-    const R ir = R(1) / r;
-    c = qx * ir;
-    sn = qy * ir;
-  }
-  const R ar[3] = {qz * c, qz * sn, -r}, ai[3] = {-sn, c, 0};
-  int comp = 0;
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j <= i; ++j, ++comp) {
-      R er = ar[i] * ar[j] - ai[i] * ai[j], ei = ar[i] * ai[j] + ai[i] * ar[j];
-      if (i == j) {
-        er *= R(0.5);
-        ei *= R(0.5);
-      }
-      pr[comp] = er;
-      pi[comp] = ei;
-    }
-  return true;
 }
 
 // X+ = sum e+ S, X- = sum conj(e+) S and the last component's conj(e+) S
@@ -543,73 +496,36 @@ __global__ void __launch_bounds__(256, 3) k_gw_accumulate_tab(const SRC *__restr
   }
 }
 
-// (hi, lo) += x: TwoSum of hi and x, the error folded into lo, then
-// renormalised (Fast2Sum); hi + lo carries about 48 significant bits
-__device__ __forceinline__ void ff_add(float &hi, float &lo, float x) {
-  const float s = hi + x;
-  const float bb = s - hi;
-  const float err = (hi - (s - bb)) + (x - bb);
-  const float l = lo + err;
-  hi = s + l;
-  lo = l - (hi - s);
-}
-
-// 2 pi = kC1 + kC2 + kC3 with kC1, kC2 of 8 significant bits (Cody-Waite), so
-// m kC1 and m kC2 are exact for |m| < 2^16, i.e. phases below 4e5 rad
-constexpr float kC1 = 6.28125f;
-constexpr float kC2 = 0.0019378662109375f;
-constexpr float kC3 = -2.559031372584286e-06f;
-constexpr float kInv2Pi = 0.15915493667125702f;
-
-// |k| dk tau reduced to about [-pi, pi] (absolute error ~3e-7): the product
-// of the float-float omega and tau keeps its rounding error exactly (fmaf)
-__device__ __forceinline__ float gw_phase(float2 om, float th, float tl) {
-  const float ph = om.x * th;
-  const float pl = fmaf(om.x, th, -ph) + fmaf(om.x, tl, om.y * th);
-  const float m = rintf(ph * kInv2Pi);
-  float r = fmaf(-m, kC1, ph);
-  r = fmaf(-m, kC2, r);
-  r = r + pl;
-  return fmaf(-m, kC3, r);
-}
-
-// float-float accumulators at site s from FP32 X+, X- and the weights
 __device__ __forceinline__ void f32_update(float4 *__restrict__ acc, int64_t astride, int64_t s, float wc, float ws,
                                            const float xp[2], const float xm[2], const float lm[2], int ref_compat) {
-  float4 a11 = acc[s], a21 = acc[astride + s], a12 = acc[2 * astride + s], a22 = acc[3 * astride + s];
-  ff_add(a11.x, a11.y, wc * xp[0]);
-  ff_add(a11.z, a11.w, wc * xp[1]);
-  ff_add(a22.x, a22.y, ws * xm[0]);
-  ff_add(a22.z, a22.w, ws * xm[1]);
-  if (ref_compat) {
-    ff_add(a12.x, a12.y, fmaf(wc, xm[0], ws * xp[0]));
-    ff_add(a12.z, a12.w, fmaf(wc, xm[1], ws * xp[1]));
-    a21 = a12;
-    ff_add(a21.x, a21.y, -wc * lm[0]);
-    ff_add(a21.z, a21.w, -wc * lm[1]);
-  } else {
-    ff_add(a21.x, a21.y, ws * xp[0]);
-    ff_add(a21.z, a21.w, ws * xp[1]);
-    ff_add(a12.x, a12.y, wc * xm[0]);
-    ff_add(a12.z, a12.w, wc * xm[1]);
-  }
-  acc[s] = a11;
-  acc[astride + s] = a21;
-  acc[2 * astride + s] = a12;
-  acc[3 * astride + s] = a22;
+  F32Acc a;
+  a.load(acc, astride, s, ref_compat);
+  a.update(wc, ws, xp, xm, lm, ref_compat);
+  a.store(acc, astride, s);
+}
+
+// the entry of its own of the mirror of (hx, hy, hz), hy or hz = n/2
+__device__ __forceinline__ void f32_mirror(const float2 *__restrict__ srcF, int64_t nspec, int64_t hs, int hx, int hy,
+                                           int hz, int n, float wc, float ws, int ref_compat, int64_t astride,
+                                           float4 *__restrict__ acc) {
+  const int jx = n - hx, jy = hy == 0 ? 0 : n - hy, jz = hz == 0 ? 0 : n - hz;
+  const float jkx = (float)kint(jx, n), jky = (float)kint(jy, n), jkz = (float)kint(jz, n);
+  float pr[6], pi[6], xp[2], xm[2], lm[2];
+  gw_polarisation<float>(jkx, jky, jkz, sqrtf(jkx * jkx + jky * jky + jkz * jkz), pr, pi);
+  gw_contract<float, float2>(srcF, nspec, hs, false, pr, pi, xp, xm, lm);
+  f32_update(acc, astride, (int64_t)n * n * (n / 2 + 1) + gw_nyq_extra(hx, hy, hz, n), wc, ws, xp, xm, lm, ref_compat);
 }
 
 // FP32-mixed Green accumulation: FP32 sources, polarisation, phase and
 // contraction; the accumulators are float-float pairs (re hi, re lo, im hi,
 // im lo), so no FP64 instruction is issued per k-site.  One thread per stored
 // half-spectrum entry; the accumulators hold that half spectrum and the
-// Nyquist-row mirrors, as in k_gw_accumulate_tab.  The source spectra have
-// kx rows of sp entries (the own transforms pad them), the accumulators and
-// phase rates rows of n/2 + 1.
-__global__ void __launch_bounds__(256, 4) k_gw_accumulate_f32(const float2 *__restrict__ srcF, int sp,
-                                                              const float2 *__restrict__ om, int n, float th,
-                                                              float tl, float dw, int ref_compat, int64_t astride,
-                                                              float4 *__restrict__ acc) {
+// Nyquist-row mirrors, as in k_gw_accumulate_tab.  For the cuFFT transforms and
+// the own ones up to 64^3; above, those accumulate inside their z pass
+// (k_z_sink<GreenSink>).  The source spectra have kx rows of sp entries.
+__global__ void __launch_bounds__(256, 4) k_gw_accumulate_f32(const float2 *__restrict__ srcF, int sp, int n, float Th,
+                                                              float Tl, float dw, float dwl, int ref_compat,
+                                                              int64_t astride, float4 *__restrict__ acc) {
   const int nh = n / 2 + 1;
   const int64_t nhalf = (int64_t)n * n * nh, nspec = (int64_t)n * n * sp;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -617,25 +533,38 @@ __global__ void __launch_bounds__(256, 4) k_gw_accumulate_f32(const float2 *__re
     const int hx = (int)(h % nh), hy = (int)((h / nh) % n), hz = (int)(h / ((int64_t)nh * n));
     const int64_t hs = (h / nh) * sp + hx;  // the entry in the source spectra
     const float kx = (float)kint(hx, n), ky = (float)kint(hy, n), kz = (float)kint(hz, n);
-    const float qq = sqrtf(kx * kx + ky * ky + kz * kz);
+    const float k2 = kx * kx + ky * ky + kz * kz, qq = sqrtf(k2);
     float pr[6], pi[6];
     if (!gw_polarisation<float>(kx, ky, kz, qq, pr, pi)) {
       if (ref_compat) acc[astride + h] = acc[2 * astride + h];  // k = 0 (h = 0)
       continue;
     }
     float sq, cq;
-    sincosf(gw_phase(om[h], th, tl), &sq, &cq);
-    const float wc = dw * cq, ws = dw * sq;
+    gw_cos_sin(k2, 1.f / qq, Th, Tl, &cq, &sq);
+    const float wc = fmaf(dwl, cq, dw * cq), ws = fmaf(dwl, sq, dw * sq);
     float xp[2], xm[2], lm[2];
     gw_contract<float, float2>(srcF, nspec, hs, true, pr, pi, xp, xm, lm);
     f32_update(acc, astride, h, wc, ws, xp, xm, lm, ref_compat);
-    if (hx > 0 && hx < n / 2 && (hy == n / 2 || hz == n / 2)) {
-      const int jx = n - hx, jy = hy == 0 ? 0 : n - hy, jz = hz == 0 ? 0 : n - hz;
-      const float jkx = (float)kint(jx, n), jky = (float)kint(jy, n), jkz = (float)kint(jz, n);
-      gw_polarisation<float>(jkx, jky, jkz, sqrtf(jkx * jkx + jky * jky + jkz * jkz), pr, pi);
-      gw_contract<float, float2>(srcF, nspec, hs, false, pr, pi, xp, xm, lm);
-      f32_update(acc, astride, nhalf + gw_nyq_extra(hx, hy, hz, n), wc, ws, xp, xm, lm, ref_compat);
-    }
+    if (hx > 0 && hx < n / 2 && (hy == n / 2 || hz == n / 2))
+      f32_mirror(srcF, nspec, hs, hx, hy, hz, n, wc, ws, ref_compat, astride, acc);
+  }
+}
+
+// The Nyquist-row mirrors alone, after k_z_sink<GreenSink>, which leaves the
+// transforms of the rows hy = n/2 and hz = n/2 in srcF (kx rows of sp entries).
+__global__ void k_gw_accumulate_f32_mirrors(const float2 *__restrict__ srcF, int sp, int n, float Th, float Tl,
+                                            float dw, float dwl, int ref_compat, int64_t astride,
+                                            float4 *__restrict__ acc) {
+  const int per = 2 * n - 1, total = (n / 2 - 1) * per;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
+    const int m = e / (n / 2 - 1), hx = 1 + e % (n / 2 - 1);
+    const int hy = m < n ? n / 2 : (m - n < n / 2 ? m - n : m - n + 1), hz = m < n ? m : n / 2;
+    const int ky = kint(hy, n), kz = kint(hz, n);
+    const float k2 = (float)(hx * hx + ky * ky + kz * kz);
+    float sq, cq;
+    gw_cos_sin(k2, gw_rsqrt(k2), Th, Tl, &cq, &sq);
+    f32_mirror(srcF, (int64_t)n * n * sp, ((int64_t)hz * n + hy) * sp + hx, hx, hy, hz, n, fmaf(dwl, cq, dw * cq),
+               fmaf(dwl, sq, dw * sq), ref_compat, astride, acc);
   }
 }
 
@@ -672,7 +601,7 @@ template <typename A>
 __global__ void __launch_bounds__(256) k_gw_bin_green(const A *__restrict__ acc, int n, int64_t astride, int rows,
                                                       const int16_t *__restrict__ tab, int nb, int copies,
                                                       double *__restrict__ numer, double *__restrict__ denom) {
-  BlockBins bins(nb, copies);
+  BlockBins bins(bins_mem(), nb, copies);
   const int nh = n / 2 + 1;
   const int64_t nhalf = (int64_t)n * n * nh;
   BinRun<decltype(acc_norm2(acc, astride, 0))> run;
@@ -699,52 +628,20 @@ __global__ void k_uij_prepare(const R *__restrict__ u, const R *__restrict__ ud,
                               int64_t n3, double tau, int f, R *__restrict__ w) {
   const int c = f < 6 ? f : f - 6;
   const R *uc = u + c * n3, *udc = ud + c * n3, *cuc = cu ? cu + c * n3 : nullptr;
-  const R t = (R)tau;
+  const R t = (R)tau, tl = (R)(tau - (double)t);  // what R drops of tau, common to all sites
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n3; s += stride) {
     // in the precision of the spectrum: FP32 for FP32-mixed (the Kahan
     // compensation is below FP32 resolution of u; it is applied all the same)
     R uv = uc[s];
     if (cuc) uv -= cuc[s];
-    w[s] = f < 6 ? t * uv : uv + t * udc[s];
+    const R x = f < 6 ? uv : udc[s];
+    R v = f < 6 ? t * uv : uv + t * x;
+    if constexpr (sizeof(R) == 4) v = fmaf(tl, x, v);
+    w[s] = v;
   }
 }
 
-// The TT part of a symmetric tensor spectrum U (components 11, 21, 22, 31, 32,
-// 33) in the basis (m, l) normal to k: m = (-s, c, 0) with (c, s) the azimuth
-// of k, l = k x m / |k|.  |Lambda U|^2 = |U_mm - U_ll|^2 / 2 + 2 |U_ml|^2 with
-// U_mm - U_ll = sum a_c U_c and |k| U_ml = sum b_c U_c; a and b are rational
-// in the integers k:
-//   a_11 = s^2 - q^2 c^2,  a_21 = -2 s c (1 + q^2),  a_22 = c^2 - q^2 s^2,
-//   a_31 = 2 kz kx / k^2,  a_32 = 2 kz ky / k^2,     a_33 = -(a_11 + a_22),
-//   b_11 = kz s c,  b_21 = kz (s^2 - c^2),  b_22 = -b_11,  b_31 = -ky,  b_32 = kx
-// with c^2 = kx^2 / p^2, s^2 = ky^2 / p^2, s c = kx ky / p^2, q = kz / k.
-// a_33 that way, the trace drops out of the differences U_11 - U_33 and
-// U_22 - U_33 exactly.  20 multiply-adds a tensor where P U P - P tr(P U) / 2,
-// P = 1 - k k, and its squared norm took ~200 operations.
-template <typename R>
-struct TTBasis {
-  R a11, a21, a22, a31, a32, b11, b21, b31, b32, ik2;
-};
-template <typename R>
-__device__ __forceinline__ TTBasis<R> tt_basis(int kx, int ky, int kz, int k2) {
-  const int p2 = kx * kx + ky * ky;
-  const R ik2 = R(1) / (R)k2, ip2 = p2 ? R(1) / (R)p2 : R(0);
-  const R cc = p2 ? (R)(kx * kx) * ip2 : R(1), ss = (R)(ky * ky) * ip2, sc = (R)(kx * ky) * ip2;
-  const R qq = (R)(kz * kz) * ik2;
-  TTBasis<R> t;
-  t.a11 = ss - qq * cc;
-  t.a21 = R(-2) * sc * (R(1) + qq);
-  t.a22 = cc - qq * ss;
-  t.a31 = (R)(2 * kz * kx) * ik2;
-  t.a32 = (R)(2 * kz * ky) * ik2;
-  t.b11 = (R)kz * sc;
-  t.b21 = (R)kz * (ss - cc);
-  t.b31 = (R)-ky;
-  t.b32 = (R)kx;
-  t.ik2 = ik2;
-  return t;
-}
 template <typename R, typename CV>
 __device__ __forceinline__ R tt_power(const TTBasis<R> &t, const CV *__restrict__ F, int64_t stride, int64_t h) {
   const CV u11 = F[h], u21 = F[stride + h], u22 = F[2 * stride + h], u31 = F[3 * stride + h], u32 = F[4 * stride + h],
@@ -760,29 +657,31 @@ __device__ __forceinline__ R tt_power(const TTBasis<R> &t, const CV *__restrict_
   return R(0.5) * (pr * pr + pi * pi) + R(2) * t.ik2 * (xr * xr + xi * xi);
 }
 
-// F: the twelve half spectra, kx rows of sp entries.  The TT power in the
+// F: the twelve half spectra.  The TT power in the
 // precision of the spectrum (FP32 for FP32-mixed), the shell sums in FP64;
-// numer comes without its factor dv^2.  512^3 FP32 1.44 -> 0.83 ms (96 B an
-// entry: the copy peak allows 0.96 for what misses the L2); 256^3 FP64, bound
-// by the FP64 pipe, 4.41 -> 1.15.
+// numer comes without its factor dv^2.  256^3 FP64, bound by the FP64 pipe, 4.41
+// -> 1.15 ms.  The FP32 spectra of the own transforms are summed inside their z
+// pass (k_z_sink<UijSink>).
 template <typename CV>
-__global__ void __launch_bounds__(256) k_uij_bin(const CV *__restrict__ F, int sp, int n, int rows, double dwav,
+__global__ void __launch_bounds__(256) k_uij_bin(const CV *__restrict__ F, int n, int rows, double dwav,
                                                  const int16_t *__restrict__ tab, int nb, int copies,
                                                  double *__restrict__ numer, double *__restrict__ denom) {
   using R = decltype(F[0].x);
-  BlockBins bins(nb, copies);
+  BlockBins bins(bins_mem(), nb, copies);
   const int nh = n / 2 + 1;
-  const int64_t nspec = (int64_t)n * n * sp;
-  const R dwav2 = (R)(dwav * dwav);
+  const int64_t nspec = (int64_t)n * n * nh;
+  const R dwav2 = (R)(dwav * dwav), dwavl = (R)(dwav * dwav - (double)dwav2);
   BinRun<double> run;
   walk_spectrum(n, nh, rows, [&](int ix, int iy, int iz) {
     const int kx = kint(ix, n), ky = kint(iy, n), kz = kint(iz, n), k2 = kx * kx + ky * ky + kz * kz;
     const int b = tab[k2];
     if (b < 0) return;
-    const int64_t h = ((int64_t)iz * n + iy) * sp + ix;
+    const int64_t h = ((int64_t)iz * n + iy) * nh + ix;
     const TTBasis<R> t = tt_basis<R>(kx, ky, kz, k2);
     const unsigned wgt = (ix == 0 || 2 * ix == n) ? 1u : 2u;  // Hermitian partner of the half spectrum
-    const R e = tt_power(t, F + 6 * nspec, nspec, h) + (R)k2 * dwav2 * tt_power(t, F, nspec, h);
+    R q2 = (R)k2 * dwav2;
+    if constexpr (sizeof(R) == 4) q2 = fmaf((R)k2, dwavl, q2);
+    const R e = tt_power(t, F + 6 * nspec, nspec, h) + q2 * tt_power(t, F, nspec, h);
     run.add(bins, b, (double)((R)wgt * e), wgt);
   });
   run.flush(bins);
@@ -863,10 +762,7 @@ int axg_gw_init(axg_ctx *ctx) {
     AXG_CUDA_TRY(ctx, cudaMemsetAsync(ctx->gsrcF, 0, bytes, ctx->stream));  // the padding columns
   }
   AXG_CUDA_TRY(ctx, cudaMemsetAsync(ctx->acc, 0, (size_t)ctx->acc_stride * 64, ctx->stream));
-  if (fp32) {
-    AXG_TRY(axg_alloc(ctx, (void **)&ctx->gw_omega, (size_t)nhalf * 8, "GW phase rates"));
-    AXG_LAUNCH(ctx, "gw_omega", k_gw_omega, grid_for(nhalf), 256, 0, n, kRefTwoPi / ctx->gw_dspa / n, ctx->gw_omega);
-  } else {
+  if (!fp32) {
     // The FP64 polarisation table (13 doubles per half-spectrum k) when it
     // takes at most an eighth of the device memory (512^3: 7 GB); otherwise
     // the accumulation forms the polarisation per step.
@@ -910,24 +806,37 @@ int axg_gw_integration(axg_ctx *ctx, double tau, double dtau) {
   const int ref = ctx->p.compat == AXG_COMPAT_REF ? 1 : 0;
   const int64_t nhalf = (int64_t)n * n * (n / 2 + 1);
   if (ctx->p.precision == AXG_PREC_FP32_MIXED) {
+    const double phase1 = dwav * tau / (3.14159265358979323846 / 2);  // of |k| = 1, in quarter turns
+    const float th = (float)phase1, tl = (float)(phase1 - (double)th);
+    // the sources' factor 2 / d^2: its power of two in them, the rest in the
+    // weight, which keeps what a float of it drops (an error common to all k)
+    int e2;
+    const double dws = dw * std::frexp(2.0 / (d * d), &e2);
+    const float scale = std::ldexp(1.f, e2), wh = (float)dws, wl = (float)(dws - (double)wh);
     if (deg > 1) {
       float *src = (float *)ctx->gsrc;
       AXG_LAUNCH(ctx, "gw_source_degrade_fp32", k_gw_source_degrade_f32, grid_for(n3), 256, 0,
-                 (const float2 *)ctx->phi[ctx->cur], nl, deg, (float)(2.0 / (d * d)), src);
+                 (const float2 *)ctx->phi[ctx->cur], nl, deg, scale, src);
       AXG_CUFFT_TRY(ctx, cufftExecR2C(ctx->plan_gsrc, src, (cufftComplex *)ctx->gsrcF));
     } else if (ctx->gw_own_fft) {
-      AXG_TRY(axg_gw_source_r2c_f32(ctx, (const float2 *)ctx->phi[ctx->cur], (float2 *)ctx->gsrcF, n,
-                                    (float)(2.0 / (d * d))));
+      AXG_TRY(axg_gw_source_accumulate_f32(ctx, (const float2 *)ctx->phi[ctx->cur], (float2 *)ctx->gsrcF, n,
+                                           scale, phase1, wh, wl, ref));
+      if (axg_gw_fused_f32(n)) {
+        const int mirrors = (n / 2 - 1) * (2 * n - 1);
+        AXG_LAUNCH(ctx, "gw_accumulate_mirrors", k_gw_accumulate_f32_mirrors, grid_for(mirrors), 256, 0,
+                   (const float2 *)ctx->gsrcF, ctx->gsrc_pitch, n, th, tl, wh, wl, ref, ctx->acc_stride,
+                   (float4 *)ctx->acc);
+        return AXG_OK;
+      }
     } else {
       float *src = (float *)ctx->gsrc;
       AXG_LAUNCH(ctx, "gw_source_fp32", k_gw_source_f32, grid_for(n3), 256, 0,
-                 (const float2 *)ctx->phi[ctx->cur], n, (float)(2.0 / (d * d)), src);
+                 (const float2 *)ctx->phi[ctx->cur], n, scale, src);
       AXG_CUFFT_TRY(ctx, cufftExecR2C(ctx->plan_gsrc, src, (cufftComplex *)ctx->gsrcF));
     }
-    const float th = (float)tau, tl = (float)(tau - (double)th);
     AXG_LAUNCH(ctx, "gw_accumulate_fp32", k_gw_accumulate_f32, grid_for(nhalf), 256, 0,
-               (const float2 *)ctx->gsrcF, ctx->gsrc_pitch, ctx->gw_omega, n, th, tl, (float)dw, ref,
-               ctx->acc_stride, (float4 *)ctx->acc);
+               (const float2 *)ctx->gsrcF, ctx->gsrc_pitch, n, th, tl, wh, wl, ref, ctx->acc_stride,
+               (float4 *)ctx->acc);
     return AXG_OK;
   }
   int ex;
@@ -1024,8 +933,8 @@ int axg_gw_spec(axg_ctx *ctx, double tau, int log_bins, double *wave, double *po
       float *w = (float *)ctx->ubuf;
       float2 *F = ctx->uij_own_fft ? (float2 *)ctx->ubuf : (float2 *)(w + ctx->n3);
       if (ctx->uij_own_fft) {
-        AXG_TRY(axg_uij_r2c_f32(ctx, (const float *)ctx->u[ctx->cur], (const float *)ctx->ud,
-                                (const float *)ctx->cu, (float)tau, F, n));
+        AXG_TRY(axg_uij_power_f32(ctx, (const float *)ctx->u[ctx->cur], (const float *)ctx->ud,
+                                  (const float *)ctx->cu, tau, F, n, dwav, tab, nb, d_num, d_den));
       } else {
         for (int f = 0; f < 12; ++f) {
           AXG_LAUNCH(ctx, "uij_prepare_fp32", k_uij_prepare<float>, grid_for(ctx->n3), 256, 0,
@@ -1033,9 +942,9 @@ int axg_gw_spec(axg_ctx *ctx, double tau, int log_bins, double *wave, double *po
                      f, w);
           AXG_CUFFT_TRY(ctx, cufftExecR2C(ctx->plan_u, w, (cufftComplex *)F + f * nhalf));
         }
+        AXG_LAUNCH(ctx, "uij_bin_fp32", k_uij_bin<float2>, bgrid, 256, bsm, F, n, brows, dwav, tab, nb, copies,
+                   d_num, d_den);
       }
-      AXG_LAUNCH(ctx, "uij_bin_fp32", k_uij_bin<float2>, bgrid, 256, bsm, F, ctx->u_pitch, n, brows, dwav, tab, nb,
-                 copies, d_num, d_den);
     } else {
       double *w = (double *)ctx->ubuf;
       double2 *F = ctx->uij_own_fft ? (double2 *)ctx->ubuf : (double2 *)(w + ctx->n3);
@@ -1049,8 +958,8 @@ int axg_gw_spec(axg_ctx *ctx, double tau, int log_bins, double *wave, double *po
           AXG_CUFFT_TRY(ctx, cufftExecD2Z(ctx->plan_u, w, (cufftDoubleComplex *)F + f * nhalf));
         }
       }
-      AXG_LAUNCH(ctx, "uij_bin_fp64", k_uij_bin<double2>, bgrid, 256, bsm, F, ctx->u_pitch, n, brows, dwav, tab, nb,
-                 copies, d_num, d_den);
+      AXG_LAUNCH(ctx, "uij_bin_fp64", k_uij_bin<double2>, bgrid, 256, bsm, F, n, brows, dwav, tab, nb, copies, d_num,
+                 d_den);
     }
   } else {
     return axg_set_error(ctx, AXG_ERR_STATE, "gw_mode is NONE");

@@ -96,7 +96,6 @@ struct axg_ctx {
   double2 *acc = nullptr;  // Green accumulators [4][n3]; FP32-mixed: float4 (re hi, re lo, im hi, im lo)  // [4][n3]
   double *gsrc = nullptr;  // [6][n3] real sources S_ij (float for FP32-mixed)
   double2 *gsrcF = nullptr;  // [6][n*n*(n/2+1)] (float2 for FP32-mixed)
-  float2 *gw_omega = nullptr;  // [n3] |k| dwav per k-site as float hi + lo (FP32-mixed Green mode)
   double *gw_pol = nullptr;    // FP64 Green mode: [12][n*n*(n/2+1)] float2 e+ (re, im as float-float), then
                                // [n*n*(n/2+1)] double |k| dwav; or null
   bool acc_ff = false;         // Green accumulators are float-float float4 (FP32-mixed, and the FP64 paths
@@ -297,16 +296,27 @@ __host__ __device__ inline int64_t gw_nyq_extra(int hx, int hy, int hz, int n) {
 // Row pitch (complex values) of the complex-float half spectra of the own
 // transforms: n/2 + 1 rounded up to a multiple of 4, so that every kx row
 // starts on a 32-byte sector and the rows' byte stride suits TMA (a multiple
-// of 16).  Columns n/2 + 1 .. pitch - 1 are padding that no consumer reads.
-inline int axg_f32_spec_pitch(int n) { return (n / 2 + 1 + 3) & ~3; }
-// the six FP32-mixed Green sources of phi and their forward transforms, out
-// [6][n][n][pitch] complex float (cuFFT's R2C values, rows of
-// axg_f32_spec_pitch(n)); n as axg_ff_fft_supported
-int axg_gw_source_r2c_f32(axg_ctx *ctx, const float2 *phi, float2 *out, int n, float scale);
-// the u_ij spectrum's twelve real fields (tau u_c, u_c + tau u'_c) and their
-// forward transforms, out [12][n][n][pitch] complex float (rows of
-// axg_f32_spec_pitch(n)); cu: the FP32 Kahan compensation of u, or null
-int axg_uij_r2c_f32(axg_ctx *ctx, const float *u, const float *ud, const float *cu, float tau, float2 *out, int n);
+// of 16); from n = 128, where the spectra leave the L2, to a multiple of 8, so
+// that the z pass's 64-byte tile rows are aligned (512^3 u_ij: the tiles alone
+// arrive at 6.0 TB/s, 4.5 with rows half a tile row off).  Columns n/2 + 1 ..
+// pitch - 1 are padding that no consumer reads.
+__host__ __device__ constexpr int axg_f32_spec_pitch(int n) {
+  return n >= 128 ? (n / 2 + 1 + 7) & ~7 : (n / 2 + 1 + 3) & ~3;
+}
+// one FP32-mixed Green step: the six sources of phi, their forward transforms
+// and the accumulation into ctx->acc with the weights (dw + dwl) cos, sin of the phase
+// |k| phase1, phase1 in quarter turns; srcF, [6][n][n][axg_f32_spec_pitch(n)], is the transforms' workspace
+// and holds the finished values at hy = n/2 and hz = n/2 for the mirrors.  Where
+// axg_gw_fused_f32 is false: the transforms alone, all of them finished.
+bool axg_gw_fused_f32(int n);
+int axg_gw_source_accumulate_f32(axg_ctx *ctx, const float2 *phi, float2 *srcF, int n, float scale, double phase1,
+                                 float dw, float dwl, int ref_compat);
+// the u_ij spectrum's twelve real fields (tau u_c, u_c + tau u'_c), their
+// forward transforms (in F, [12][n][n][axg_f32_spec_pitch(n)]) and the shell
+// sums of the TT power (without its factor dv^2); cu: the FP32 Kahan
+// compensation of u, or null; tab, nb: axg_bin_table
+int axg_uij_power_f32(axg_ctx *ctx, const float *u, const float *ud, const float *cu, double tau, float2 *F, int n,
+                      double dwav, const int16_t *tab, int nb, double *numer, double *denom);
 int axg_uij_d2z_ff(axg_ctx *ctx, const double *u, const double *ud, double tau, double2 *out, int n);
 // the six FP64 Green sources of phi (d = 2 dx; inv_d, d_pow2 as
 // gw_sources_fp64) and their float-float D2Z, out as axg_ff_d2z for batch 6

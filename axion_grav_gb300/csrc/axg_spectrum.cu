@@ -28,8 +28,6 @@ constexpr double kRefTwoPi = 2 * kRefPi;
 constexpr int kNumLargeq = 500;
 constexpr int kNumInt = 200;
 
-__device__ __forceinline__ int kint(int j, int n) { return (j + n / 2) % n - n / 2; }
-
 template <typename V>
 __global__ void k_spec_degrade(const V *__restrict__ phid, const int8_t *__restrict__ flags, int n, int deg,
                                double inv_deg3, int window, double dv_spa, double2 *__restrict__ out) {
@@ -72,7 +70,7 @@ template <typename V>
 __global__ void __launch_bounds__(256) k_spec_bin(const V *__restrict__ F, int m, int rows,
                                                   const int16_t *__restrict__ tab, int nb, int copies,
                                                   double *__restrict__ conv, double *__restrict__ count) {
-  BlockBins bins(nb, copies);
+  BlockBins bins(bins_mem(), nb, copies);
   BinRun<decltype(norm2(F[0]))> run;
   walk_spectrum(m, m, rows, [&](int ix, int iy, int iz) {
     const int kx = kint(ix, m), ky = kint(iy, m), kz = kint(iz, m);
