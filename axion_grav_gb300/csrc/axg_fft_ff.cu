@@ -681,15 +681,13 @@ __global__ void __launch_bounds__(6 * kSrcRows * M / 8) k_gws_rows(const float2 
   });
 }
 
-// The u_ij spectrum's twelve real fields, tau u_c and u_c + tau u'_c (tau with
-// taul, what a float of it drops; c =
+// The u_ij spectrum's twelve real fields, tau u_c and u_c + tau u'_c (c =
 // 11, 21, 22, 31, 32, 33; FP32-mixed subtracts the Kahan compensation from
 // u first), formed inside the row pass as the Green sources are: one CTA per
 // x-row, twelve lines.  Output [12][n][n][n/2+1] complex float.
 template <int M>
 __global__ void __launch_bounds__(12 * M / 8) k_uij_rows(const float *__restrict__ u, const float *__restrict__ ud,
                                                          const float *__restrict__ cu, int64_t n3, float tau,
-                                                         float taul,
                                                          float2 *__restrict__ out, int sp,
                                                          const float4 *__restrict__ twff) {
   constexpr int N = 2 * M, TH = M / 8, LP = rowline_pitch<M>();
@@ -708,9 +706,8 @@ __global__ void __launch_bounds__(12 * M / 8) k_uij_rows(const float *__restrict
       uv.y -= cv.y;
     }
     const float2 dv = *reinterpret_cast<const float2 *>(ud + x);
-    s[c * LP + fswz(m)] = make_float2(fmaf(taul, uv.x, tau * uv.x), fmaf(taul, uv.y, tau * uv.y));
-    s[(6 + c) * LP + fswz(m)] =
-        make_float2(fmaf(taul, dv.x, uv.x + tau * dv.x), fmaf(taul, dv.y, uv.y + tau * dv.y));
+    s[c * LP + fswz(m)] = make_float2(tau * uv.x, tau * uv.y);
+    s[(6 + c) * LP + fswz(m)] = make_float2(uv.x + tau * dv.x, uv.y + tau * dv.y);
   }
   __syncthreads();
   {
@@ -1084,7 +1081,7 @@ struct UijSink {
   struct Args {
     const int16_t *tab;
     int nb, copies;
-    float dwav2, dwavl;  // and what a float of it drops
+    float dwav2;
     double *numer, *denom;
   };
   __device__ __forceinline__ static int field(int f) {
@@ -1148,7 +1145,7 @@ struct UijSink {
           const float kz = z_wave<L>(jf, s), k2 = fmaf(kz, kz, p2), ik = gw_rsqrt(k2), i2 = ik * ik;
           const float px = A[s].x * i2, py = A[s].y * i2, cx = B[s].x * ik, cy = B[s].y * ik;
           const float p = 0.5f * (px * px + py * py) + 2.f * (cx * cx + cy * cy);
-          e[s] = f < 6 ? p : fmaf(fmaf(k2, a.dwavl, k2 * a.dwav2), p, e[s]);
+          e[s] = f < 6 ? p : fmaf(k2 * a.dwav2, p, e[s]);
         }
       }
     }
@@ -1350,17 +1347,15 @@ int f_cols_sink(axg_ctx *ctx, const char *name, float2 *F, const float4 *tw, con
 }
 
 template <int L>
-int uij_power_t(axg_ctx *ctx, const float *u, const float *ud, const float *cu, double tau, float2 *F, double dwav,
+int uij_power_t(axg_ctx *ctx, const float *u, const float *ud, const float *cu, float tau, float2 *F, double dwav,
                 const int16_t *tab, int nb, double *numer, double *denom, const float4 *tw) {
   constexpr int n = L, M = L / 2;
   const int sp = axg_f32_spec_pitch(n);
   constexpr size_t smem = rows_f32_smem<M>(12);
   AXG_TRY(allow_smem(ctx, k_uij_rows<M>, smem));
   AXG_LAUNCH(ctx, "uij_rows_fp32", k_uij_rows<M>, (unsigned)((int64_t)n * n), 12 * M / 8, smem, u, ud, cu,
-             (int64_t)n * n * n, (float)tau, (float)(tau - (double)(float)tau), F, sp, tw);
-  const double q2 = dwav * dwav;
-  const typename UijSink<L>::Args args = {tab,  nb,   bin_copies(nb), (float)q2, (float)(q2 - (double)(float)q2),
-                                          numer, denom};
+             (int64_t)n * n * n, tau, F, sp, tw);
+  const typename UijSink<L>::Args args = {tab, nb, bin_copies(nb), (float)(dwav * dwav), numer, denom};
   return f_cols_sink<L, UijSink<L>>(ctx, "uij_z_bin_fp32", F, tw, args, bin_smem(nb));
 }
 
@@ -1527,7 +1522,7 @@ int axg_gw_source_d2z_ff(axg_ctx *ctx, const double2 *phi, double d, double inv_
   }
 }
 
-int axg_uij_power_f32(axg_ctx *ctx, const float *u, const float *ud, const float *cu, double tau, float2 *F, int n,
+int axg_uij_power_f32(axg_ctx *ctx, const float *u, const float *ud, const float *cu, float tau, float2 *F, int n,
                       double dwav, const int16_t *tab, int nb, double *numer, double *denom) {
   if (!axg_ff_fft_supported(n)) return axg_set_error(ctx, AXG_ERR_UNSUPPORTED, "FP32 u_ij transform size");
   AXG_TRY(ensure_twiddles(ctx, n));

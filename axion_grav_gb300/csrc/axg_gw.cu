@@ -628,17 +628,14 @@ __global__ void k_uij_prepare(const R *__restrict__ u, const R *__restrict__ ud,
                               int64_t n3, double tau, int f, R *__restrict__ w) {
   const int c = f < 6 ? f : f - 6;
   const R *uc = u + c * n3, *udc = ud + c * n3, *cuc = cu ? cu + c * n3 : nullptr;
-  const R t = (R)tau, tl = (R)(tau - (double)t);  // what R drops of tau, common to all sites
+  const R t = (R)tau;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n3; s += stride) {
     // in the precision of the spectrum: FP32 for FP32-mixed (the Kahan
     // compensation is below FP32 resolution of u; it is applied all the same)
     R uv = uc[s];
     if (cuc) uv -= cuc[s];
-    const R x = f < 6 ? uv : udc[s];
-    R v = f < 6 ? t * uv : uv + t * x;
-    if constexpr (sizeof(R) == 4) v = fmaf(tl, x, v);
-    w[s] = v;
+    w[s] = f < 6 ? t * uv : uv + t * udc[s];
   }
 }
 
@@ -670,7 +667,7 @@ __global__ void __launch_bounds__(256) k_uij_bin(const CV *__restrict__ F, int n
   BlockBins bins(bins_mem(), nb, copies);
   const int nh = n / 2 + 1;
   const int64_t nspec = (int64_t)n * n * nh;
-  const R dwav2 = (R)(dwav * dwav), dwavl = (R)(dwav * dwav - (double)dwav2);
+  const R dwav2 = (R)(dwav * dwav);
   BinRun<double> run;
   walk_spectrum(n, nh, rows, [&](int ix, int iy, int iz) {
     const int kx = kint(ix, n), ky = kint(iy, n), kz = kint(iz, n), k2 = kx * kx + ky * ky + kz * kz;
@@ -679,9 +676,7 @@ __global__ void __launch_bounds__(256) k_uij_bin(const CV *__restrict__ F, int n
     const int64_t h = ((int64_t)iz * n + iy) * nh + ix;
     const TTBasis<R> t = tt_basis<R>(kx, ky, kz, k2);
     const unsigned wgt = (ix == 0 || 2 * ix == n) ? 1u : 2u;  // Hermitian partner of the half spectrum
-    R q2 = (R)k2 * dwav2;
-    if constexpr (sizeof(R) == 4) q2 = fmaf((R)k2, dwavl, q2);
-    const R e = tt_power(t, F + 6 * nspec, nspec, h) + q2 * tt_power(t, F, nspec, h);
+    const R e = tt_power(t, F + 6 * nspec, nspec, h) + (R)k2 * dwav2 * tt_power(t, F, nspec, h);
     run.add(bins, b, (double)((R)wgt * e), wgt);
   });
   run.flush(bins);
@@ -934,7 +929,7 @@ int axg_gw_spec(axg_ctx *ctx, double tau, int log_bins, double *wave, double *po
       float2 *F = ctx->uij_own_fft ? (float2 *)ctx->ubuf : (float2 *)(w + ctx->n3);
       if (ctx->uij_own_fft) {
         AXG_TRY(axg_uij_power_f32(ctx, (const float *)ctx->u[ctx->cur], (const float *)ctx->ud,
-                                  (const float *)ctx->cu, tau, F, n, dwav, tab, nb, d_num, d_den));
+                                  (const float *)ctx->cu, (float)tau, F, n, dwav, tab, nb, d_num, d_den));
       } else {
         for (int f = 0; f < 12; ++f) {
           AXG_LAUNCH(ctx, "uij_prepare_fp32", k_uij_prepare<float>, grid_for(ctx->n3), 256, 0,

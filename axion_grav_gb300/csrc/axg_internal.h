@@ -315,7 +315,7 @@ int axg_gw_source_accumulate_f32(axg_ctx *ctx, const float2 *phi, float2 *srcF, 
 // forward transforms (in F, [12][n][n][axg_f32_spec_pitch(n)]) and the shell
 // sums of the TT power (without its factor dv^2); cu: the FP32 Kahan
 // compensation of u, or null; tab, nb: axg_bin_table
-int axg_uij_power_f32(axg_ctx *ctx, const float *u, const float *ud, const float *cu, double tau, float2 *F, int n,
+int axg_uij_power_f32(axg_ctx *ctx, const float *u, const float *ud, const float *cu, float tau, float2 *F, int n,
                       double dwav, const int16_t *tab, int nb, double *numer, double *denom);
 int axg_uij_d2z_ff(axg_ctx *ctx, const double *u, const double *ud, double tau, double2 *out, int n);
 // the six FP64 Green sources of phi (d = 2 dx; inv_d, d_pow2 as
