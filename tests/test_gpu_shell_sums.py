@@ -59,9 +59,9 @@ def test_green_shells(n, nb, precision):
     assert np.all(np.abs(gnu - nu) <= 1e-9 * np.max(nu / np.maximum(de, 1)) * de)
 
 
-# the window matrix by prefix sums and the device's table of it: one bin, more
-# than a warp of bins, degraded transforms, sizes with and without own FFTs
-@pytest.mark.parametrize("n,nb,deg", [(6, 1, 0), (6, 3, 0), (16, 4, 1), (34, 17, 0), (40, 9, 1), (80, 40, 0)])
+# the window matrix, directly below m = 104 and by prefix sums from there, and the
+# device's table of it: one bin, more than a warp of bins, degraded transforms
+@pytest.mark.parametrize("n,nb,deg", [(6, 1, 0), (6, 3, 0), (16, 4, 1), (34, 17, 0), (40, 9, 1), (80, 40, 0), (102, 12, 0), (104, 12, 0), (112, 40, 0)])
 def test_window_matrix(n, nb, deg):
     phi, phid = state(n, 5 * n)
     p = spec_params(n, num_bin=nb, degrade_spec=deg)
