@@ -70,9 +70,15 @@ __device__ __forceinline__ void load_c(const V *a, const V *comp, int64_t s, dou
 // field's truncation to float.
 // About 20 instructions against some 40 of atan2f, whose care for special
 // operands the range test replaces: outside [2^-100, 2^120] of the larger
-// component, and for zeros, infinities and NaN, the phase is unknown.
+// component, and for zeros, infinities and NaN (in either component: d is then
+// NaN), the phase is unknown.
+__device__ __forceinline__ float max_nan(float a, float b) {  // fmaxf drops a NaN
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 __device__ __forceinline__ float phase_fast(float re, float im, float unknown) {
-  const float ar = fabsf(re), ai = fabsf(im), d = fmaxf(ar, ai), q = __fdividef(fminf(ar, ai), d), t = q * q;
+  const float ar = fabsf(re), ai = fabsf(im), d = max_nan(ar, ai), q = __fdividef(fminf(ar, ai), d), t = q * q;
   float p = fmaf(t, 0.0028662257f, -0.0161657367f);
   p = fmaf(t, p, 0.0429096138f);
   p = fmaf(t, p, -0.0752896400f);
