@@ -343,11 +343,9 @@ struct LoadReals {
 };
 struct LoadWindow {
   const int8_t *flags;
-  float hi, lo;  // dv
   __device__ __forceinline__ float4 pair(int64_t r, int n, int m) const {
     const char2 f = reinterpret_cast<const char2 *>(flags + r * n)[m];
-    const bool a = f.x & 4, b = f.y & 4;
-    return make_float4(a ? 0.f : hi, a ? 0.f : lo, b ? 0.f : hi, b ? 0.f : lo);
+    return make_float4(f.x & 4 ? 0.f : 1.f, 0.f, f.y & 4 ? 0.f : 1.f, 0.f);
   }
 };
 struct LoadComplex {
@@ -1483,9 +1481,8 @@ int axg_ff_d2z(axg_ctx *ctx, const double *in, double2 *out, int n, int batch, b
   return d2z_n(ctx, LoadReals{in}, out, n, batch, keep_ff);
 }
 
-int axg_ff_d2z_window(axg_ctx *ctx, const int8_t *flags, double dv, double2 *out, int n) {
-  const float hi = (float)dv;
-  return d2z_n(ctx, LoadWindow{flags, hi, (float)(dv - (double)hi)}, out, n, 1, true);
+int axg_ff_d2z_window(axg_ctx *ctx, const int8_t *flags, double2 *out, int n) {
+  return d2z_n(ctx, LoadWindow{flags}, out, n, 1, true);
 }
 
 bool axg_gw_fused_f32(int n) { return axg_ff_fft_supported(n) && n > kGreenUnfused; }

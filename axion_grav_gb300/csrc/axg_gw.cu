@@ -591,6 +591,19 @@ __device__ __forceinline__ F2 acc_norm2(const float4 *__restrict__ acc, int64_t 
   }
   return v;
 }
+// in FP64, for entries that fail squares_fit
+__device__ double acc_norm2_wide(const double2 *__restrict__ acc, int64_t astride, int64_t h) {
+  return acc_norm2(acc, astride, h);
+}
+__device__ __noinline__ double acc_norm2_wide(const float4 *__restrict__ acc, int64_t astride, int64_t h) {
+  double v = 0.0;
+  for (int a = 0; a < 4; ++a) {
+    const float4 z = acc[a * astride + h];
+    const double re = (double)z.x + (double)z.y, im = (double)z.z + (double)z.w;
+    v += re * re + im * im;
+  }
+  return v;
+}
 // Green accumulators -> numer / denom per bin (bin of |k|^2 from the table).
 // A stored entry with 0 < hx < n/2 stands for k and -k (the same |k|): its
 // |A|^2 counts twice, or once plus the Nyquist-row mirror's own entry.
@@ -609,12 +622,16 @@ __global__ void __launch_bounds__(256) k_gw_bin_green(const A *__restrict__ acc,
     const int kx = kint(hx, n), ky = kint(hy, n), kz = kint(hz, n);
     const int b = tab[kx * kx + ky * ky + kz * kz];
     if (b < 0) return;
-    const bool mirror = hx > 0 && hx < n / 2;
-    const auto v1 = acc_norm2(acc, astride, ((int64_t)hz * n + hy) * nh + hx);
-    auto v = v1;
-    if (mirror)
-      v = run_sum(v1, hy == n / 2 || hz == n / 2 ? acc_norm2(acc, astride, nhalf + gw_nyq_extra(hx, hy, hz, n)) : v1);
-    run.add(bins, b, v, mirror ? 2u : 1u);
+    const bool mirror = hx > 0 && hx < n / 2, own = mirror && (hy == n / 2 || hz == n / 2);
+    const int64_t h = ((int64_t)hz * n + hy) * nh + hx, e = nhalf + gw_nyq_extra(hx, hy, hz, n);
+    const auto v1 = acc_norm2(acc, astride, h), v2 = own ? acc_norm2(acc, astride, e) : v1;
+    const auto v = mirror ? run_sum(v1, v2) : v1;
+    if (squares_fit(v1) && squares_fit(v2)) {
+      run.add(bins, b, v, mirror ? 2u : 1u);
+    } else {
+      const double d = acc_norm2_wide(acc, astride, h);
+      bins.add(b, mirror ? d + (own ? acc_norm2_wide(acc, astride, e) : d) : d, mirror ? 2u : 1u);
+    }
   });
   run.flush(bins);
   bins.finish(numer, denom);

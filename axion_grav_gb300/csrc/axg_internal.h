@@ -277,9 +277,9 @@ bool axg_ff_use(int n);
 int axg_ff_d2z(axg_ctx *ctx, const double *in, double2 *out, int n, int batch, bool keep_ff = false);
 int axg_ff_z2z(axg_ctx *ctx, double2 *data, int n, int inverse, bool keep_ff = false);  // in place, one n^3 volume
 // the same of a field that the defect flags mask (zero where bit 4 is set)
-// into out, kept float-float; and the D2Z of the window, dv where it is clear
+// into out, kept float-float; and the D2Z of the window, 1 where it is clear
 int axg_ff_z2z_masked(axg_ctx *ctx, const void *field, bool fp32, const int8_t *flags, double2 *out, int n, int inverse);
-int axg_ff_d2z_window(axg_ctx *ctx, const int8_t *flags, double dv, double2 *out, int n);
+int axg_ff_d2z_window(axg_ctx *ctx, const int8_t *flags, double2 *out, int n);
 // The Green accumulators hold the stored half spectrum only: component a of
 // the entry h = (hz n + hy) (n/2 + 1) + hx is acc[a acc_stride + h], and the
 // site of -k is its conjugate (real sources, and e+(-k) = conj e+(k)).  On

@@ -60,12 +60,17 @@ __global__ void k_spec_degrade(const V *__restrict__ phid, const int8_t *__restr
   }
 }
 
-// |F|^2 per k-site into the bins of |k|^2, F in FP64 (cuFFT, the Monte-Carlo
-// fields) or float-float; the sums are scaled on the host
+// |F|^2 per k-site into the bins of |k|^2, F in FP64 (cuFFT) or float-float;
+// the sums are scaled on the host
 __device__ __forceinline__ double norm2(double2 w) { return w.x * w.x + w.y * w.y; }
 __device__ __forceinline__ F2 norm2(float4 w) {
   const F2 r = {w.x, w.y}, i = {w.z, w.w};
   return f2_dot2(r, r, i, i, 1.f);
+}
+// in FP64, for sites that fail squares_fit
+__device__ __forceinline__ double norm2_wide(double2 w) { return norm2(w); }
+__device__ __forceinline__ double norm2_wide(float4 w) {
+  return norm2(make_double2((double)w.x + (double)w.y, (double)w.z + (double)w.w));
 }
 template <typename V>
 __global__ void __launch_bounds__(256) k_spec_bin(const V *__restrict__ F, int m, int rows,
@@ -76,15 +81,19 @@ __global__ void __launch_bounds__(256) k_spec_bin(const V *__restrict__ F, int m
   walk_spectrum(m, m, rows, [&](int ix, int iy, int iz) {
     const int kx = kint(ix, m), ky = kint(iy, m), kz = kint(iz, m);
     const int b = tab[kx * kx + ky * ky + kz * kz];
-    if (b >= 0) run.add(bins, b, norm2(F[((int64_t)iz * m + iy) * m + ix]), 1u);
+    if (b < 0) return;
+    const V f = F[((int64_t)iz * m + iy) * m + ix];
+    const auto v = norm2(f);
+    if (squares_fit(v)) run.add(bins, b, v, 1u);
+    else bins.add(b, norm2_wide(f), 1u);
   });
   run.flush(bins);
   bins.finish(conv, count);
 }
 
-// the real window of compute_matrix_deconv: dx^3 on unmasked coarse cells
-__global__ void k_spec_window(const int8_t *__restrict__ flags, int n, int deg, double dv_spa,
-                              double *__restrict__ out) {
+// the real window of compute_matrix_deconv over its dx^3: 1 on unmasked coarse
+// cells (the pair sums take dx^6 on the host)
+__global__ void k_spec_window(const int8_t *__restrict__ flags, int n, int deg, double *__restrict__ out) {
   const int m = n / deg;
   const int64_t m3 = (int64_t)m * m * m, n2 = (int64_t)n * n;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -99,12 +108,14 @@ __global__ void k_spec_window(const int8_t *__restrict__ flags, int n, int deg, 
               masked = true;
               break;
             }
-    out[c] = masked ? 0.0 : dv_spa;
+    out[c] = masked ? 0.0 : 1.0;
   }
 }
 
 // |W|^2 per integer |k|^2 from the half spectrum of the real window
-// (|W(-k)| = |W(k)|: interior kx planes count twice)
+// (|W(-k)| = |W(k)|: interior kx planes count twice).  W is the transform of
+// ones and zeros: at most m^3, and below 2^-48 of that it is its own rounding,
+// so float-float squares have the range for it.
 template <typename V>
 __global__ void k_spec_w2_hist(const V *__restrict__ W, int m, double *__restrict__ h) {
   const int mh = m / 2 + 1;
@@ -606,9 +617,9 @@ int axg_spec_estimation(axg_ctx *ctx, double tau, double *wave, double *power, d
     const bool ff = axg_ff_use(m), direct = ff && deg == 1;
     const int wgrid = walk_grid(m, m / 2 + 1, 1);
     if (direct) {
-      AXG_TRY(axg_ff_d2z_window(ctx, ctx->flags, dv_spa, whalf, m));
+      AXG_TRY(axg_ff_d2z_window(ctx, ctx->flags, whalf, m));
     } else {
-      AXG_LAUNCH(ctx, "spec_window", k_spec_window, grid_for(m3), 256, 0, ctx->flags, n, deg, dv_spa, wreal);
+      AXG_LAUNCH(ctx, "spec_window", k_spec_window, grid_for(m3), 256, 0, ctx->flags, n, deg, wreal);
       if (ff) AXG_TRY(axg_ff_d2z(ctx, wreal, whalf, m, 1, true));
       else AXG_CUFFT_TRY(ctx, cufftExecD2Z(ctx->plan_window, wreal, (cufftDoubleComplex *)whalf));
     }
@@ -648,7 +659,8 @@ int axg_spec_estimation(axg_ctx *ctx, double tau, double *wave, double *power, d
     AXG_CUDA_TRY(ctx, cudaMemcpyAsync(hb.data(), d_conv, hb.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
     AXG_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     std::vector<double> mat(num_cov);
-    for (int ij = 0; ij < num_cov; ++ij) mat[ij] = hm[ij] / hm[num_cov + ij] * dv_wav * dv_wav;
+    for (int ij = 0; ij < num_cov; ++ij)
+      mat[ij] = hm[ij] / hm[num_cov + ij] * (dv_spa * dv_spa) * dv_wav * dv_wav;
     if (pp_inverse(nb, mat.data()) != 0) {
       rc = axg_set_error(ctx, AXG_ERR_NUMERIC, "deconvolution matrix not positive definite");
       break;

@@ -1,0 +1,92 @@
+"""Spectra of fields and accumulators far from one, and of very small and very
+large lattice spacings: scaling by a power of two scales the sums of squares by
+its square, whichever numbers single precision could square."""
+import numpy as np
+import pytest
+
+import axion_grav_gb300 as ag
+from oracle import axo
+from tests.test_gpu_shell_sums import gw_params, noise
+from tests.test_gpu_spectrum import params as spec_params, state
+
+pytestmark = pytest.mark.gpu
+
+
+# The transforms hold values as pairs of floats, so a power of two commutes with
+# them; a term of a sum is off by at most 2^-45 of itself, and all are positive.
+TOL = 1e-12
+SHIFTS = [-80, -62, -45, 55, 66, 80]
+
+
+def field_spectrum(n, precision, deg, shift):
+    phi, phid = state(n, 11 * n + deg)
+    if precision == ag.PREC_FP32_MIXED:
+        phi, phid = (a.astype(np.complex64).astype(np.complex128) for a in (phi, phid))
+    with ag.Lattice(spec_params(n, precision, degrade_spec=deg)) as lat:
+        lat.upload(phi, np.ldexp(1.0, shift) * phid)
+        lat.classify_cells(7)
+        return lat.spectrum_estimation(3.0)
+
+
+# 16 to 64: the transforms in pairs of floats; 24: cuFFT's in FP64
+@pytest.mark.parametrize("n,deg", [(16, 0), (64, 0), (64, 1), (24, 0)])
+@pytest.mark.parametrize("precision", [ag.PREC_FP64_PLAIN, ag.PREC_FP32_MIXED])
+def test_field_spectrum_scales(n, deg, precision):
+    w, pw, cv, ct = field_spectrum(n, precision, deg, 0)
+    for s in SHIFTS:
+        _, gpw, gcv, gct = field_spectrum(n, precision, deg, s)
+        np.testing.assert_array_equal(gct, ct)
+        np.testing.assert_allclose(np.ldexp(gcv, -2 * s), cv, rtol=TOL, err_msg=str(s))
+        np.testing.assert_allclose(np.ldexp(gpw, -2 * s), pw, rtol=1e-8, atol=1e-10 * np.max(np.abs(pw)))
+
+
+# dx^3 is a factor of the window and of the field
+@pytest.mark.parametrize("n,deg", [(16, 0), (32, 1), (112, 0), (24, 0)])
+@pytest.mark.parametrize("dspa", [1e-8, 2.0 ** -10, 3e5])
+def test_field_spectrum_of_any_spacing(n, deg, dspa):
+    phi, phid = state(n, n)
+    p = spec_params(n, degrade_spec=deg, dspa=dspa)
+    flags, _ = axo.classify_cells(p, phi, 7, 0)
+    w, pw, cv, ct, md = axo.spectrum_estimation(p, phid, flags, 3.0)
+    with ag.Lattice(p) as lat:
+        lat.upload(phi, phid)
+        lat.classify_cells(7)
+        gw, gpw, gcv, gct = lat.spectrum_estimation(3.0)
+    np.testing.assert_array_equal(gct, ct)
+    np.testing.assert_allclose(gcv, cv, rtol=1e-10)
+    np.testing.assert_allclose(gpw, pw, rtol=1e-8, atol=1e-10 * np.max(np.abs(pw)))
+
+
+@pytest.mark.parametrize("shift", [-66, 60])
+def test_covariance_scales(shift):
+    n = 16
+    phi, phid = state(n, 3)
+    cov = {}
+    for s in (0, shift):
+        with ag.Lattice(spec_params(n)) as lat:
+            lat.upload(phi, np.ldexp(1.0, s) * phid)
+            lat.classify_cells(7)
+            lat.spectrum_estimation(3.0)
+            cov[s], _ = lat.spectrum_covariance(4, 4, 0.05)
+    want = cov[0]
+    np.testing.assert_allclose(np.ldexp(cov[shift], -4 * shift), want, rtol=1e-8, atol=1e-10 * np.max(np.abs(want)))
+
+
+# accumulators as pairs of floats (16, 32, and every FP32-mixed size) and FP64
+# ones (18), with the edges of the shell walk: one bin, some, the most
+@pytest.mark.parametrize("n", [16, 18, 32])
+@pytest.mark.parametrize("nb", [1, 25, 256])
+@pytest.mark.parametrize("precision", [ag.PREC_FP64_PLAIN, ag.PREC_FP64_FUSED, ag.PREC_FP32_MIXED])
+def test_green_shells_scale(n, nb, precision):
+    phi, phid = 1.0 + noise(n, n, 0.2), noise(n, n + 1, 0.1)
+    p = gw_params(n, ag.PREC_FP64_PLAIN, ag.GW_GREEN, nb)
+    acc = np.zeros((4, n, n, n), np.complex128)
+    axo.symplectic_integration(p, phi.copy(), phid.copy(), None, None, acc, 2.0, 2.4, 0.4)
+    w, pw, nu, de = axo.grav_spec_estimation(p, acc)
+    with ag.Lattice(gw_params(n, precision, ag.GW_GREEN, nb)) as lat:
+        for s in [0] + SHIFTS:
+            lat.upload_gw_green(np.ldexp(1.0, s) * acc)
+            _, _, gnu, gde = lat.grav_spec_estimation(2.4)
+            np.testing.assert_array_equal(gde, de)
+            # an accumulator is held to 2^-48, its square to 2^-46
+            np.testing.assert_allclose(np.ldexp(gnu, -2 * s), nu, rtol=TOL, err_msg=str(s))
