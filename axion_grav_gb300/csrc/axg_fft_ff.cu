@@ -1167,17 +1167,22 @@ struct UijSink {
     if (ix <= L / 2) {
       const unsigned wgt = (ix == 0 || ix == L / 2) ? 1u : 2u;  // Hermitian partner of the half spectrum
       const int p2 = (int)(kx * kx + ky * ky);
-      auto put = [&](int z, F2 v, unsigned w) {
+      auto put = [&](int z, float p, float q, unsigned w) {  // p + q, floats whose sums need not be
         const int b = a.tab[p2 + z * z];
-        if (b >= 0) run.add(bins, b, F2{(float)wgt * v.h, (float)wgt * v.l}, wgt * w);
+        if (b < 0) return;
+        if (fmaxf(p, q) < 0x1p118f) {
+          const F2 v = f2_add(F2{p, 0.f}, F2{q, 0.f});
+          run.add(bins, b, F2{(float)wgt * v.h, (float)wgt * v.l}, wgt * w);
+        } else {
+          bins.add(b, (double)wgt * ((double)p + (double)q), wgt * w);
+        }
       };
-      if (j == 0) put(0, F2{x[0], 0.f}, 1u);
+      if (j == 0) put(0, x[0], 0.f, 1u);
 #pragma unroll
       for (int i = 1; i <= PER; ++i) {
         const int z = j * PER + i;
-        const F2 v = {x[at(z)], 0.f};
-        if (z < L / 2) put(z, f2_add(v, F2{x[at(L - z)], 0.f}), 2u);
-        else put(z, v, 1u);
+        if (z < L / 2) put(z, x[at(z)], x[at(L - z)], 2u);
+        else put(z, x[at(z)], 0.f, 1u);
       }
       run.flush(bins);
     }

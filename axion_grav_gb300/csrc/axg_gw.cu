@@ -694,7 +694,9 @@ __global__ void __launch_bounds__(256) k_uij_bin(const CV *__restrict__ F, int n
     const TTBasis<R> t = tt_basis<R>(kx, ky, kz, k2);
     const unsigned wgt = (ix == 0 || 2 * ix == n) ? 1u : 2u;  // Hermitian partner of the half spectrum
     const R e = tt_power(t, F + 6 * nspec, nspec, h) + (R)k2 * dwav2 * tt_power(t, F, nspec, h);
-    run.add(bins, b, (double)((R)wgt * e), wgt);
+    double v = (double)e;
+    if (wgt == 2u) v += v;  // here: twice a float may not be one
+    run.add(bins, b, v, wgt);
   });
   run.flush(bins);
   bins.finish(numer, denom);

@@ -90,3 +90,25 @@ def test_green_shells_scale(n, nb, precision):
             np.testing.assert_array_equal(gde, de)
             # an accumulator is held to 2^-48, its square to 2^-46
             np.testing.assert_allclose(np.ldexp(gnu, -2 * s), nu, rtol=TOL, err_msg=str(s))
+
+
+def test_uij_powers_near_the_largest_float():
+    """One plane wave along z: the power of an entry is a float, the sum of a
+    shell need not be one."""
+    n, m, tau = 16, 3, 0.5
+    p = gw_params(n, ag.PREC_FP64_PLAIN, ag.GW_UIJ, 25)
+    u = np.zeros((6, n, n, n))
+    u[1] = np.cos(2 * np.pi * m * np.arange(n) / n)[:, None, None]
+    ud = np.zeros_like(u)
+    k = m * 2 * np.pi / n / p.dspa
+    # an entry's power is 2 A^2 (n^3/2)^2 (1 + k^2 tau^2): 0.8 of the largest float
+    u *= np.sqrt(0.8 * np.finfo(np.float32).max / 2 / (n ** 3 / 2) ** 2 / (1 + (k * tau) ** 2))
+    u = u.astype(np.float32).astype(np.float64)
+    w, pw, nu, de = axo.uij_grav_spec(p, u, ud, tau)
+    with ag.Lattice(gw_params(n, ag.PREC_FP32_MIXED, ag.GW_UIJ, 25)) as lat:
+        lat.upload(np.ones((n, n, n), np.complex128), np.zeros((n, n, n), np.complex128))
+        lat.upload_uij(u, ud)
+        _, _, gnu, gde = lat.grav_spec_estimation(tau)
+    np.testing.assert_array_equal(gde, de)
+    assert np.all(np.isfinite(gnu))
+    assert np.all(np.abs(gnu - nu) <= 1e-5 * np.max(nu))
