@@ -122,6 +122,7 @@ struct axg_ctx {
   int64_t last_ns = 0, last_nw = 0, last_nm = 0;
 
   // spectra
+  bool spec_ready = false;     // axg_spec_init has finished: everything below exists
   double *spec_mat = nullptr;  // mat_spec [num_cov][501]
   double *spec_largeq0 = nullptr, *spec_dq = nullptr;  // per ij
   double *spec_modes = nullptr;      // per ij: sum over the lattice's modes of the pair's table

@@ -513,7 +513,17 @@ int window_sums(axg_ctx *ctx, const double *h, int64_t iq2max, double dwav, Sums
 
 // init_spectrum (spectrum.f90:23-103): bin pairs on the host, tables on the device
 int axg_spec_init(axg_ctx *ctx) {
-  if (ctx->spec_mat) return AXG_OK;
+  if (ctx->spec_ready) return AXG_OK;
+  // an attempt that fails leaves nothing behind, so that the next one starts again
+  auto undo = axg_on_exit([&] {
+    if (ctx->spec_ready) return;
+    for (void **q : {(void **)&ctx->spec_mat, (void **)&ctx->spec_largeq0, (void **)&ctx->spec_dq,
+                     (void **)&ctx->spec_range, (void **)&ctx->spec_modes, (void **)&ctx->spec_buf})
+      axg_free(ctx, q);
+    if (ctx->plan_spec_ok) cufftDestroy(ctx->plan_spec);
+    if (ctx->plan_window_ok) cufftDestroy(ctx->plan_window);
+    ctx->plan_spec_ok = ctx->plan_window_ok = false;
+  });
   const int nb = ctx->p.num_bin;
   const int num_cov = nb * (nb + 1) / 2;
   const int deg = 1 << ctx->p.degrade_spec;
@@ -580,6 +590,7 @@ int axg_spec_init(axg_ctx *ctx) {
   AXG_CUFFT_TRY(ctx, cufftPlan3d(&ctx->plan_window, m, m, m, CUFFT_D2Z));
   ctx->plan_window_ok = true;
   AXG_CUFFT_TRY(ctx, cufftSetStream(ctx->plan_window, ctx->stream));
+  ctx->spec_ready = true;
   return AXG_OK;
 }
 
