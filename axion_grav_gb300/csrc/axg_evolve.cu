@@ -69,12 +69,17 @@ __host__ __device__ inline Coef64 make_coef64(const double f[4], const double po
 // Every product of a site runs on the integer pipes (axg_soft64.h), beside
 // the FP64 pipe that the stencil is bound by: 79 sums stay there of a kick's
 // 128 operations (phi and six u_ij).  Each block counts its operands through
-// the `ok` flags; a block with an operand outside the window (a zero of the
-// initial u_ij, say) is redone with hardware operations, out of line.
+// the `ok` flags.  One whose inputs are outside the window (a zero of the
+// initial u_ij, say, or a coefficient: lambda = 0) runs on hardware operations
+// alone, out of line; one that leaves it on the way is redone so.  Counted only
+// at the end, inputs outside did their work twice: a free field's step at 128^3
+// took 681 us, now 556 (610 with hardware products throughout), phi alone 220,
+// now 164 (172).
 // Us per launch at 128^3, phi and u_ij: kick 535 -> 347 (the 79 sums alone
 // are 310 at the measured FP64 rate), drift 77 -> 66, fused 602 -> 415; phi
 // alone 167 -> 101.  At 100^3, where 2 dx is no power of two, the kick 360 ->
-// 278 and the fused step 382 -> 249.
+// 278 and the fused step 382 -> 249.  Three CTAs of the kick an SM: with two the
+// step of 128^3 took 439, with three 412.
 
 __device__ __forceinline__ double sum6_64(double xm, double xp, double ym, double yp, double zm, double zp) {
   double l = AXD_ADD(xm, xp);
@@ -111,7 +116,8 @@ __device__ __noinline__ double2 phi_kick64_hw(const Coef64 &k, double2 c, double
 
 // sum: the six neighbours' sum
 __device__ __forceinline__ double2 phi_kick64(const Coef64 &k, double2 c, double2 sum, double2 pd) {
-  uint32_t ok = k.soft;
+  uint32_t ok = k.soft & axs_window2(c.x, c.y) & axs_window2(pd.x, pd.y);
+  if (!(ok & AXS_WINDOW)) return phi_kick64_hw(k, c, sum, pd);
   const double lr = AXD_SUB(sum.x, six64(c.x, ok)), li = AXD_SUB(sum.y, six64(c.y, ok));
   const double s2 = AXD_ADD(axs_mul(c.x, c.x, &ok), axs_mul(c.y, c.y, &ok));
   const double g = AXD_ADD(axs_mulc(s2, &k.A, &ok), k.B);
@@ -137,7 +143,8 @@ __device__ __noinline__ double u_kick64_hw(const Coef64 &k, double S, double uc,
 }
 
 __device__ __forceinline__ double u_kick64(const Coef64 &k, double S, double uc, double sum, double udv) {
-  uint32_t ok = k.soft;
+  uint32_t ok = k.soft & axs_window2(uc, udv) & axs_window2(S, S);
+  if (!(ok & AXS_WINDOW)) return u_kick64_hw(k, S, uc, sum, udv);
   const double lu = AXD_SUB(sum, six64(uc, ok));
   const double v = AXD_ADD(axs_mulc(udv, &k.f1, &ok), axs_mulc(lu, &k.f2, &ok));
   const double r = AXD_ADD(v, axs_mulc(S, &k.fs, &ok));
@@ -148,10 +155,9 @@ __device__ __forceinline__ double u_kick64(const Coef64 &k, double S, double uc,
 // x + h v
 __device__ __noinline__ double drift64_hw(double x, double v, double h) { return AXD_ADD(x, AXD_MUL(h, v)); }
 __device__ __forceinline__ double drift64(const axs_const &h, double x, double v) {
-  uint32_t ok = h.ok ? 0xffffffffu : 0u;
-  const double r = AXD_ADD(x, axs_mulc(v, &h, &ok));
-  if (ok & AXS_WINDOW) return r;
-  return drift64_hw(x, v, h.v);
+  uint32_t ok = axs_window2(v, v);
+  if (!h.ok || !(ok & AXS_WINDOW)) return drift64_hw(x, v, h.v);
+  return AXD_ADD(x, axs_mulc(v, &h, &ok));
 }
 
 __global__ void k_drift_fp64(double2 *__restrict__ phi, const double2 *__restrict__ phid,
@@ -179,7 +185,7 @@ __device__ __forceinline__ int wrapi(int i, int n) { return i < 0 ? i + n : (i >
 // UIJ: also kick the six u_ij (a template parameter, so the phi-only kick
 // keeps the registers, and the resident warps, of its own work)
 template <bool UIJ>
-__global__ void __launch_bounds__(256) k_kick_fp64(const double2 *__restrict__ phi,
+__global__ void __launch_bounds__(256, UIJ ? 3 : 1) k_kick_fp64(const double2 *__restrict__ phi,
                                                    double2 *__restrict__ phid,
                                                    const double *__restrict__ u,
                                                    double *__restrict__ ud, int n, const __grid_constant__ Coef64 k) {

@@ -38,15 +38,30 @@ __device__ __forceinline__ double gw_div_d(double x, double d, const axs_const &
   return AXD_FMA(AXD_FMA(-d, q, x), inv_d.v, q);
 }
 
+// copies, so that the arrays of the usual path stay in registers
+__device__ __forceinline__ void gw_sources_redo(const double xr[3], const double xi[3], double d, double inv_d,
+                                                int d_pow2, double S[6]) {
+  const double a[3] = {xr[0], xr[1], xr[2]}, b[3] = {xi[0], xi[1], xi[2]};
+  double T[6];
+  gw_sources_from_diff_hw(a, b, d, inv_d, d_pow2, T);
+#pragma unroll
+  for (int k = 0; k < 6; ++k) S[k] = T[k];
+}
+
 // The same with the products on the integer pipes (axg_soft64.h), for kernels
 // that the FP64 pipe bounds; a site with an operand outside their window (a
-// zero difference, say) is redone above.  The float-float row pass keeps the
+// zero difference, say) is done above.  The float-float row pass keeps the
 // hardware products (gw_sources_fp64<false>): its butterflies fill the issue
 // slots, and 256^3 rows took 1.39 ms with integer products against 1.29.
 __device__ __forceinline__ void gw_sources_from_diff(const double xr[3], const double xi[3], double d, double inv_d,
                                                      int d_pow2, double S[6]) {
   const axs_const ic = axs_const_of(inv_d), dc = axs_const_of(d);
   uint32_t ok = d_pow2 || (ic.ok && dc.ok && !(dc.hi == 0x1fffffu && dc.lo == 0xffffffffu)) ? 0xffffffffu : 0u;
+  ok &= axs_window2(xr[0], xi[0]) & axs_window2(xr[1], xi[1]) & axs_window2(xr[2], xi[2]);
+  if (!(ok & AXS_WINDOW)) {
+    gw_sources_redo(xr, xi, d, inv_d, d_pow2, S);
+    return;
+  }
   double dr[3], di[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -59,13 +74,7 @@ __device__ __forceinline__ void gw_sources_from_diff(const double xr[3], const d
 #pragma unroll
     for (int j = 0; j <= i; ++j, ++c)
       S[c] = axg_mul_pow2(AXD_ADD(axs_mul(dr[i], dr[j], &ok), axs_mul(di[i], di[j], &ok)), 2.0);  // == r1 + r1
-  if (!(ok & AXS_WINDOW)) {  // copies, so that the arrays of the usual path stay in registers
-    const double a[3] = {xr[0], xr[1], xr[2]}, b[3] = {xi[0], xi[1], xi[2]};
-    double T[6];
-    gw_sources_from_diff_hw(a, b, d, inv_d, d_pow2, T);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) S[k] = T[k];
-  }
+  if (!(ok & AXS_WINDOW)) gw_sources_redo(xr, xi, d, inv_d, d_pow2, S);
 }
 
 // pa[k], pb[k]: phi at x + e_k and x - e_k, k = x, y, z

@@ -78,6 +78,7 @@ AXS_FN double axs_make(uint32_t hi, uint32_t lo) {
  * [-511, 512], i.e. when the top two bits of its exponent field differ */
 AXS_FN uint32_t axs_in_window(uint32_t h) { return h ^ (h + h); }
 #define AXS_WINDOW 0x40000000u
+AXS_FN uint32_t axs_window2(double a, double b) { return axs_in_window(axs_hi(a)) & axs_in_window(axs_hi(b)); }
 
 AXS_FN axs_const axs_const_of(double v) {
   const uint32_t h = axs_hi(v);
