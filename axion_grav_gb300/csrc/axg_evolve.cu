@@ -1077,6 +1077,8 @@ StepShape step_shape(const axg_ctx *ctx) {
 }
 }  // namespace
 
+bool axg_evo_step_is_plain(const axg_ctx *ctx) { return step_shape(ctx).cfg < 0; }
+
 int axg_evo_kick_drift(axg_ctx *ctx, double t, double dt, double dtd) {
   if (ctx->p.precision == AXG_PREC_FP64_PLAIN)
     return axg_set_error(ctx, AXG_ERR_STATE, "fused step requested on the FP64-plain path");

@@ -263,6 +263,7 @@ int axg_encode_tmap(axg_ctx *ctx, CUtensorMap *m, CUtensorMapDataType dt, int ra
 int axg_evo_tile_count();
 axg_tile_cfg axg_evo_tile(int i);
 int axg_evo_tile_supported(const axg_ctx *ctx, int i);
+bool axg_evo_step_is_plain(const axg_ctx *ctx);  // a fused step would run the kernel without tiles
 int axg_evo_tile_preference(bool fp32, int rank);  // tile index of the rank-th preferred shape
 int axg_evo_build_tmaps(axg_ctx *ctx, int cfg);
 // one launch over every member's columns (ensemble.cu drives it); persistent

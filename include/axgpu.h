@@ -162,7 +162,10 @@ int axg_leapfrog(axg_ctx *ctx, double t1, double dt, int64_t nsteps, int first_h
 /* Tile shapes of the fused kick+drift kernel: a CTA owns a tx x ty column of
  * the lattice and marches through zc z-planes.  The autotuner times every
  * shape the lattice supports for `steps` steps on a snapshot of the state
- * (restored afterwards) and keeps the fastest.  *pointwise_tma (may be NULL)
+ * (restored afterwards) and keeps the fastest, whose index is *best_cfg; where
+ * the kernel that runs without a choice is faster than all of them (small
+ * lattices) that one stays.  *best_ms_per_step is the time of the kernel
+ * kept.  *pointwise_tma (may be NULL)
  * is 1 for shapes that also stage the pointwise fields (phi', u' and the
  * compensations) by TMA, one plane ahead. */
 int axg_tile_count(void);
