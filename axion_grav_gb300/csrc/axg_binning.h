@@ -23,6 +23,27 @@ enum axg_bin_kind {
 int axg_bin_table(axg_ctx *ctx, int kind, int m, double dwav, double dq, int nb, int logmode,
                   const double *edges, const int16_t **d_tab);
 
+// The walk of walk_spectrum below: `rows` consecutive ky a thread, its threads
+// counted in 32 bits (32-bit divisions), so at most 2^31 of them.
+inline int64_t walk_threads(int n, int nx, int rows) { return (int64_t)nx * n * ((n + rows - 1) / rows); }
+// long runs, but at least ~8 threads for each resident one
+inline int walk_rows(int n, int nx) {
+  int rows = 32;
+  while (rows > 2 && walk_threads(n, nx, rows) < 4 * 152 * 2048) rows /= 2;
+  return rows;
+}
+// no runs (kernels that add every entry by itself): a row a thread, more only
+// where the threads would not count in 32 bits (1025 x 2048 x 2048 is 2^32)
+inline int walk_rows_single(int n, int nx) {
+  int rows = 1;
+  while (walk_threads(n, nx, rows) > (1LL << 31)) rows *= 2;
+  return rows;
+}
+inline int walk_grid(int n, int nx, int rows) {
+  const int64_t b = (walk_threads(n, nx, rows) + 255) / 256;
+  return (int)(b > 152 * 8 ? 152 * 8 : b);
+}
+
 #ifdef __CUDACC__
 #include "axg_ff.h"
 
@@ -125,16 +146,5 @@ __device__ __forceinline__ void walk_spectrum(int n, int nx, int rows, F f) {
     const int y1 = min((int)(g + 1) * rows, n);
     for (int hy = (int)g * rows; hy < y1; ++hy) f((int)hx, hy, (int)hz);
   }
-}
-// rows per thread: long runs, but at least ~8 threads for each resident one
-inline int walk_rows(int n, int nx) {
-  int rows = 32;
-  while (rows > 2 && (int64_t)nx * n * ((n + rows - 1) / rows) < 4 * 152 * 2048) rows /= 2;
-  return rows;
-}
-inline int walk_grid(int n, int nx, int rows) {
-  const int64_t t = (int64_t)nx * n * ((n + rows - 1) / rows);
-  const int64_t b = (t + 255) / 256;
-  return (int)(b > 152 * 8 ? 152 * 8 : b);
 }
 #endif

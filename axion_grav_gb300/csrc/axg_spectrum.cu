@@ -117,9 +117,9 @@ __global__ void k_spec_window(const int8_t *__restrict__ flags, int n, int deg, 
 // ones and zeros: at most m^3, and below 2^-48 of that it is its own rounding,
 // so float-float squares have the range for it.
 template <typename V>
-__global__ void k_spec_w2_hist(const V *__restrict__ W, int m, double *__restrict__ h) {
+__global__ void k_spec_w2_hist(const V *__restrict__ W, int m, int rows, double *__restrict__ h) {
   const int mh = m / 2 + 1;
-  walk_spectrum(m, mh, 1, [&](int ix, int iy, int iz) {
+  walk_spectrum(m, mh, rows, [&](int ix, int iy, int iz) {
     const int kx = kint(ix, m), ky = kint(iy, m), kz = kint(iz, m);
     auto v = norm2(W[((int64_t)iz * m + iy) * mh + ix]);
     if (ix != 0 && 2 * ix != m) v = run_sum(v, v);
@@ -626,7 +626,7 @@ int axg_spec_estimation(axg_ctx *ctx, double tau, double *wave, double *power, d
     double2 *whalf = (double2 *)(((uintptr_t)(wreal + m3) + 255) & ~(uintptr_t)255);
     // (our own transforms of an undegraded field read the flags in their row pass)
     const bool ff = axg_ff_use(m), direct = ff && deg == 1;
-    const int wgrid = walk_grid(m, m / 2 + 1, 1);
+    const int wrows = walk_rows_single(m, m / 2 + 1), wgrid = walk_grid(m, m / 2 + 1, wrows);
     if (direct) {
       AXG_TRY(axg_ff_d2z_window(ctx, ctx->flags, whalf, m));
     } else {
@@ -634,8 +634,8 @@ int axg_spec_estimation(axg_ctx *ctx, double tau, double *wave, double *power, d
       if (ff) AXG_TRY(axg_ff_d2z(ctx, wreal, whalf, m, 1, true));
       else AXG_CUFFT_TRY(ctx, cufftExecD2Z(ctx->plan_window, wreal, (cufftDoubleComplex *)whalf));
     }
-    if (ff) AXG_LAUNCH(ctx, "spec_w2_hist", k_spec_w2_hist<float4>, wgrid, 256, 0, (const float4 *)whalf, m, h);
-    else AXG_LAUNCH(ctx, "spec_w2_hist", k_spec_w2_hist<double2>, wgrid, 256, 0, whalf, m, h);
+    if (ff) AXG_LAUNCH(ctx, "spec_w2_hist", k_spec_w2_hist<float4>, wgrid, 256, 0, (const float4 *)whalf, m, wrows, h);
+    else AXG_LAUNCH(ctx, "spec_w2_hist", k_spec_w2_hist<double2>, wgrid, 256, 0, whalf, m, wrows, h);
     AXG_TRY(window_sums(ctx, h, iq2max, dwav, (Sums *)(scratch + nscr), mat0));
     // ---- compute_conv_spec (spectrum.f90:466-567) ----
     if (direct) {
