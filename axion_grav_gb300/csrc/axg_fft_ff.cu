@@ -41,6 +41,7 @@
 #include "axg_gw_site.h"
 #include "axg_gw_source.h"
 #include "axg_internal.h"
+#include "axg_soft64.h"
 #include "axg_tma.h"
 
 namespace {
@@ -114,12 +115,14 @@ __device__ __forceinline__ T c_zero() {
   return z;
 }
 
-// a complex float-float from two doubles (re, im), split on the integer
-// pipes (zeros, common in masked fields, past f2_from_bits' FP64 branch): by
-// conversions, 8 FP64-pipe operations, the complex row pass was bound by the
-// FP64 pipe, 254 us at 256^3
+// a complex float-float from two doubles (re, im), split on the integer pipes
+// (zeros, common in masked fields, past the FP64 conversions): by conversions, 8
+// FP64-pipe operations, the complex row pass was bound by the FP64 pipe, 254 us
+// at 256^3
 __device__ __forceinline__ F2 f2_split(double x) {
-  return (__double_as_longlong(x) << 1) == 0 ? F2{0.f, 0.f} : f2_from_bits(x);
+  if ((__double_as_longlong(x) << 1) == 0) return F2{0.f, 0.f};
+  F2 v;
+  return axs_split(x, &v.h, &v.l) ? v : f2_from(x);
 }
 __device__ __forceinline__ float4 c_from(double2 x) { return cx(f2_split(x.x), f2_split(x.y)); }
 

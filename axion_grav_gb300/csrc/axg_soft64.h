@@ -1,6 +1,7 @@
 /*
  * axg_soft64.h -- IEEE double products on the integer pipes, correctly
- * rounded (round to nearest, ties to even), bit for bit the hardware's.
+ * rounded (round to nearest, ties to even), bit for bit the hardware's; and
+ * the split of a double into two floats there (axs_split).
  *
  * GB300 issues FP64 at 1/64 of the FP32 rate: measured, an SM retires 1.7
  * FP64 operations a clock against 57 32 x 32 -> 64-bit integer products, 57
@@ -156,6 +157,33 @@ AXS_FN double axs_mul(double a, double b, uint32_t *ok) {
   *ok &= axs_in_window(h) & axs_in_window(g);
   if (rh >= 0x7ff00000u) *ok = 0;
   return r;
+}
+
+/* x as the sum of two floats, the bits of (float)x and (float)(x - (float)x):
+ * h is x rounded to 24 bits (a tie away from zero, which moves h and l but not
+ * their sum), l the low 29 bits less what h took, as a signed integer converted
+ * to float and scaled by the power of two of its place.  |x - h - l| <= 2^-49
+ * |x|.  0: outside [2^-74, 2^127) (zeros, subnormals, non-finite x too), where
+ * the conversions have to do it. */
+AXS_FN int axs_split(double x, float *h, float *l) {
+  const uint32_t hi = axs_hi(x), lo = axs_lo(x), e = (hi >> 20) & 0x7ffu, sign = hi & 0x80000000u;
+  const uint32_t hb = sign | ((((e - 896u) << 23) | (hi & 0xfffffu) << 3 | lo >> 29) + (lo >> 28 & 1u));
+  const float r = (float)((int32_t)(lo << 3) >> 3);
+#if defined(__CUDA_ARCH__)
+  *h = __uint_as_float(hb);
+  *l = __uint_as_float(__float_as_uint(__fmul_rn(r, __uint_as_float((e - 948u) << 23))) ^ sign);
+#else
+  const uint32_t sb = ((e - 948u) & 0xffu) << 23;
+  uint32_t lb;
+  float scale, v;
+  memcpy(h, &hb, 4);
+  memcpy(&scale, &sb, 4);
+  v = r * scale;
+  memcpy(&lb, &v, 4);
+  lb ^= sign;
+  memcpy(l, &lb, 4);
+#endif
+  return e >= 949u && e <= 1149u;
 }
 
 #endif
