@@ -615,6 +615,7 @@ constexpr int kIdle = 2;                // groups of a warp without work that en
 constexpr int kRounds = 4;              // random starts screened per lane before the next evaluations
 constexpr int kFitStride = 5 * 4 + 5;   // doubles per cell of the simplex scratch: p[vertex][coordinate], chi2[vertex]
 constexpr int64_t kFitChunk = 1 << 21;  // cells per pass of the three kernels (420 MB of scratch at most)
+constexpr int64_t kFitChunkMin = 1 << 9;  // ... at least, where memory is short
 
 // a double as an integer of the same order; -0 becomes +0.  An involution.
 __device__ __forceinline__ long long dkey(double v) {
@@ -2013,16 +2014,21 @@ int axg_def_id_defects(axg_ctx *ctx, double tau, double sl[3], double wa[3], dou
       constexpr int per_cta = kFitThreads / kGrp;
       // scratch: simplexes, the cells handed over to k_string_simplex_warp (at most the resident groups), their count
       const int64_t rcap = resident * per_cta;
-      if ((rc = axg_alloc(ctx, (void **)&sim, (size_t)(std::min(ns, kFitChunk) * kFitStride + rcap + 1) * 8, "string fits")))
-        break;
-      int2 *rest = (int2 *)(sim + std::min(ns, kFitChunk) * kFitStride);
+      // (a lattice that leaves little memory is fitted in smaller rounds)
+      int64_t chunk = std::min(ns, kFitChunk);
+      while ((rc = axg_alloc(ctx, (void **)&sim, (size_t)(chunk * kFitStride + rcap + 1) * 8, "string fits")) ==
+                 AXG_ERR_NOMEM &&
+             chunk > kFitChunkMin)
+        chunk = (chunk + 1) / 2;
+      if (rc) break;
+      int2 *rest = (int2 *)(sim + chunk * kFitStride);
       unsigned *nrest = (unsigned *)(rest + rcap);
       // few cells: a warp each from the start.  An iteration then costs the
       // issue slots of two but a third of the time (64^3, 1.5e4 cells: 9.3
       // against 11.5 ms through k_string_simplex; 128^3, 1.3e5: 30 ms through it)
       const int64_t few = 5 * (kFitThreads / 32) * resident;
-      for (int64_t c0 = 0; c0 < ns; c0 += kFitChunk) {
-        const int64_t nc = std::min(kFitChunk, ns - c0);
+      for (int64_t c0 = 0; c0 < ns; c0 += chunk) {
+        const int64_t nc = std::min(chunk, ns - c0);
         AXG_LAUNCH(ctx, "string_start", k_string_start, (unsigned)((nc + per_cta - 1) / per_cta), kFitThreads, 0,
                    ctx->phase64, n, (uint64_t)ctx->p.seed, cells + c0, nc, sim);
         AXG_CUDA_TRY(ctx, cudaMemsetAsync(next, 0, sizeof(unsigned long long), ctx->stream));
