@@ -1980,11 +1980,13 @@ int axg_def_id_defects(axg_ctx *ctx, double tau, double sl[3], double wa[3], dou
     if ((rc = axg_alloc(ctx, (void **)&cells, (size_t)(ns + nw + 1) * 8, "defect cells"))) break;
     if (ns > ctx->cap_strings) {
       axg_free(ctx, (void **)&ctx->d_strings);
+      ctx->cap_strings = ctx->last_ns = 0;  // until there is a list again
       if ((rc = axg_alloc(ctx, (void **)&ctx->d_strings, (size_t)ns * 13 * 8, "string list"))) break;
       ctx->cap_strings = ns;
     }
     if (nw > ctx->cap_walls) {
       axg_free(ctx, (void **)&ctx->d_walls);
+      ctx->cap_walls = ctx->last_nw = 0;
       if ((rc = axg_alloc(ctx, (void **)&ctx->d_walls, (size_t)nw * 10 * 8, "wall list"))) break;
       ctx->cap_walls = nw;
     }
