@@ -728,10 +728,8 @@ int ensure_uij_fft(axg_ctx *ctx) {
   // our own transforms (power-of-two N up to 512; AXG_FFT_FF=0: cuFFT) form
   // the twelve fields in their row pass: only the 12 half spectra are stored
   ctx->uij_own_fft = axg_ff_use(n);
-  ctx->u_pitch = n / 2 + 1;
   if (ctx->uij_own_fft) {
-    if (fp32) ctx->u_pitch = axg_f32_spec_pitch(n);
-    const size_t bytes = (size_t)12 * n * n * ctx->u_pitch * 2 * rs;
+    const size_t bytes = (size_t)12 * n * n * (fp32 ? axg_f32_spec_pitch(n) : n / 2 + 1) * 2 * rs;
     AXG_TRY(axg_alloc(ctx, &ctx->ubuf, bytes, "u_ij spectra"));
     AXG_CUDA_TRY(ctx, cudaMemsetAsync(ctx->ubuf, 0, bytes, ctx->stream));  // the padding columns
     return AXG_OK;

@@ -105,7 +105,6 @@ struct axg_ctx {
                                // the fused source + R2C), else by cuFFT; fixed when the context is made
   bool uij_own_fft = false;    // u_ij spectrum: fields formed in our own row transforms (no real buffer, no plan)
   int gsrc_pitch = 0;          // kx row pitch of gsrcF (axg_f32_spec_pitch for the FP32 own transforms, else n/2+1)
-  int u_pitch = 0;             // kx row pitch of the u_ij spectra in ubuf (likewise)
   float *ff_tw = nullptr;      // float-float FFT twiddles W_n^k, k < n/2 (axg_fft_ff.cu)
   int ff_tw_n = 0;
   cufftHandle plan_gsrc = 0;

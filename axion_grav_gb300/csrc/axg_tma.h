@@ -63,10 +63,6 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, uint32_t sr
                "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                : "memory");
 }
-// brings [p, p + bytes) into the L2 (both multiples of 16)
-__device__ __forceinline__ void l2_prefetch(const void *p, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // the bulk stores committed so far have read their shared memory
 __device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
