@@ -1200,8 +1200,9 @@ struct UijSink {
 // whose coefficients are polynomials in kz:
 //   Sa = sum k^2 Re(e) Re(S), Se = sum k^2 Re(e) Im(S),
 //   Sb = sum |k| Im(e) Im(S), Sg = sum |k| Im(e) Re(S)   (S conjugated),
-// X+ = (Sa - Sb', Se + Sg'), X- = (Sa + Sb', Se - Sg') over k^2.  A chunk is the
-// accumulators of one output slot of every thread.
+// X+ = (Sa - Sb', Se + Sg'), X- = (Sa + Sb', Se - Sg') over k^2.  The sums carry
+// k^2 <= 2e5, so a source spectrum may reach 1e33.  A chunk is the accumulators
+// of one output slot of every thread.
 template <int L>
 struct GreenSink {
   static constexpr int kFields = 6, kChunks = 8;

@@ -285,7 +285,10 @@ int axg_event_record(axg_ctx *ctx, int slot);
 /* Milliseconds between two recorded slots (synchronises on the later one). */
 int axg_event_elapsed(axg_ctx *ctx, int slot_a, int slot_b, float *ms);
 /* When on, every kernel launch is bracketed by events and its time is
- * accumulated per kernel name (for the roofline). */
+ * accumulated per kernel name (for the roofline).  fused_kd_* is the fused
+ * step; _plain follows where the kernel without tiles ran and ngrid is no
+ * multiple of 32 or AXG_FUSED_PLAIN=1 asked for it (a small lattice of 32 or
+ * 64 sites a side runs that kernel too, under the short name). */
 int axg_set_kernel_timing(axg_ctx *ctx, int on);
 /* Name, launches and total ms of the i-th timed kernel; AXG_ERR_ARG past the end. */
 int axg_kernel_timing(axg_ctx *ctx, int i, char *name, int64_t name_len, int64_t *launches,
