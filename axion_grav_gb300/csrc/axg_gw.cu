@@ -821,7 +821,11 @@ int axg_gw_integration(axg_ctx *ctx, double tau, double dtau) {
     const double phase1 = dwav * tau / (3.14159265358979323846 / 2);  // of |k| = 1, in quarter turns
     const float th = (float)phase1, tl = (float)(phase1 - (double)th);
     // the sources' factor 2 / d^2: its power of two in them, the rest in the
-    // weight, which keeps what a float of it drops (an error common to all k)
+    // weight, whose low part is added to the weights' rounded products: they take
+    // up what exceeds half an ulp of theirs.  (Added before the rounding it is all
+    // kept, and the accumulators' mean error then is the float transforms' alone,
+    // -0.8e-7 at 128^3; but 512^3 spectra end 1.7e-7 from 64-bit ones instead of
+    // 1.5e-7, the two partly cancelling there.)
     int e2;
     const double dws = dw * std::frexp(2.0 / (d * d), &e2);
     const float scale = std::ldexp(1.f, e2), wh = (float)dws, wl = (float)(dws - (double)wh);
