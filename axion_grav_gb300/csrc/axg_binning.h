@@ -69,14 +69,14 @@ struct BlockBins {
     atomicAdd(&v[b * copies + (threadIdx.x & (copies - 1))], val);
     atomicAdd(&w[b], wt);
   }
-  // the block's totals into the global sums and counts
-  __device__ void finish(double *__restrict__ sum, double *__restrict__ count) {
+  // the block's totals, times a power of two, into the global sums and counts
+  __device__ void finish(double *__restrict__ sum, double *__restrict__ count, double scale = 1.0) {
     __syncthreads();
     for (int b = threadIdx.x; b < nb; b += blockDim.x)
       if (w[b]) {
         double t = 0.0;
         for (int c = 0; c < copies; ++c) t += v[b * copies + c];
-        atomicAdd(&sum[b], t);
+        atomicAdd(&sum[b], t * scale);
         atomicAdd(&count[b], (double)w[b]);
       }
   }
@@ -108,12 +108,35 @@ __device__ __forceinline__ double run_value(F2 a) { return f2_to(a); }
 // squares within [2^-96, 2^116] is good to 2^-46 of itself (no error term falls
 // below 2^-149) and a run of 2^9 of them stays finite; a site outside (or zero)
 // is squared in FP64 and added to the block's bins by itself: 256^3 k_spec_bin
-// 98 us, with every site outside 240; k_gw_bin_green 101 and 445.
+// 100 us, with every site outside 240; k_gw_bin_green 106 and 445.
 __device__ __forceinline__ bool squares_fit(F2 v) {
   const unsigned lo = (127u - 96u) << 23, hi = (127u + 116u) << 23;
   return __float_as_uint(v.h) - lo <= hi - lo;
 }
 __device__ __forceinline__ bool squares_fit(double) { return true; }
+// So that few sites are outside, the values are multiplied by a power of two
+// that puts the largest of a sample, one `m` a thread of the block, at 2^34:
+// sites from 2^-82 to 2^24 of it are inside, which spans the FP64 noise of a
+// smooth field's spectrum.  Without it a band-limited 128^3 lattice's Green bins
+// took 98 us a call instead of 60, most sites being such noise.  The sample only
+// decides how fast a site is summed; finish() takes the factor out again.
+struct SquareScale {
+  float s = 1.f;     // 2^k
+  double inv = 1.0;  // 2^-2k
+  __device__ SquareScale() {}
+  __device__ explicit SquareScale(float m) {
+    __shared__ unsigned top;
+    if (threadIdx.x == 0) top = 0u;
+    __syncthreads();
+    const unsigned u = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0 && u) atomicMax(&top, u);
+    __syncthreads();
+    const int e = (int)(top >> 23);
+    const int k = e == 0 || e == 255 ? 0 : min(127 + 34 - e, 100);  // zeros, infinities, NaN: as they are
+    s = __int_as_float((127 + k) << 23);
+    inv = __hiloint2double((1023 - 2 * k) << 20, 0);
+  }
+};
 template <typename Val>
 struct BinRun {
   int bin = -1;

@@ -571,8 +571,9 @@ __global__ void k_gw_accumulate_f32_mirrors(const float2 *__restrict__ srcF, int
 // ---------------- shell histograms ----------------
 constexpr int kMaxBins = 256;
 
-// sum of |A|^2 over the four accumulators of an entry: FP64, or float-float
-__device__ __forceinline__ double acc_norm2(const double2 *__restrict__ acc, int64_t astride, int64_t h) {
+// sum of |s A|^2 over the four accumulators of an entry: FP64 (s = 1), or
+// float-float
+__device__ __forceinline__ double acc_norm2(const double2 *__restrict__ acc, int64_t astride, int64_t h, float) {
   double v = 0.0;
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
@@ -581,28 +582,34 @@ __device__ __forceinline__ double acc_norm2(const double2 *__restrict__ acc, int
   }
   return v;
 }
-__device__ __forceinline__ F2 acc_norm2(const float4 *__restrict__ acc, int64_t astride, int64_t h) {
+__device__ __forceinline__ F2 acc_norm2(const float4 *__restrict__ acc, int64_t astride, int64_t h, float s) {
   F2 v = {0.f, 0.f};
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
     const float4 z = acc[a * astride + h];
-    const F2 r = {z.x, z.y}, i = {z.z, z.w};
+    const F2 r = {s * z.x, s * z.y}, i = {s * z.z, s * z.w};
     v = f2_add(v, f2_dot2(r, r, i, i, 1.f));
   }
   return v;
 }
 // in FP64, for entries that fail squares_fit
-__device__ double acc_norm2_wide(const double2 *__restrict__ acc, int64_t astride, int64_t h) {
-  return acc_norm2(acc, astride, h);
+__device__ double acc_norm2_wide(const double2 *__restrict__ acc, int64_t astride, int64_t h, float) {
+  return acc_norm2(acc, astride, h, 1.f);
 }
-__device__ __noinline__ double acc_norm2_wide(const float4 *__restrict__ acc, int64_t astride, int64_t h) {
+__device__ __noinline__ double acc_norm2_wide(const float4 *__restrict__ acc, int64_t astride, int64_t h, float s) {
   double v = 0.0;
   for (int a = 0; a < 4; ++a) {
     const float4 z = acc[a * astride + h];
-    const double re = (double)z.x + (double)z.y, im = (double)z.z + (double)z.w;
+    const double re = ((double)z.x + (double)z.y) * (double)s, im = ((double)z.z + (double)z.w) * (double)s;
     v += re * re + im * im;
   }
   return v;
+}
+// the sample of a block: component (t / 32) & 3 of the entries along kx
+__device__ __forceinline__ SquareScale acc_scale(const double2 *, int64_t, int) { return SquareScale(); }
+__device__ __forceinline__ SquareScale acc_scale(const float4 *__restrict__ acc, int64_t astride, int nh) {
+  const float4 z = acc[((threadIdx.x >> 5) & 3) * astride + min((int)(threadIdx.x & 31), nh - 1)];
+  return SquareScale(fmaxf(fabsf(z.x), fabsf(z.z)));
 }
 // Green accumulators -> numer / denom per bin (bin of |k|^2 from the table).
 // A stored entry with 0 < hx < n/2 stands for k and -k (the same |k|): its
@@ -617,24 +624,25 @@ __global__ void __launch_bounds__(256) k_gw_bin_green(const A *__restrict__ acc,
   BlockBins bins(bins_mem(), nb, copies);
   const int nh = n / 2 + 1;
   const int64_t nhalf = (int64_t)n * n * nh;
-  BinRun<decltype(acc_norm2(acc, astride, 0))> run;
+  const SquareScale scale = acc_scale(acc, astride, nh);
+  BinRun<decltype(acc_norm2(acc, astride, 0, 1.f))> run;
   walk_spectrum(n, nh, rows, [&](int hx, int hy, int hz) {
     const int kx = kint(hx, n), ky = kint(hy, n), kz = kint(hz, n);
     const int b = tab[kx * kx + ky * ky + kz * kz];
     if (b < 0) return;
     const bool mirror = hx > 0 && hx < n / 2, own = mirror && (hy == n / 2 || hz == n / 2);
     const int64_t h = ((int64_t)hz * n + hy) * nh + hx, e = nhalf + gw_nyq_extra(hx, hy, hz, n);
-    const auto v1 = acc_norm2(acc, astride, h), v2 = own ? acc_norm2(acc, astride, e) : v1;
+    const auto v1 = acc_norm2(acc, astride, h, scale.s), v2 = own ? acc_norm2(acc, astride, e, scale.s) : v1;
     const auto v = mirror ? run_sum(v1, v2) : v1;
     if (squares_fit(v1) && squares_fit(v2)) {
       run.add(bins, b, v, mirror ? 2u : 1u);
     } else {
-      const double d = acc_norm2_wide(acc, astride, h);
-      bins.add(b, mirror ? d + (own ? acc_norm2_wide(acc, astride, e) : d) : d, mirror ? 2u : 1u);
+      const double d = acc_norm2_wide(acc, astride, h, scale.s);
+      bins.add(b, mirror ? d + (own ? acc_norm2_wide(acc, astride, e, scale.s) : d) : d, mirror ? 2u : 1u);
     }
   });
   run.flush(bins);
-  bins.finish(numer, denom);
+  bins.finish(numer, denom, scale.inv);
 }
 
 // u_ij: one of the 12 real fields (f < 6: tau u_f; else u_c + tau u'_c,

@@ -67,28 +67,39 @@ __device__ __forceinline__ F2 norm2(float4 w) {
   const F2 r = {w.x, w.y}, i = {w.z, w.w};
   return f2_dot2(r, r, i, i, 1.f);
 }
-// in FP64, for sites that fail squares_fit
-__device__ __forceinline__ double norm2_wide(double2 w) { return norm2(w); }
-__device__ __forceinline__ double norm2_wide(float4 w) {
-  return norm2(make_double2((double)w.x + (double)w.y, (double)w.z + (double)w.w));
+// times s (FP64: 1), and in FP64 for sites that fail squares_fit
+__device__ __forceinline__ double norm2(double2 w, float) { return norm2(w); }
+__device__ __forceinline__ F2 norm2(float4 w, float s) {
+  return norm2(make_float4(s * w.x, s * w.y, s * w.z, s * w.w));
+}
+__device__ __forceinline__ double norm2_wide(double2 w, float) { return norm2(w); }
+__device__ __forceinline__ double norm2_wide(float4 w, float s) {
+  return norm2(make_double2(((double)w.x + (double)w.y) * (double)s, ((double)w.z + (double)w.w) * (double)s));
+}
+// the sample of a block: the first sites of rows 0, 1, ... of the plane kz = 0
+__device__ __forceinline__ SquareScale field_scale(const double2 *, int) { return SquareScale(); }
+__device__ __forceinline__ SquareScale field_scale(const float4 *__restrict__ F, int m) {
+  const float4 w = F[min((int)(threadIdx.x >> 5), m - 1) * m + min((int)(threadIdx.x & 31), m - 1)];
+  return SquareScale(fmaxf(fabsf(w.x), fabsf(w.z)));
 }
 template <typename V>
 __global__ void __launch_bounds__(256) k_spec_bin(const V *__restrict__ F, int m, int rows,
                                                   const int16_t *__restrict__ tab, int nb, int copies,
                                                   double *__restrict__ conv, double *__restrict__ count) {
   BlockBins bins(bins_mem(), nb, copies);
+  const SquareScale scale = field_scale(F, m);
   BinRun<decltype(norm2(F[0]))> run;
   walk_spectrum(m, m, rows, [&](int ix, int iy, int iz) {
     const int kx = kint(ix, m), ky = kint(iy, m), kz = kint(iz, m);
     const int b = tab[kx * kx + ky * ky + kz * kz];
     if (b < 0) return;
     const V f = F[((int64_t)iz * m + iy) * m + ix];
-    const auto v = norm2(f);
+    const auto v = norm2(f, scale.s);
     if (squares_fit(v)) run.add(bins, b, v, 1u);
-    else bins.add(b, norm2_wide(f), 1u);
+    else bins.add(b, norm2_wide(f, scale.s), 1u);
   });
   run.flush(bins);
-  bins.finish(conv, count);
+  bins.finish(conv, count, scale.inv);
 }
 
 // the real window of compute_matrix_deconv over its dx^3: 1 on unmasked coarse

@@ -112,3 +112,46 @@ def test_uij_powers_near_the_largest_float():
     np.testing.assert_array_equal(gde, de)
     assert np.all(np.isfinite(gnu))
     assert np.all(np.abs(gnu - nu) <= 1e-5 * np.max(nu))
+
+
+@pytest.mark.parametrize("precision", [ag.PREC_FP64_PLAIN, ag.PREC_FP32_MIXED])
+@pytest.mark.parametrize("n", [16, 32])
+def test_green_shells_of_uneven_entries(n, precision):
+    """Entries from 2^-110 to 2^60 side by side, a power of two for every |k|^2:
+    whatever a sample of them says, each is summed with its own digits."""
+    phi, phid = 1.0 + noise(n, n, 0.2), noise(n, n + 1, 0.1)
+    p = gw_params(n, ag.PREC_FP64_PLAIN, ag.GW_GREEN, 256)
+    acc = np.zeros((4, n, n, n), np.complex128)
+    axo.symplectic_integration(p, phi.copy(), phid.copy(), None, None, acc, 2.0, 2.4, 0.4)
+    k = np.round(np.fft.fftfreq(n) * n).astype(int)
+    k2 = k[:, None, None] ** 2 + k[None, :, None] ** 2 + k[None, None, :] ** 2
+    rng = np.random.default_rng(n)
+    # numbers per entry: with acc of order one, within FP32's range as pairs
+    acc *= np.ldexp(1.0, rng.choice([-110, -90, -60, -40, 0, 0, 30, 60], k2.max() + 1))[k2]
+    w, pw, nu, de = axo.grav_spec_estimation(p, acc)
+    with ag.Lattice(gw_params(n, precision, ag.GW_GREEN, 256)) as lat:
+        lat.upload_gw_green(acc)
+        _, _, gnu, gde = lat.grav_spec_estimation(2.4)
+    np.testing.assert_array_equal(gde, de)
+    # at 2^-110 a pair keeps 2^-149 of one: 39 bits, 2^-38 in the square
+    np.testing.assert_allclose(gnu, nu, rtol=2.0 ** -36)
+
+
+@pytest.mark.parametrize("shift", [-80, 0, 66])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_field_spectrum_of_one_wave(shift, axis):
+    """All power in one wave, the rest of the spectrum its transform's rounding."""
+    n = 32
+    phi = np.full((n, n, n), 1.0 + 0j)
+    z = np.exp(2j * np.pi * 5 * np.arange(n) / n)
+    phid = np.ldexp(1.0, shift) * np.broadcast_to(z.reshape([n if a == axis else 1 for a in range(3)]), (n, n, n)).copy()
+    p = spec_params(n)
+    flags, _ = axo.classify_cells(p, phi, 7, 0)
+    w, pw, cv, ct, md = axo.spectrum_estimation(p, phid, flags, 3.0)
+    with ag.Lattice(p) as lat:
+        lat.upload(phi, phid)
+        lat.classify_cells(7)
+        _, gpw, gcv, gct = lat.spectrum_estimation(3.0)
+    np.testing.assert_array_equal(gct, ct)
+    top = np.max(cv)
+    assert top > 0 and np.all(np.abs(gcv - cv) <= 1e-11 * top)
